@@ -54,6 +54,25 @@ int rows_fwd<T>(int M, const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw,
 }
 
 template <>
+int rows_fwd_real<T>(int M, const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw, cudaStream_t s) {
+#define X(MM, A, B, L32, L64) \
+  case MM: return Launch<T, A, B, kF32 ? L32 : L64>::rows_fwd_real(a, f0, nfg, S1, tw, s);
+  switch (M) { GATO_FAST_SHAPES(X) }
+#undef X
+  return kNotHandled;
+}
+
+template <>
+int rows_inv_real<T>(int M, const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,
+                     bool j, cudaStream_t s) {
+#define X(MM, A, B, L32, L64) \
+  case MM: return Launch<T, A, B, kF32 ? L32 : L64>::rows_inv_real(a, f0, nfg, S1, tw, accumulate, j, s);
+  switch (M) { GATO_FAST_SHAPES(X) }
+#undef X
+  return kNotHandled;
+}
+
+template <>
 int rows_inv<T>(int M, const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,
                 bool energy, double* partials, int64_t slot_stride, cudaStream_t s) {
 #define X(MM, A, B, L32, L64)                                                             \

@@ -106,33 +106,32 @@ static void block_pairs(PassArgs& a, const gato_operator& op, void* out, bool en
   }
   a.nout = energy ? 0 : n;
   int part = 0;
-  const int nd = n, no = n * (n - 1) / 2;
-  const int f_mixed = (1 + nd + no + 1) / 2, f_split = 1 + (nd + 1) / 2 + (no + 1) / 2;
-  if (energy && op.pp && poisson_fe_supported(op.pp->p) && f_split < 2 * f_mixed) {
-    // The spectral energy pass (half the work of a field's full solve) sums
-    // both parts of a field with one weight: the density rides alone, the
-    // diagonal pairs (weight -1) and the off-diagonal pairs (weight -2) fill
-    // fields of their own.
+  if (energy && op.pp && poisson_fe_supported(op.pp->p)) {
+    // The spectral energy pass sums both parts of a field with one weight: the diagonal pairs
+    // (weight -1) and the off-diagonal ones (weight -2) pair up among themselves, and what is left
+    // over rides alone at the end with the density (lone real fields cost half a field).
     a.in[n] = op.rho;
-    PartDesc& d = a.f[0].p[0];
-    d.a = (int8_t)n;
-    d.ew = 0.5;
-    d.eslot = 0;
-    int nf = 1;
+    int nf = 0, nl = 0;
+    PartDesc lone[3];
+    lone[nl].a = (int8_t)n;
+    lone[nl].ew = 0.5;
+    lone[nl++].eslot = 0;
     for (int w = 0; w < 2; ++w) {
+      const int count = w == 0 ? n : n * (n - 1) / 2;
       part = 0;
       for (int i = 0; i < n; ++i)
         for (int j = i; j < n; ++j) {
           if ((i == j) != (w == 0)) continue;
-          PartDesc& e = a.f[nf + part / 2].p[part % 2];
+          PartDesc& e = part % 2 == 0 && part + 1 == count ? lone[nl++] : a.f[nf + part / 2].p[part % 2];
           e.a = (int8_t)i;
           e.b = (int8_t)j;
           e.ew = i == j ? -1.0 : -2.0;   // E_x = -sum_ij <phi_i phi_j | J[phi_i phi_j]>
           e.eslot = 1;
           ++part;
         }
-      nf += (part + 1) / 2;
+      nf += count / 2;
     }
+    for (int k = 0; k < nl; ++k) a.f[nf++].p[0] = lone[k];
     a.nf = nf;
     return;
   }
@@ -245,7 +244,9 @@ extern "C" int gato_op_apply_block(gato_op_t op, void* out, void* stream) {
   GATO_TRY(fork_local(*op, op->orbitals, out, op->n_orb, s, &join));
   PassArgs a;
   block_pairs(a, *op, out, false);
-  if (op->block_epi != 2 && poisson_j_supported(op->pp->p)) {
+  // one orbital has one pair potential with one use: its z-inverse epilogue applies it directly
+  const bool jf = op->block_epi == 1 || (op->block_epi == 0 && op->n_orb > 1);
+  if (jf && poisson_j_supported(op->pp->p)) {
     // pair potentials to J fields, then one elementwise pass: out_i -= sum_j phi_j J_ij
     const size_t need = (size_t)2 * a.nf * op_n3(*op) * op_esize(*op);
     if (op->jbuf_bytes < need) {

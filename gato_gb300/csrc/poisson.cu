@@ -319,7 +319,6 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
   const int Linv = Lf > 0 ? Lf : Li;
   const int nblk_i = (int)((nrows + Linv - 1) / Linv);
   const int group = pl.group > 0 ? std::min(pl.group, pl.max_fields) : pl.max_fields;
-  const int ngroups = (args.nf + group - 1) / group;
   // FP64 energies on the register engine take the spectral (Parseval) pass
   // when both parts of every field carry one weight and one slot: x forward
   // and the kernel-weighted power, no x, y or z inverse.
@@ -340,6 +339,23 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
     fa.partials = pl.partials;
     fa.slot_stride = args.nf * fe_nb;
   }
+  // Trailing lone real fields (no imaginary part) take the half-spectrum passes: two rows per z line,
+  // columns kz <= N only, about half the arithmetic and traffic of a full field (96^3 FP64 Hartree
+  // solve 1306 -> 736 us). FP64, arithmetic-bound, always gains. An FP32 lone field behind full ones
+  // would cost a second set of launches, more than the half field it saves (exchange with three
+  // orbitals, split against not: 68 against 47 us at 64^3, 88 against 73 us at 80^3, 203 against 192 us at
+  // 128^3), so FP32 takes them only where no full field rides along. Energies take them in the
+  // spectral pass only, and a lone field's epilogue writes its terms straight to the outputs, so
+  // without accumulation it must be the call's one term.
+  int nlone = 0;
+  if (Lf > 0 && pl.engine == 0 && (epi != EPI_ENERGY || fe)) {
+    while (nlone < args.nf && args.f[args.nf - 1 - nlone].p[1].a < 0) ++nlone;
+    const PartDesc& d0 = args.f[args.nf - 1].p[0];
+    if (epi == EPI_ACC && (nlone > 1 || (!accumulate && (args.nf > 1 || args.nout != 1 || d0.nt != 1)))) nlone = 0;
+    if (sizeof(T) == 4 && nlone < args.nf) nlone = 0;
+  }
+  const int nfull = args.nf - nlone;
+  const int gfull = (nfull + group - 1) / group, ngroups = gfull + (nlone + group - 1) / group;
   if (epi == EPI_ENERGY && !fe && (int64_t)ngroups * 2 * nblk_i > pl.npart_cap)
     return fail(GATO_EUNSUPPORTED, "poisson: energy partials exceed plan capacity");
   if (Lf == 0) {
@@ -351,13 +367,43 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
   ColGeom gx{(int64_t)N * M * M, (int64_t)N * M * M, M, M, (int64_t)M * M, (int64_t)M * M, M, N, N};
   ColGeom gyi{(int64_t)N * M * M, nrows * M, (int64_t)M * M, (int64_t)N * M, M, M, M, M, N};
   for (int g = 0; g < ngroups; ++g) {
-    const int f0 = g * group;
-    const int nfg = std::min(group, args.nf - f0);
+    const bool lone = g >= gfull;
+    const int f0 = lone ? nfull + (g - gfull) * group : g * group;
+    const int nfg = std::min(group, (lone ? args.nf : nfull) - f0);
     const bool acc_here = accumulate || g > 0;
     double* part = pl.partials + (int64_t)g * nblk_i;
     const int64_t sstride = (int64_t)ngroups * nblk_i;
     if (Lf > 0) {
       // register-resident two-pass engine
+      if (lone) {
+        auto half = [&](ColGeom q, int tile) {   // the N + 1 columns, rounded up to whole tiles
+          q.ncols = std::min(M, (N + tile) / tile * tile);
+          return q;
+        };
+        GATO_TRY(fast::rows_fwd_real<T>(M, args, f0, nfg, S1, tw2, s));
+        if (packed) {
+          const float4* t4 = (const float4*)pl.tw4;
+          GATO_TRY(fast::packed_cols(M, COL_FWD, (const float2*)S1, (float2*)S2, half(gy, 16), N, nfg, t4, nullptr, pl.H, s));
+          GATO_TRY(fast::packed_cols(M, COL_FMI, (const float2*)S2, (float2*)S2, half(gx, 16), M, nfg, t4,
+                                     (const float*)pl.ghat2, pl.H, s));
+          GATO_TRY(fast::packed_cols(M, COL_INV, (const float2*)S2, (float2*)S1, half(gyi, 16), N, nfg, t4, nullptr, pl.H, s));
+        } else {
+          GATO_TRY(fast::cols<T>(M, COL_FWD, S1, S2, half(gy, Lf), N, nfg, tw2, nullptr, pl.H, s));
+          if constexpr (sizeof(T) == 8) {
+            if (fe) {
+              fa.f0 = f0;
+              fa.half = 1;
+              GATO_TRY(fast::cols_fe<T>(M, S2, gx, M, nfg, tw2, (const T*)pl.ghat, pl.H, fa, s));
+              continue;
+            }
+          }
+          GATO_TRY(fast::cols<T>(M, COL_FMI, S2, S2, half(gx, Lf), M, nfg, tw2, (const T*)pl.ghat, pl.H, s));
+          GATO_TRY(fast::cols<T>(M, COL_INV, S2, S1, half(gyi, Lf), N, nfg, tw2, nullptr, pl.H, s));
+        }
+        if (join && g == 0 && epi == EPI_ACC) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
+        GATO_TRY(fast::rows_inv_real<T>(M, args, f0, nfg, S1, tw2, acc_here ? 1 : 0, epi == EPI_J, s));
+        continue;
+      }
       // engine 0: multi-field z forward from two fields, 2: never, 3: from three
       GATO_TRY(fast::rows_fwd<T>(M, args, f0, nfg, S1, tw2, pl.engine == 2 ? 0 : (pl.engine == 3 ? 1 : (pl.engine == 4 ? 3 : 2)), s));
       if (packed) {

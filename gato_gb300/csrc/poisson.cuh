@@ -84,6 +84,7 @@ struct FeArgs {
   double* partials = nullptr;
   int64_t slot_stride = 0;
   int f0 = 0;                  // first field of this launch within the call
+  int half = 0;                // 1: lone real fields, columns kz <= M/2 with the weight of their mirror
   double w[kMaxFields] = {};
   int8_t slot[kMaxFields] = {};
 };
@@ -116,6 +117,13 @@ template <typename T>
 int rows_inv(int M, const PassArgs& a, int f0, int nfg, const typename Cplx<T>::type* S1,
              const typename Cplx<T>::type* tw, int accumulate, bool energy, double* partials,
              int64_t slot_stride, cudaStream_t s);
+// z passes of lone real fields (parts p[1] absent), two rows per line, half spectra (columns kz <= M/2).
+template <typename T>
+int rows_fwd_real(int M, const PassArgs& a, int f0, int nfg, typename Cplx<T>::type* S1,
+                  const typename Cplx<T>::type* tw, cudaStream_t s);
+template <typename T>
+int rows_inv_real(int M, const PassArgs& a, int f0, int nfg, const typename Cplx<T>::type* S1,
+                  const typename Cplx<T>::type* tw, int accumulate, bool j, cudaStream_t s);
 // z inverse writing the real and imaginary parts of J as separate fields (EPI_J).
 template <typename T>
 int rows_inv_j(int M, const PassArgs& a, int f0, int nfg, const typename Cplx<T>::type* S1,

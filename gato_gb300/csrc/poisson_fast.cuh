@@ -144,6 +144,12 @@ __device__ __forceinline__ double block_sum0(const Acc<double>& a, double* sh) {
   return block_sum(a.value(), sh);
 }
 
+// acc times a small whole number w (exact for 0, 1 and 2).
+__device__ __forceinline__ Acc<double> scaled(Acc<double> a, int w) {
+  a.v = w == 0 ? 0.0 : a.v * w;   // a column without weight may hold anything
+  return a;
+}
+
 // Energies without the inverse passes (Parseval). The kernel spectrum is
 // stored as ghat = G^ dV / M^3, so a part's epilogue energy sum_r rho J with
 // J = IDFT(ghat DFT(rho)) (unnormalised) equals sum_k ghat(k) |rho^(k)|^2 over
@@ -169,6 +175,13 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   const int outer = blockIdx.x, col0 = blockIdx.y * L, f = blockIdx.z;
   const int t = threadIdx.x;
   const int line = t % L, q = t / L;
+  if (fa.half && col0 > M / 2) {   // no column of a lone real field's half spectrum
+    if (t == 0) {
+      const int64_t b = ((int64_t)(fa.f0 + f) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+      fa.partials[b] = fa.partials[fa.slot_stride + b] = 0.0;
+    }
+    return;
+  }
   const bool live = FULL || line < g.ncols - col0;
   const T2* src = in + f * g.in_fs + outer * g.in_os + col0 + line;
   const int64_t ips = g.in_ps;
@@ -198,6 +211,9 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
       const T gv = live ? (k2 < R2 / 2 ? glo[k2 * st] : ghi[-k2 * st]) : (T)0;
       acc.add_prod(gv, X[k2].x * X[k2].x + X[k2].y * X[k2].y);
     }
+    // a lone real field's columns kz and M - kz carry the same power: 0 < kz < M/2 counts twice
+    // (the sum is linear in the weight, so it scales the column's finished sum)
+    if (fa.half) acc = scaled(acc, kz == 0 || kz == M / 2 ? 1 : (kz < M / 2 ? 2 : 0));
   }
   const double s = block_sum0(acc, sh);
   if (t == 0) {
@@ -634,6 +650,140 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX, (rows_inv_min_ctas<T,
   }
 }
 
+// ---- lone real fields ------------------------------------------------------------------
+// A field whose imaginary part is absent (a Hartree density, the last pair of an odd count) is
+// real, so its spectrum is Hermitian and the columns kz <= N = M/2 hold all of it. Its z passes
+// transform TWO rows per line, rows 2l and 2l + 1 as real and imaginary part, and the column
+// passes run over the N + 1 columns alone (rounded up to whole tiles): about half the arithmetic
+// and half the spectral traffic of a complex field with a zero imaginary part. The FP64 passes are
+// bound by the FP64 pipe, so the arithmetic is what counts: a 96^3 Hartree solve took 1306 us with
+// the zero imaginary part and takes 736 us; the helium matvec at 64^3 falls in the same ratio.
+
+// z forward: Z = FFT(row_2l + i row_2l+1), A = (Z_k + conj Z_-k) / 2 and B = (Z_k - conj Z_-k) / 2i
+// are the two rows' spectra; the halves are taken on the inputs (exact). One field per grid.y.
+template <typename T, int R1, int R2, int L>
+__global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
+    k_rows_fwd_real(PassArgs args, int f0, typename Cplx<T>::type* S1, const typename Cplx<T>::type* tw) {
+  using T2 = typename Cplx<T>::type;
+  constexpr int M = R1 * R2, N = M / 2, RM = Shape<R1, R2>::RMAX, NT = L * RM, LS = RowBuf<R1, R2>::LS;
+  static_assert(N % 2 == 0 && LS >= M, "rows pair up; a line's buffer holds its whole spectrum");
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T2* buf = reinterpret_cast<T2*>(smraw);
+  T2* tws = buf + L * LS;
+  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  const int p = blockIdx.y;
+  const PartDesc& pd = args.f[f0 + p].p[0];
+  const int64_t npair = (int64_t)N * N / 2;
+  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
+  const int64_t l = (int64_t)blockIdx.x * L + line;
+  const bool live = l < npair;
+  const T* a = reinterpret_cast<const T*>(args.in[pd.a]);
+  const T* b = pd.b >= 0 ? reinterpret_cast<const T*>(args.in[pd.b]) : nullptr;
+  T2 v[R1];
+  if (j < R2) {
+#pragma unroll
+    for (int n1 = 0; n1 < R1 / 2; ++n1) {
+      const int64_t gi = 2 * l * N + R2 * n1 + j;
+      v[n1].x = live ? (T)0.5 * part_density(a, b, gi) : (T)0;
+      v[n1].y = live ? (T)0.5 * part_density(a, b, gi + N) : (T)0;
+    }
+  }
+  twp.store(tws);
+  if (j < R2) row_fwd_stage1<T2, R1, R2, true>(buf, line, j, v);
+  __syncthreads();
+  T2 X[R2];
+  if (j < R1) row_fwd_stage2<T2, R1, R2>(buf, line, j, tws, X);
+  __syncthreads();   // stage-2 reads of buf are complete
+  if (j < R1) {
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) buf[line * LS + j + R1 * k2] = X[k2];
+  }
+  __syncthreads();
+  if (!live) return;
+  T2* d = S1 + ((int64_t)p * N * N + 2 * l) * M;
+  for (int k = j; k <= N; k += RM) {
+    const T2 z = buf[line * LS + k], c = buf[line * LS + (k == 0 ? 0 : M - k)];
+    T2 A, B;
+    A.x = z.x + c.x;
+    A.y = z.y - c.y;
+    B.x = z.y + c.y;
+    B.y = c.x - z.x;
+    d[k] = A;
+    d[M + k] = B;
+  }
+}
+
+// z inverse of row pairs: Z_k = A_k + i B_k for k <= N and conj(A_M-k) + i conj(B_M-k) above, whose
+// transform is row_2l + i row_2l+1. J: the potential goes to field 2 (f0 + p) of jbase (one field per
+// grid.y); otherwise one field's terms are added to (or, not accumulating, written to) the outputs.
+template <typename T, int R1, int R2, int L, bool J>
+__global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
+    k_rows_inv_real(PassArgs args, int f0, const typename Cplx<T>::type* S1, const typename Cplx<T>::type* tw,
+                    int accumulate) {
+  using T2 = typename Cplx<T>::type;
+  constexpr int M = R1 * R2, N = M / 2, RM = Shape<R1, R2>::RMAX, NT = L * RM;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T2* buf = reinterpret_cast<T2*>(smraw);
+  T2* tws = buf + L * RowBuf<R1, R2>::LS;
+  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  const int p = blockIdx.y;
+  const int64_t npair = (int64_t)N * N / 2;
+  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
+  const int64_t l = (int64_t)blockIdx.x * L + line;
+  const bool live = l < npair;
+  T2 X[R2];
+  if (j < R1) {
+    const T2* A = S1 + ((int64_t)p * N * N + 2 * l) * M;
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) {
+      const int k = j + R1 * k2;
+      const bool up = k > N;
+      T2 a, b;
+      a.x = a.y = b.x = b.y = 0;
+      if (live) {
+        a = A[up ? M - k : k];
+        b = A[M + (up ? M - k : k)];
+      }
+      X[k2].x = up ? a.x + b.y : a.x - b.y;
+      X[k2].y = up ? b.x - a.y : a.y + b.x;
+    }
+  }
+  twp.store(tws);
+  __syncthreads();
+  if (j < R1) row_inv_stageA<T2, R1, R2>(buf, line, j, tws, X);
+  __syncthreads();
+  if (j >= R2 || !live) return;
+  T2 w[R1];
+  row_inv_stageB<T2, R1, R2>(buf, line, j, w);
+  const int64_t g0 = 2 * l * N + j;
+  if constexpr (J) {
+    T* o = reinterpret_cast<T*>(args.jbase) + (int64_t)(2 * (f0 + p)) * args.jstride + g0;
+#pragma unroll
+    for (int e = 0; e < R1 / 2; ++e) {
+      o[R2 * e] = w[e].x;
+      o[N + R2 * e] = w[e].y;
+    }
+  } else {
+    const PartDesc& d = args.f[f0 + p].p[0];
+#pragma unroll 1
+    for (int k = 0; k < d.nt; ++k) {
+      T* o = reinterpret_cast<T*>(args.out[d.to[k]]) + g0;
+      const T* u = d.tc[k] >= 0 ? reinterpret_cast<const T*>(args.in[d.tc[k]]) + g0 : nullptr;
+      const T cf = (T)d.coef[k];
+#pragma unroll
+      for (int e = 0; e < R1 / 2; ++e)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = R2 * e + h * N;
+          T m = cf;
+          if (u) m *= u[i];
+          const T val = m * (h == 0 ? w[e].x : w[e].y);
+          o[i] = accumulate ? o[i] + val : val;
+        }
+    }
+  }
+}
+
 // z inverse of one field per CTA (grid.y = field), writing J_re and J_im of
 // the row block to their own real fields (the EPI_J epilogue).
 template <typename T, int R1, int R2, int L>
@@ -722,6 +872,29 @@ struct Launch {
     } else {
       GATO_TRY(smem_attr(k_cols_fe<T, R1, R2, L, false>, sm));
       k_cols_fe<T, R1, R2, L, false><<<grid, NT, sm, s>>>(in, g, tw, ghat, H, fa);
+    }
+    GATO_LAUNCH_TRY();
+    return GATO_OK;
+  }
+  static int rows_fwd_real(const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw, cudaStream_t s) {
+    const size_t sm = sm_rows();
+    GATO_TRY(smem_attr(k_rows_fwd_real<T, R1, R2, L>, sm));
+    const unsigned nblk = (unsigned)(((int64_t)N * N / 2 + L - 1) / L);
+    k_rows_fwd_real<T, R1, R2, L><<<dim3(nblk, nfg), NT, sm, s>>>(a, f0, S1, tw);
+    GATO_LAUNCH_TRY();
+    return GATO_OK;
+  }
+  // j: potentials to the J fields (nfg fields at once), else one field's terms to the outputs
+  static int rows_inv_real(const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,
+                           bool j, cudaStream_t s) {
+    const size_t sm = sm_rows();
+    const unsigned nblk = (unsigned)(((int64_t)N * N / 2 + L - 1) / L);
+    if (j) {
+      GATO_TRY(smem_attr(k_rows_inv_real<T, R1, R2, L, true>, sm));
+      k_rows_inv_real<T, R1, R2, L, true><<<dim3(nblk, nfg), NT, sm, s>>>(a, f0, S1, tw, 0);
+    } else {
+      GATO_TRY(smem_attr(k_rows_inv_real<T, R1, R2, L, false>, sm));
+      k_rows_inv_real<T, R1, R2, L, false><<<dim3(nblk, 1), NT, sm, s>>>(a, f0, S1, tw, accumulate);
     }
     GATO_LAUNCH_TRY();
     return GATO_OK;

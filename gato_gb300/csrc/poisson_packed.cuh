@@ -220,8 +220,8 @@ struct LaunchP {
   // in: the pass's input buffer (S1 for the y forward, S2 otherwise), nfa fields allocated.
   static int cols(int mode, const float2* in, float2* out, const ColGeom& g, int outer, int nf,
                   const float4* tw4, const float* ghat2, cudaStream_t s) {
-    if (g.ncols != M || g.ncols % CW != 0)
-      return fail(GATO_EUNSUPPORTED, "packed column pass: columns must be the M = %d spectrum columns", M);
+    if (g.ncols > M || g.ncols % CW != 0)
+      return fail(GATO_EUNSUPPORTED, "packed column pass: whole tiles of the M = %d spectrum columns", M);
     alignas(64) unsigned char tm[128];
     alignas(64) unsigned char gm[128] = {};
     TmaBox b;
