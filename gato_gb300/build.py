@@ -66,7 +66,7 @@ def build(verbose: bool = False, force: bool = False, extra_flags=()) -> str:
             print(r.stdout + r.stderr, file=sys.stderr)
         return obj
 
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with ThreadPoolExecutor(max_workers=min(16, len(srcs))) as ex:
         objs = list(ex.map(compile_one, srcs))
     tmp = LIB + ".tmp"
     cmd = [nvcc, "-shared", *ARCH, "-o", tmp, *objs]

@@ -1,0 +1,5 @@
+// Register-engine pair-solve kernels, FP32 fields, shape group 0.
+#define GATO_FAST_T float
+#define GATO_FAST_G 0
+#define GATO_FAST_SHAPES GATO_FAST_SHAPES_0
+#include "fast_inst.cuh"

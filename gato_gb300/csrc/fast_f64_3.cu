@@ -1,0 +1,6 @@
+// Register-engine pair-solve kernels, FP64 fields, shape group 3.
+#define GATO_FAST_T double
+#define GATO_FAST_G 3
+#define GATO_FAST_FE
+#define GATO_FAST_SHAPES GATO_FAST_SHAPES_3
+#include "fast_inst.cuh"

@@ -21,6 +21,8 @@ namespace gato {
 namespace fft2 {
 
 template <int R> struct Split;
+template <> struct Split<9> { static constexpr int A = 3, B = 3; };
+template <> struct Split<18> { static constexpr int A = 2, B = 9; };
 template <> struct Split<6> { static constexpr int A = 2, B = 3; };
 template <> struct Split<10> { static constexpr int A = 2, B = 5; };
 template <> struct Split<12> { static constexpr int A = 4, B = 3; };

@@ -2,7 +2,7 @@
 import math
 import os
 
-RADICES = [4, 6, 8, 10, 12, 14, 16, 20, 24]
+RADICES = [4, 6, 8, 9, 10, 12, 14, 16, 18, 20, 24]
 
 
 def _exact(x):

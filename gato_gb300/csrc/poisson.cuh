@@ -89,45 +89,91 @@ struct FeArgs {
   int8_t slot[kMaxFields] = {};
 };
 
-// Register-resident two-pass kernels for the common sizes M = 2N (see
-// fft2.cuh); each returns kNotHandled when M has no instantiation.
+// Register-resident two-pass kernels for the sizes M = 2N of fast_shapes.cuh (see fft2.cuh), compiled
+// in kFastGroups translation units per field type; each call returns kNotHandled when M has no
+// instantiation (of the group).
 namespace fast {
 constexpr int kNotHandled = 1;
-template <typename T> int rows_L(int M);   // lines per CTA of the z kernels, 0 if unsupported
-int shape_r2(int M);                        // R2 of the register engine's M = R1 R2, 0 if none
+constexpr int kFastGroups = 4;
 template <typename T>
-int cols(int M, int mode, const typename Cplx<T>::type* in, typename Cplx<T>::type* out,
-         const ColGeom& g, int outer, int nf, const typename Cplx<T>::type* tw, const T* ghat,
-         int H, cudaStream_t s);
+using C2 = typename Cplx<T>::type;
+
+template <typename T, int G> int rows_L_g(int M);
+template <typename T, int G>
+int cols_g(int M, int mode, const C2<T>* in, C2<T>* out, const ColGeom& g, int outer, int nf, const C2<T>* tw,
+           const T* ghat, int H, cudaStream_t s);
+template <typename T, int G>
+int cols_fe_g(int M, const C2<T>* in, const ColGeom& g, int outer, int nf, const C2<T>* tw, const T* ghat, int H,
+              const FeArgs& fa, cudaStream_t s);
+template <typename T, int G>
+int rows_fwd_g(int M, const PassArgs& a, int f0, int nfg, C2<T>* S1, const C2<T>* tw, int multi, cudaStream_t s);
+template <typename T, int G>
+int rows_inv_g(int M, const PassArgs& a, int f0, int nfg, const C2<T>* S1, const C2<T>* tw, int accumulate,
+               bool energy, double* partials, int64_t slot_stride, cudaStream_t s);
+template <typename T, int G>
+int rows_inv_j_g(int M, const PassArgs& a, int f0, int nfg, const C2<T>* S1, const C2<T>* tw, cudaStream_t s);
+template <typename T, int G>
+int rows_fwd_real_g(int M, const PassArgs& a, int f0, int nfg, C2<T>* S1, const C2<T>* tw, cudaStream_t s);
+template <typename T, int G>
+int rows_inv_real_g(int M, const PassArgs& a, int f0, int nfg, const C2<T>* S1, const C2<T>* tw, int accumulate,
+                    bool j, cudaStream_t s);
+
+// Calls FN<T, 0>, FN<T, 1>, ... until one handles M.
+#define GATO_FAST_GROUPS(FN, ...)                          \
+  int r = FN<T, 0>(__VA_ARGS__);                           \
+  if (r == kNotHandled) r = FN<T, 1>(__VA_ARGS__);         \
+  if (r == kNotHandled) r = FN<T, 2>(__VA_ARGS__);         \
+  if (r == kNotHandled) r = FN<T, 3>(__VA_ARGS__);         \
+  return r
+
+int shape_r2(int M);   // R2 of the register engine's M = R1 R2, 0 if none
+template <typename T>
+int rows_L(int M) {    // lines per CTA of the z kernels, 0 if unsupported
+  const int r = rows_L_g<T, 0>(M) + rows_L_g<T, 1>(M) + rows_L_g<T, 2>(M) + rows_L_g<T, 3>(M);
+  return r;
+}
+template <typename T>
+int cols(int M, int mode, const C2<T>* in, C2<T>* out, const ColGeom& g, int outer, int nf, const C2<T>* tw,
+         const T* ghat, int H, cudaStream_t s) {
+  GATO_FAST_GROUPS(cols_g, M, mode, in, out, g, outer, nf, tw, ghat, H, s);
+}
+// x forward of the y-transformed fields and the kernel-weighted spectral power
+// per CTA (the energy epilogue without the inverse passes); FP64.
+template <typename T>
+int cols_fe(int M, const C2<T>* in, const ColGeom& g, int outer, int nf, const C2<T>* tw, const T* ghat, int H,
+            const FeArgs& fa, cudaStream_t s) {
+  GATO_FAST_GROUPS(cols_fe_g, M, in, g, outer, nf, tw, ghat, H, fa, s);
+}
+template <typename T>
+int rows_fwd(int M, const PassArgs& a, int f0, int nfg, C2<T>* S1, const C2<T>* tw, int multi, cudaStream_t s) {
+  GATO_FAST_GROUPS(rows_fwd_g, M, a, f0, nfg, S1, tw, multi, s);
+}
+template <typename T>
+int rows_inv(int M, const PassArgs& a, int f0, int nfg, const C2<T>* S1, const C2<T>* tw, int accumulate,
+             bool energy, double* partials, int64_t slot_stride, cudaStream_t s) {
+  GATO_FAST_GROUPS(rows_inv_g, M, a, f0, nfg, S1, tw, accumulate, energy, partials, slot_stride, s);
+}
+// z inverse writing the real and imaginary parts of J as separate fields (EPI_J).
+template <typename T>
+int rows_inv_j(int M, const PassArgs& a, int f0, int nfg, const C2<T>* S1, const C2<T>* tw, cudaStream_t s) {
+  GATO_FAST_GROUPS(rows_inv_j_g, M, a, f0, nfg, S1, tw, s);
+}
+// z passes of lone real fields (parts p[1] absent), two rows per line, half spectra (columns kz <= M/2).
+template <typename T>
+int rows_fwd_real(int M, const PassArgs& a, int f0, int nfg, C2<T>* S1, const C2<T>* tw, cudaStream_t s) {
+  GATO_FAST_GROUPS(rows_fwd_real_g, M, a, f0, nfg, S1, tw, s);
+}
+template <typename T>
+int rows_inv_real(int M, const PassArgs& a, int f0, int nfg, const C2<T>* S1, const C2<T>* tw, int accumulate,
+                  bool j, cudaStream_t s) {
+  GATO_FAST_GROUPS(rows_inv_real_g, M, a, f0, nfg, S1, tw, accumulate, j, s);
+}
+
 // FP32 column passes on the packed two-line engine (poisson_packed.cuh): R2 of
 // M = R1 R2 when M has an instantiation, else 0.
 int packed_r2(int M);
 int packed_cols(int M, int mode, const float2* in, float2* out, const ColGeom& g, int outer, int nf,
                 const float4* tw4, const float* ghat2, int H, cudaStream_t s);
-// x forward of the y-transformed fields and the kernel-weighted spectral power
-// per CTA (the energy epilogue without the inverse passes).
-template <typename T>
-int cols_fe(int M, const typename Cplx<T>::type* in, const ColGeom& g, int outer, int nf,
-            const typename Cplx<T>::type* tw, const T* ghat, int H, const FeArgs& fa,
-            cudaStream_t s);
-template <typename T>
-int rows_fwd(int M, const PassArgs& a, int f0, int nfg, typename Cplx<T>::type* S1,
-             const typename Cplx<T>::type* tw, int multi, cudaStream_t s);
-template <typename T>
-int rows_inv(int M, const PassArgs& a, int f0, int nfg, const typename Cplx<T>::type* S1,
-             const typename Cplx<T>::type* tw, int accumulate, bool energy, double* partials,
-             int64_t slot_stride, cudaStream_t s);
-// z passes of lone real fields (parts p[1] absent), two rows per line, half spectra (columns kz <= M/2).
-template <typename T>
-int rows_fwd_real(int M, const PassArgs& a, int f0, int nfg, typename Cplx<T>::type* S1,
-                  const typename Cplx<T>::type* tw, cudaStream_t s);
-template <typename T>
-int rows_inv_real(int M, const PassArgs& a, int f0, int nfg, const typename Cplx<T>::type* S1,
-                  const typename Cplx<T>::type* tw, int accumulate, bool j, cudaStream_t s);
-// z inverse writing the real and imaginary parts of J as separate fields (EPI_J).
-template <typename T>
-int rows_inv_j(int M, const PassArgs& a, int f0, int nfg, const typename Cplx<T>::type* S1,
-               const typename Cplx<T>::type* tw, cudaStream_t s);
 }  // namespace fast
 
 // out_a -= phi_b J_ab and out_b -= phi_a J_ab for every pair a <= b of n

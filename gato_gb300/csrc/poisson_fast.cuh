@@ -226,11 +226,23 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
 }
 
 // ---- z passes (rows) ---------------------------------------------------------------
-// A CTA owns L consecutive rows (x, y) of the z axis; thread t works on line
-// t / RMAX as item j = t % RMAX: n2 in stages 1 and B, k1 in stages 2 and A
-// (the RowBuf layout of fft2.cuh). Field rows are read and spectra written
+// A CTA owns L consecutive rows (x, y) of the z axis; each stage deals its
+// items to the lowest threads: n2 of line l1 in stages 1 and B, k1 of line l2
+// in stages 2 and A (RowMap; the RowBuf layout of fft2.cuh), so where R1 and
+// R2 differ whole warps idle in the smaller stage, not lanes of every warp (an
+// FP64 instruction takes its 64 cycles of the narrow pipe whatever its lanes;
+// 96^3 Hartree solve, 12 x 16, 626 -> 609 us). Field rows are read and spectra written
 // straight from registers with lanes on consecutive z (or kz), so every
 // global access is coalesced and no shared-memory transpose is needed.
+
+template <int R1, int R2, int L>
+struct RowMap {
+  int l1, n2, l2, k1;
+  bool a1, a2;   // this thread has an item in stages 1/B, in stages 2/A
+  __device__ __forceinline__ RowMap()
+      : l1(threadIdx.x / R2), n2(threadIdx.x % R2), l2(threadIdx.x / R1), k1(threadIdx.x % R1),
+        a1(R2 >= R1 || threadIdx.x < L * R2), a2(R1 >= R2 || threadIdx.x < L * R1) {}
+};
 
 // Pair density of part q of a field at element gi (0 when the part is absent).
 template <typename T>
@@ -254,41 +266,41 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   const int p = blockIdx.y;
   const FieldDesc& fd = args.f[f0 + p];
   const int64_t nrows = (int64_t)N * N;
-  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
-  const int64_t r = (int64_t)blockIdx.x * L + line;
-  const bool live = r < nrows;
+  const RowMap<R1, R2, L> q;
+  const int64_t row0 = (int64_t)blockIdx.x * L;
   // the pair-density factors of the real and imaginary parts (null: factor absent)
   const T* a0 = reinterpret_cast<const T*>(args.in[fd.p[0].a]);
   const T* b0 = fd.p[0].b >= 0 ? reinterpret_cast<const T*>(args.in[fd.p[0].b]) : nullptr;
   const T* a1 = fd.p[1].a >= 0 ? reinterpret_cast<const T*>(args.in[fd.p[1].a]) : nullptr;
   const T* b1 = (a1 && fd.p[1].b >= 0) ? reinterpret_cast<const T*>(args.in[fd.p[1].b]) : nullptr;
   T2 v[R1];
-  if (j < R2) {
+  if (q.a1) {
+    const bool live = row0 + q.l1 < nrows;
 #pragma unroll
     for (int n1 = 0; n1 < R1 / 2; ++n1) {
-      const int64_t gi = r * N + R2 * n1 + j;
+      const int64_t gi = (row0 + q.l1) * N + R2 * n1 + q.n2;
       v[n1].x = live ? part_density(a0, b0, gi) : (T)0;
       v[n1].y = live ? part_density(a1, b1, gi) : (T)0;
     }
   }
   twp.store(tws);
-  if (j < R2) row_fwd_stage1<T2, R1, R2, true>(buf, line, j, v);
+  if (q.a1) row_fwd_stage1<T2, R1, R2, true>(buf, q.l1, q.n2, v);
   __syncthreads();
-  if (j < R1) {
+  if (q.a2) {
     T2 X[R2];
-    row_fwd_stage2<T2, R1, R2>(buf, line, j, tws, X);
-    if (live) {
-      T2* d = S1 + (int64_t)p * nrows * M + r * M + j;
+    row_fwd_stage2<T2, R1, R2>(buf, q.l2, q.k1, tws, X);
+    if (row0 + q.l2 < nrows) {
+      T2* d = S1 + (int64_t)p * nrows * M + (row0 + q.l2) * M + q.k1;
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2) d[R1 * k2] = X[k2];
     }
   }
 }
 
-// Padded length of a staged input row: N rounded up to RMAX modulo 32 words.
+// Padded length of a staged input row: N rounded up to R2 modulo 32 words.
 template <int R1, int R2> struct StageRow {
-  static constexpr int N = R1 * R2 / 2, RM = Shape<R1, R2>::RMAX;
-  static constexpr int NP = N + ((RM - N % 32) % 32 + 32) % 32;
+  static constexpr int N = R1 * R2 / 2;
+  static constexpr int NP = N + ((R2 - N % 32) % 32 + 32) % 32;
 };
 
 // The inputs a launch group of pair fields reads, staged once per CTA by
@@ -303,8 +315,8 @@ struct RowsIn {
 // input (the orbitals, psi) are staged in shared memory once, then each field's
 // pair densities are formed straight into the stage-1 registers of its FFT.
 // Same transform and output as k_rows_fwd, without re-reading the inputs per
-// field. Stage-1 lanes read consecutive z of RMAX-lane lines, so a staged row
-// is padded to a multiple of 32 words plus RMAX (StageRow): the lines a warp
+// field. Stage-1 lanes read consecutive z of R2-lane lines, so a staged row
+// is padded to a multiple of 32 words plus R2 (StageRow): the lines a warp
 // reads fall in disjoint bank ranges.
 // BULK: one elected thread stages every row with a 1-D bulk copy
 // (cp.async.bulk, one mbarrier for the whole block, a bounded wait), so the
@@ -382,11 +394,12 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   twp.store(tws);
   __syncthreads();
   }
-  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
-  const int64_t r = row0 + line;
+  const RowMap<R1, R2, L> q;
+  const int64_t r = row0 + q.l2;
   for (int p = 0; p < nfg; ++p) {
     const FieldDesc& fd = args.f[f0 + p];
-    if (j < R2) {
+    if (q.a1) {
+      const int line = q.l1, j = q.n2;
       const int a0 = ri.slot_of[fd.p[0].a];
       const int b0 = fd.p[0].b >= 0 ? ri.slot_of[fd.p[0].b] : -1;
       const int a1 = fd.p[1].a >= 0 ? ri.slot_of[fd.p[1].a] : -1;
@@ -408,11 +421,11 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
       row_fwd_stage1<T2, R1, R2, true>(buf, line, j, v);
     }
     __syncthreads();
-    if (j < R1) {
+    if (q.a2) {
       T2 X[R2];
-      row_fwd_stage2<T2, R1, R2>(buf, line, j, tws, X);
+      row_fwd_stage2<T2, R1, R2>(buf, q.l2, q.k1, tws, X);
       if (r < nrows) {
-        T2* d = S1 + (int64_t)p * nrows * M + r * M + j;
+        T2* d = S1 + (int64_t)p * nrows * M + r * M + q.k1;
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2) d[R1 * k2] = X[k2];
       }
@@ -469,7 +482,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
     }
   };
   if (threadIdx.x == 0 && (int)blockIdx.x < nblk) issue(blockIdx.x, 0);
-  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
+  const RowMap<R1, R2, L> q;
   int it = 0;
   for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x, ++it) {
     const int slot = it & 1;
@@ -485,10 +498,11 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
       return;
     }
     const T* stage = stage0 + slot * SB;
-    const int64_t r = (int64_t)blk * L + line;
+    const int64_t r = (int64_t)blk * L + q.l2;
     for (int p = 0; p < nfg; ++p) {
       const FieldDesc& fd = args.f[f0 + p];
-      if (j < R2) {
+      if (q.a1) {
+        const int line = q.l1, j = q.n2;
         const int a0 = ri.slot_of[fd.p[0].a];
         const int b0 = fd.p[0].b >= 0 ? ri.slot_of[fd.p[0].b] : -1;
         const int a1 = fd.p[1].a >= 0 ? ri.slot_of[fd.p[1].a] : -1;
@@ -511,10 +525,10 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
       }
       fence_proxy_async_smem();   // this slot's reads precede the copies issued into it next
       __syncthreads();
-      if (j < R1) {
+      if (q.a2) {
         T2 X[R2];
-        row_fwd_stage2<T2, R1, R2>(buf, line, j, tws, X);
-        T2* d = S1 + (int64_t)p * nrows * M + r * M + j;
+        row_fwd_stage2<T2, R1, R2>(buf, q.l2, q.k1, tws, X);
+        T2* d = S1 + (int64_t)p * nrows * M + r * M + q.k1;
 #pragma unroll
         for (int k2 = 0; k2 < R2; ++k2) d[R1 * k2] = X[k2];
       }
@@ -547,9 +561,11 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX, (rows_inv_min_ctas<T,
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
   const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
   const int64_t nrows = (int64_t)N * N;
-  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
-  const int64_t r = (int64_t)blockIdx.x * L + line;
-  const bool own = j < R2 && r < nrows;   // this thread owns elements of the output
+  const RowMap<R1, R2, L> q;
+  const int j = q.n2;
+  const int64_t r = (int64_t)blockIdx.x * L + q.l1;     // row of this thread's outputs
+  const int64_t rk = (int64_t)blockIdx.x * L + q.l2;    // row of its spectrum entries
+  const bool own = q.a1 && r < nrows;   // this thread owns elements of the output
   T acc[ENERGY ? 1 : NO][EPT];
 #pragma unroll
   for (int o = 0; o < (ENERGY ? 1 : NO); ++o)
@@ -584,22 +600,22 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX, (rows_inv_min_ctas<T,
     };
     if constexpr (PREFETCH) load_fac();
     T2 X[R2];
-    if (j < R1) {
-      const T2* src = S1 + (int64_t)p * nrows * M + r * M + j;
+    if (q.a2) {
+      const T2* src = S1 + (int64_t)p * nrows * M + rk * M + q.k1;
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2) {
-        if (r < nrows) X[k2] = src[R1 * k2];
+        if (rk < nrows) X[k2] = src[R1 * k2];
         else X[k2].x = X[k2].y = 0;
       }
     }
     if (p == 0) twp.store(tws);
     __syncthreads();   // tws is visible; the previous field's stage-B reads of buf are done
-    if (j < R1) row_inv_stageA<T2, R1, R2>(buf, line, j, tws, X);
+    if (q.a2) row_inv_stageA<T2, R1, R2>(buf, q.l2, q.k1, tws, X);
     __syncthreads();
     if (own) {
       if constexpr (!PREFETCH) load_fac();
       T2 w[R1];
-      row_inv_stageB<T2, R1, R2>(buf, line, j, w);
+      row_inv_stageB<T2, R1, R2>(buf, q.l1, j, w);
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const int64_t gi = r * N + j + R2 * e;
@@ -674,32 +690,34 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   const int p = blockIdx.y;
   const PartDesc& pd = args.f[f0 + p].p[0];
   const int64_t npair = (int64_t)N * N / 2;
-  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
-  const int64_t l = (int64_t)blockIdx.x * L + line;
-  const bool live = l < npair;
+  const RowMap<R1, R2, L> q;
+  const int64_t l0 = (int64_t)blockIdx.x * L;
   const T* a = reinterpret_cast<const T*>(args.in[pd.a]);
   const T* b = pd.b >= 0 ? reinterpret_cast<const T*>(args.in[pd.b]) : nullptr;
   T2 v[R1];
-  if (j < R2) {
+  if (q.a1) {
+    const bool live = l0 + q.l1 < npair;
 #pragma unroll
     for (int n1 = 0; n1 < R1 / 2; ++n1) {
-      const int64_t gi = 2 * l * N + R2 * n1 + j;
+      const int64_t gi = 2 * (l0 + q.l1) * N + R2 * n1 + q.n2;
       v[n1].x = live ? (T)0.5 * part_density(a, b, gi) : (T)0;
       v[n1].y = live ? (T)0.5 * part_density(a, b, gi + N) : (T)0;
     }
   }
   twp.store(tws);
-  if (j < R2) row_fwd_stage1<T2, R1, R2, true>(buf, line, j, v);
+  if (q.a1) row_fwd_stage1<T2, R1, R2, true>(buf, q.l1, q.n2, v);
   __syncthreads();
   T2 X[R2];
-  if (j < R1) row_fwd_stage2<T2, R1, R2>(buf, line, j, tws, X);
+  if (q.a2) row_fwd_stage2<T2, R1, R2>(buf, q.l2, q.k1, tws, X);
   __syncthreads();   // stage-2 reads of buf are complete
-  if (j < R1) {
+  if (q.a2) {
 #pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) buf[line * LS + j + R1 * k2] = X[k2];
+    for (int k2 = 0; k2 < R2; ++k2) buf[q.l2 * LS + q.k1 + R1 * k2] = X[k2];
   }
   __syncthreads();
-  if (!live) return;
+  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
+  const int64_t l = l0 + line;
+  if (l >= npair) return;
   T2* d = S1 + ((int64_t)p * N * N + 2 * l) * M;
   for (int k = j; k <= N; k += RM) {
     const T2 z = buf[line * LS + k], c = buf[line * LS + (k == 0 ? 0 : M - k)];
@@ -728,15 +746,15 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
   const int p = blockIdx.y;
   const int64_t npair = (int64_t)N * N / 2;
-  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
-  const int64_t l = (int64_t)blockIdx.x * L + line;
-  const bool live = l < npair;
+  const RowMap<R1, R2, L> q;
+  const int64_t l0 = (int64_t)blockIdx.x * L;
   T2 X[R2];
-  if (j < R1) {
-    const T2* A = S1 + ((int64_t)p * N * N + 2 * l) * M;
+  if (q.a2) {
+    const bool live = l0 + q.l2 < npair;
+    const T2* A = S1 + ((int64_t)p * N * N + 2 * (l0 + q.l2)) * M;
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) {
-      const int k = j + R1 * k2;
+      const int k = q.k1 + R1 * k2;
       const bool up = k > N;
       T2 a, b;
       a.x = a.y = b.x = b.y = 0;
@@ -750,12 +768,13 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   }
   twp.store(tws);
   __syncthreads();
-  if (j < R1) row_inv_stageA<T2, R1, R2>(buf, line, j, tws, X);
+  if (q.a2) row_inv_stageA<T2, R1, R2>(buf, q.l2, q.k1, tws, X);
   __syncthreads();
-  if (j >= R2 || !live) return;
+  const int64_t l = l0 + q.l1;
+  if (!q.a1 || l >= npair) return;
   T2 w[R1];
-  row_inv_stageB<T2, R1, R2>(buf, line, j, w);
-  const int64_t g0 = 2 * l * N + j;
+  row_inv_stageB<T2, R1, R2>(buf, q.l1, q.n2, w);
+  const int64_t g0 = 2 * l * N + q.n2;
   if constexpr (J) {
     T* o = reinterpret_cast<T*>(args.jbase) + (int64_t)(2 * (f0 + p)) * args.jstride + g0;
 #pragma unroll
@@ -798,25 +817,25 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
   const int p = blockIdx.y;
   const int64_t nrows = (int64_t)N * N;
-  const int line = threadIdx.x / RM, j = threadIdx.x % RM;
-  const int64_t r = (int64_t)blockIdx.x * L + line;
+  const RowMap<R1, R2, L> q;
+  const int64_t r = (int64_t)blockIdx.x * L + q.l1, rk = (int64_t)blockIdx.x * L + q.l2;
   T2 X[R2];
-  if (j < R1) {
-    const T2* src = S1 + (int64_t)p * nrows * M + r * M + j;
+  if (q.a2) {
+    const T2* src = S1 + (int64_t)p * nrows * M + rk * M + q.k1;
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) {
-      if (r < nrows) X[k2] = src[R1 * k2];
+      if (rk < nrows) X[k2] = src[R1 * k2];
       else X[k2].x = X[k2].y = 0;
     }
   }
   twp.store(tws);
   __syncthreads();
-  if (j < R1) row_inv_stageA<T2, R1, R2>(buf, line, j, tws, X);
+  if (q.a2) row_inv_stageA<T2, R1, R2>(buf, q.l2, q.k1, tws, X);
   __syncthreads();
-  if (j < R2 && r < nrows) {
+  if (q.a1 && r < nrows) {
     T2 w[R1];
-    row_inv_stageB<T2, R1, R2>(buf, line, j, w);
-    T* jre = jbase + (int64_t)(2 * (f0 + p)) * jstride + r * N + j;
+    row_inv_stageB<T2, R1, R2>(buf, q.l1, q.n2, w);
+    T* jre = jbase + (int64_t)(2 * (f0 + p)) * jstride + r * N + q.n2;
     T* jim = jre + jstride;
 #pragma unroll
     for (int n1 = 0; n1 < R1 / 2; ++n1) {
@@ -839,14 +858,12 @@ struct Launch {
   static constexpr int TWN = R1 * TwRow<T2, R2>::S;   // stage-twiddle table entries
   static size_t sm_cols() { return (size_t)(M * (L + 1) + TWN) * sizeof(T2); }
   static size_t sm_rows() { return (size_t)(L * RowBuf<R1, R2>::LS + TWN) * sizeof(T2); }
+  // Whole tiles only where L divides the M columns (the callers pass all of them, or a multiple of L
+  // that is at most M).
+  static constexpr bool FULL = M % L == 0;
   static int cols(int mode, const T2* in, T2* out, const ColGeom& g, int outer, int nf, const T2* tw,
                   const T* ghat, int H, cudaStream_t s) {
-    if (g.ncols % L == 0) return cols_t<true>(mode, in, out, g, outer, nf, tw, ghat, H, s);
-    return cols_t<false>(mode, in, out, g, outer, nf, tw, ghat, H, s);
-  }
-  template <bool FULL>
-  static int cols_t(int mode, const T2* in, T2* out, const ColGeom& g, int outer, int nf, const T2* tw,
-                    const T* ghat, int H, cudaStream_t s) {
+    if (FULL && g.ncols % L != 0) return fail(GATO_EUNSUPPORTED, "column pass: whole tiles of %d columns", L);
     dim3 grid(outer, (g.ncols + L - 1) / L, nf);
     const size_t sm = sm_cols();
     if (mode == COL_FWD) {
@@ -866,13 +883,8 @@ struct Launch {
                      const FeArgs& fa, cudaStream_t s) {
     dim3 grid(outer, (g.ncols + L - 1) / L, nf);
     const size_t sm = sm_cols();
-    if (g.ncols % L == 0) {
-      GATO_TRY(smem_attr(k_cols_fe<T, R1, R2, L, true>, sm));
-      k_cols_fe<T, R1, R2, L, true><<<grid, NT, sm, s>>>(in, g, tw, ghat, H, fa);
-    } else {
-      GATO_TRY(smem_attr(k_cols_fe<T, R1, R2, L, false>, sm));
-      k_cols_fe<T, R1, R2, L, false><<<grid, NT, sm, s>>>(in, g, tw, ghat, H, fa);
-    }
+    GATO_TRY(smem_attr(k_cols_fe<T, R1, R2, L, FULL>, sm));
+    k_cols_fe<T, R1, R2, L, FULL><<<grid, NT, sm, s>>>(in, g, tw, ghat, H, fa);
     GATO_LAUNCH_TRY();
     return GATO_OK;
   }

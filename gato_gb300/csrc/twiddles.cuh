@@ -78,6 +78,36 @@ template <> struct TwC<8> {
     }
   }
 };
+template <> struct TwC<9> {
+  __host__ __device__ static constexpr double c(int e) {
+    switch (e) {
+      case 0: return 1.0;
+      case 1: return 0.766044443118978;
+      case 2: return 0.17364817766693036;
+      case 3: return -0.5;
+      case 4: return -0.9396926207859084;
+      case 5: return -0.9396926207859084;
+      case 6: return -0.5;
+      case 7: return 0.17364817766693036;
+      case 8: return 0.766044443118978;
+      default: return 0.0;
+    }
+  }
+  __host__ __device__ static constexpr double s(int e) {
+    switch (e) {
+      case 0: return 0.0;
+      case 1: return 0.6427876096865394;
+      case 2: return 0.984807753012208;
+      case 3: return 0.8660254037844386;
+      case 4: return 0.3420201433256687;
+      case 5: return -0.3420201433256687;
+      case 6: return -0.8660254037844386;
+      case 7: return -0.984807753012208;
+      case 8: return -0.6427876096865394;
+      default: return 0.0;
+    }
+  }
+};
 template <> struct TwC<10> {
   __host__ __device__ static constexpr double c(int e) {
     switch (e) {
@@ -226,6 +256,54 @@ template <> struct TwC<16> {
       case 13: return -0.9238795325112867;
       case 14: return -0.7071067811865476;
       case 15: return -0.3826834323650898;
+      default: return 0.0;
+    }
+  }
+};
+template <> struct TwC<18> {
+  __host__ __device__ static constexpr double c(int e) {
+    switch (e) {
+      case 0: return 1.0;
+      case 1: return 0.9396926207859084;
+      case 2: return 0.766044443118978;
+      case 3: return 0.5;
+      case 4: return 0.17364817766693036;
+      case 5: return -0.17364817766693036;
+      case 6: return -0.5;
+      case 7: return -0.766044443118978;
+      case 8: return -0.9396926207859084;
+      case 9: return -1.0;
+      case 10: return -0.9396926207859084;
+      case 11: return -0.766044443118978;
+      case 12: return -0.5;
+      case 13: return -0.17364817766693036;
+      case 14: return 0.17364817766693036;
+      case 15: return 0.5;
+      case 16: return 0.766044443118978;
+      case 17: return 0.9396926207859084;
+      default: return 0.0;
+    }
+  }
+  __host__ __device__ static constexpr double s(int e) {
+    switch (e) {
+      case 0: return 0.0;
+      case 1: return 0.3420201433256687;
+      case 2: return 0.6427876096865394;
+      case 3: return 0.8660254037844386;
+      case 4: return 0.984807753012208;
+      case 5: return 0.984807753012208;
+      case 6: return 0.8660254037844386;
+      case 7: return 0.6427876096865394;
+      case 8: return 0.3420201433256687;
+      case 9: return 0.0;
+      case 10: return -0.3420201433256687;
+      case 11: return -0.6427876096865394;
+      case 12: return -0.8660254037844386;
+      case 13: return -0.984807753012208;
+      case 14: return -0.984807753012208;
+      case 15: return -0.8660254037844386;
+      case 16: return -0.6427876096865394;
+      case 17: return -0.3420201433256687;
       default: return 0.0;
     }
   }

@@ -13,7 +13,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 TOL = {torch.float64: 100 * 2.0 ** -53, torch.float32: 100 * 2.0 ** -24}
-SIZES = [16, 24, 32, 40, 48, 64, 80, 96, 128, 160]   # every register shape, the packed ones among them
+# every register shape, the packed ones among them
+SIZES = [16, 18, 20, 24, 28, 30, 32, 36, 40, 42, 48, 50, 54, 56, 60, 64, 70, 72, 80, 84, 90, 96, 98, 100, 108, 112,
+         120, 126, 128, 140, 144, 160]
 
 
 def rel(a, b):
@@ -55,8 +57,20 @@ def test_hartree(N, dtype):
     assert rel(got, ref) < TOL[dtype]
 
 
+@pytest.mark.parametrize("N", SIZES)
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+def test_every_shape_solves_pairs(N, dtype):
+    """Two fields of two pair densities (the multi-field z forward) on every register shape."""
+    from gato_gb300.solvers.poisson import PoissonPlan
+    h = 10.0 / N
+    plan = PoissonPlan(N, h, h / 2, dtype, 2)
+    orb, psi = smooth(4, N, N + 1, dtype), smooth(1, N, 5, dtype)[0]
+    got, ref = both(plan, lambda: plan.exchange_into(psi, orb, torch.zeros_like(psi)))
+    assert rel(got, ref) < TOL[dtype]
+
+
 @pytest.mark.parametrize("n", [1, 2, 3])
-@pytest.mark.parametrize("N", [24, 40, 64, 96])
+@pytest.mark.parametrize("N", [24, 40, 50, 64, 96])
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
 def test_exchange_block_and_energy(N, n, dtype):
     from gato_gb300.grid import Grid3D
