@@ -33,21 +33,73 @@ __device__ __forceinline__ double axis_coord(int i, double L, double h) {
   return -L / 2 + (i + 0.5) * h;  // grid.py:44
 }
 
-template <typename T>
-__global__ void k_softened(T* V, int N, double L, double h, AtomTable at, double eps) {
-  const int64_t n3 = (int64_t)N * N * N;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n3;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int z = (int)(i % N), y = (int)((i / N) % N), x = (int)(i / ((int64_t)N * N));
-    const double X = axis_coord(x, L, h), Y = axis_coord(y, L, h), Zc = axis_coord(z, L, h);
-    double v = 0.0;
-    for (int k = 0; k < at.K; ++k) {
-      const double dx = X - at.x[k], dy = Y - at.y[k], dz = Zc - at.z[k];
-      v += -at.Z[k] / sqrt(dx * dx + dy * dy + dz * dz + eps * eps);
+// Grid-stride walk over the N^3 points with the indices carried along: one add and compare per axis
+// and step instead of two divisions by N per point.
+struct PointWalk {
+  int x, y, z;
+  int64_t i;
+  int sx, sy, sz;
+  int64_t stride;
+  __device__ __forceinline__ explicit PointWalk(int N) {
+    i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    stride = (int64_t)gridDim.x * blockDim.x;
+    split(i, N, x, y, z);
+    split(stride, N, sx, sy, sz);
+  }
+  __device__ static __forceinline__ void split(int64_t v, int N, int& x, int& y, int& z) {
+    const int64_t r = v / N;
+    z = (int)(v - r * N);
+    x = (int)(r / N);
+    y = (int)(r - (int64_t)x * N);
+  }
+  __device__ __forceinline__ void next(int N) {
+    i += stride;
+    z += sz;
+    y += sy;
+    x += sx;
+    if (z >= N) {
+      z -= N;
+      ++y;
     }
-    V[i] = (T)v;
+    if (y >= N) {
+      y -= N;
+      ++x;
+    }
+  }
+};
+
+// The three axes' coordinates relative to a centre, d[axis * N + i] = (T)(x_i - R_axis), formed in FP64
+// once per block: per point they would be nine FP64 operations on GB300's narrow pipe (the FP32 force
+// integral over 128^3 points spent 180 of its 212 us on them).
+template <typename T>
+__device__ __forceinline__ void axis_table(T* d, int N, double L, double h, double rx, double ry, double rz) {
+  for (int t = threadIdx.x; t < 3 * N; t += blockDim.x) {
+    const int ax = t / N, i = t - ax * N;
+    d[t] = (T)(axis_coord(i, L, h) - (ax == 0 ? rx : (ax == 1 ? ry : rz)));
   }
 }
+
+template <typename T>
+__global__ void k_softened(T* V, int N, double L, double h, AtomTable at, double eps) {
+  extern __shared__ double ctab[];   // x_i of one axis (the axes agree)
+  for (int i = threadIdx.x; i < N; i += blockDim.x) ctab[i] = axis_coord(i, L, h);
+  __syncthreads();
+  const int64_t n3 = (int64_t)N * N * N;
+  for (PointWalk w(N); w.i < n3; w.next(N)) {
+    double v = 0.0;
+    for (int k = 0; k < at.K; ++k) {
+      const double dx = ctab[w.x] - at.x[k], dy = ctab[w.y] - at.y[k], dz = ctab[w.z] - at.z[k];
+      v += -at.Z[k] / sqrt(dx * dx + dy * dy + dz * dz + eps * eps);
+    }
+    V[w.i] = (T)v;
+  }
+}
+
+// From 8 sqrt(2) r_loc outwards erf(r / (sqrt(2) r_loc)) is 1 in FP64 and exp(-r^2 / (2 r_loc^2)) < 2e-28
+// is far below the last bit of anything it is added to: only the Coulomb tail is left there. That is
+// all but a sphere of 2 to 9 bohr around each centre, and the erf, the exp and the divisions are most
+// of the FP64 work (64^3 water, V_loc: 180 -> 50 us; its force integral 304 -> 73).
+constexpr double kFar = 8.0 * 1.4142135623730951;
 
 // V_loc of one centre at distance r (pseudopotentials.py:214-227).
 __device__ __forceinline__ double hgh_vloc(double r, double Z, double rloc, const double* c) {
@@ -60,18 +112,19 @@ __device__ __forceinline__ double hgh_vloc(double r, double Z, double rloc, cons
 
 template <typename T>
 __global__ void k_hgh_local(T* V, int N, double L, double h, AtomTable at) {
+  extern __shared__ double ctab[];
+  for (int i = threadIdx.x; i < N; i += blockDim.x) ctab[i] = axis_coord(i, L, h);
+  __syncthreads();
   const int64_t n3 = (int64_t)N * N * N;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n3;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int z = (int)(i % N), y = (int)((i / N) % N), x = (int)(i / ((int64_t)N * N));
-    const double X = axis_coord(x, L, h), Y = axis_coord(y, L, h), Zc = axis_coord(z, L, h);
+  for (PointWalk w(N); w.i < n3; w.next(N)) {
     double v = 0.0;
     for (int k = 0; k < at.K; ++k) {
-      const double dx = X - at.x[k], dy = Y - at.y[k], dz = Zc - at.z[k];
-      const double r = sqrt(dx * dx + dy * dy + dz * dz + 1e-30);
-      v += hgh_vloc(r, at.Z[k], at.rloc[k], at.c[k]);
+      const double dx = ctab[w.x] - at.x[k], dy = ctab[w.y] - at.y[k], dz = ctab[w.z] - at.z[k];
+      const double r2 = dx * dx + dy * dy + dz * dz + 1e-30, rf = kFar * at.rloc[k];
+      if (r2 > rf * rf) v -= at.Z[k] * rsqrt(r2);
+      else v += hgh_vloc(sqrt(r2), at.Z[k], at.rloc[k], at.c[k]);
     }
-    V[i] = (T)v;
+    V[w.i] = (T)v;
   }
 }
 
@@ -96,28 +149,51 @@ __device__ __forceinline__ R hgh_dvloc_dr(R r, R Z, R rloc, const double* c) {
   return d_erf + exp((R)-0.5 * rho2) * ((R)-0.5 * poly + dpoly) * drho2;
 }
 
-// partials[(k*3 + c) * nblk + block] = sum rho * dV_k/dR_c.
+// |d|^2 + e with the two adds fused into multiply-adds in a fixed order (FP32 force integrals keep their bits).
+template <typename T>
+__device__ __forceinline__ T norm2(T dx, T dy, T dz, T e) {
+  return fma(dz, dz, fma(dy, dy, dx * dx)) + e;
+}
+
+// rho dV_k/dR is w d with w = -rho (dV/dr) / r; in the far region (kFar; FP32: 6 sqrt(2) r_loc, where
+// erf is 1 and the exponentials are below 2^-30 of the rest) dV/dr = Z / r^2.
+template <typename T>
+__device__ __forceinline__ T local_grad_weight(T rho, T r2, T far2, T Z, T rloc, const double* c) {
+  if (r2 > far2) {
+    if constexpr (sizeof(T) == 8) {
+      const double ri = rsqrt(r2);
+      return -rho * Z * (ri * ri * ri);
+    } else {
+      const T r = sqrt(r2);
+      return -rho * (Z * ((T)1 / (r * r))) / r;
+    }
+  }
+  const T r = sqrt(r2);
+  const T dv = hgh_dvloc_dr<T>(r, Z, rloc, c);
+  return -rho * dv / r;   // dV/dR = dV/dr * (-(x - R)/r)
+}
+
+// partials[(k*3 + c) * gridDim.x + block] = sum rho * dV_k/dR_c, centre k = blockIdx.y (the centres side
+// by side keep more warps on the long square root and division chains than a loop over them).
 template <typename T>
 __global__ void k_local_grad(const T* __restrict__ rho, int N, double L, double h, AtomTable at,
                              double* partials) {
+  extern __shared__ double ctab[];
   __shared__ double sh[32];
+  T* d = reinterpret_cast<T*>(ctab);
   const int64_t n3 = (int64_t)N * N * N;
-  for (int k = 0; k < at.K; ++k) {
+  {
+    const int k = blockIdx.y;
+    axis_table(d, N, L, h, at.x[k], at.y[k], at.z[k]);
+    __syncthreads();
+    const T rf = (T)((sizeof(T) == 8 ? kFar : 0.75 * kFar) * at.rloc[k]), far2 = rf * rf;
     Acc<T> g[3];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n3;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      const int z = (int)(i % N), y = (int)((i / N) % N), x = (int)(i / ((int64_t)N * N));
-      const double dxd = axis_coord(x, L, h) - at.x[k];
-      const double dyd = axis_coord(y, L, h) - at.y[k];
-      const double dzd = axis_coord(z, L, h) - at.z[k];
-      const T dx = (T)dxd, dy = (T)dyd, dz = (T)dzd;
-      const T r = sqrt(dx * dx + dy * dy + dz * dz + (T)1e-30);
-      const T dv = hgh_dvloc_dr<T>(r, (T)at.Z[k], (T)at.rloc[k], at.c[k]);
-      // dV/dR = dV/dr * (-(x - R)/r)
-      const T w = -rho[i] * dv / r;
-      g[0].add_prod(w, dx);
-      g[1].add_prod(w, dy);
-      g[2].add_prod(w, dz);
+    for (PointWalk w(N); w.i < n3; w.next(N)) {
+      const T dx = d[w.x], dy = d[N + w.y], dz = d[2 * N + w.z];
+      const T wt = local_grad_weight<T>(rho[w.i], norm2(dx, dy, dz, (T)1e-30), far2, (T)at.Z[k], (T)at.rloc[k], at.c[k]);
+      g[0].add_prod(wt, dx);
+      g[1].add_prod(wt, dy);
+      g[2].add_prod(wt, dz);
     }
     for (int cc = 0; cc < 3; ++cc) {
       const double v = block_sum(g[cc].value(), sh);
@@ -131,22 +207,23 @@ __global__ void k_local_grad(const T* __restrict__ rho, int N, double L, double 
 template <typename T>
 __global__ void k_softened_grad(const T* __restrict__ rho, int N, double L, double h, AtomTable at,
                                 double eps, double* partials) {
+  extern __shared__ double ctab[];
   __shared__ double sh[32];
+  T* d = reinterpret_cast<T*>(ctab);
   const int64_t n3 = (int64_t)N * N * N;
   const T e2 = (T)(eps * eps);
-  for (int k = 0; k < at.K; ++k) {
+  {
+    const int k = blockIdx.y;
+    axis_table(d, N, L, h, at.x[k], at.y[k], at.z[k]);
+    __syncthreads();
     Acc<T> g[3];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n3;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      const int z = (int)(i % N), y = (int)((i / N) % N), x = (int)(i / ((int64_t)N * N));
-      const T dx = (T)(axis_coord(x, L, h) - at.x[k]);
-      const T dy = (T)(axis_coord(y, L, h) - at.y[k]);
-      const T dz = (T)(axis_coord(z, L, h) - at.z[k]);
-      const T u = dx * dx + dy * dy + dz * dz + e2;
-      const T w = -(T)at.Z[k] * rho[i] / (u * sqrt(u));
-      g[0].add_prod(w, dx);
-      g[1].add_prod(w, dy);
-      g[2].add_prod(w, dz);
+    for (PointWalk w(N); w.i < n3; w.next(N)) {
+      const T dx = d[w.x], dy = d[N + w.y], dz = d[2 * N + w.z];
+      const T u = norm2(dx, dy, dz, e2);
+      const T wt = -(T)at.Z[k] * rho[w.i] / (u * sqrt(u));
+      g[0].add_prod(wt, dx);
+      g[1].add_prod(wt, dy);
+      g[2].add_prod(wt, dz);
     }
     for (int cc = 0; cc < 3; ++cc) {
       const double v = block_sum(g[cc].value(), sh);
@@ -201,25 +278,34 @@ __device__ __forceinline__ void angular_grad(int ell, int m, double hx, double h
   }
 }
 
+// r^n for the whole powers 0 .. 6 of the radial parts, r2 = r^2 (pow() is some hundred FP64
+// operations: the projector-force kernel of a 128^3 water took 30 us, 11 without it).
+__device__ __forceinline__ double rpow(double r, double r2, int n) {
+  double v = n & 1 ? r : 1.0;
+  for (int k = n >> 1; k > 0; --k) v *= r2;
+  return v;
+}
+
 // p(d) of pseudopotentials.py:265-327, r = sqrt(|d|^2 + 1e-30), hat = d / r.
 __device__ __forceinline__ double proj_value(const ProjParams& p, double dx, double dy, double dz) {
-  const double r = sqrt(dx * dx + dy * dy + dz * dz + 1e-30);
-  const double radial = p.norm * pow(r, (double)p.power) * exp(-(r * r) / (2.0 * p.r * p.r));
-  return radial * angular(p.ell, p.m, dx / r, dy / r, dz / r);
+  const double r2 = dx * dx + dy * dy + dz * dz + 1e-30, r = sqrt(r2);
+  const double radial = p.norm * rpow(r, r2, p.power) * exp(-r2 / (2.0 * p.r * p.r));
+  const double ri = 1.0 / r;
+  return radial * angular(p.ell, p.m, dx * ri, dy * ri, dz * ri);
 }
 
 __device__ __forceinline__ void proj_grad(const ProjParams& p, double dx, double dy, double dz,
                                           double* g) {
-  const double r = sqrt(dx * dx + dy * dy + dz * dz + 1e-30);
-  const double R = p.norm * pow(r, (double)p.power) * exp(-(r * r) / (2.0 * p.r * p.r));
-  const double hx = dx / r, hy = dy / r, hz = dz / r;
-  const double Y = angular(p.ell, p.m, hx, hy, hz);
+  const double r2 = dx * dx + dy * dy + dz * dz + 1e-30, r = sqrt(r2), ri = 1.0 / r;
+  const double is2 = 1.0 / (p.r * p.r);
+  const double R = p.norm * rpow(r, r2, p.power) * exp(-0.5 * r2 * is2);
+  const double hat[3] = {dx * ri, dy * ri, dz * ri};
+  const double Y = angular(p.ell, p.m, hat[0], hat[1], hat[2]);
   double gY[3];
-  angular_grad(p.ell, p.m, hx, hy, hz, gY);
-  const double dRr = (p.power / r - r / (p.r * p.r)) * Y;
-  const double d[3] = {dx, dy, dz};
-  const double hd = gY[0] * hx + gY[1] * hy + gY[2] * hz;
-  for (int c = 0; c < 3; ++c) g[c] = R * (dRr * d[c] / r + (gY[c] - hd * d[c] / r) / r);
+  angular_grad(p.ell, p.m, hat[0], hat[1], hat[2], gY);
+  const double dRr = (p.power * ri - r * is2) * Y;
+  const double hd = gY[0] * hat[0] + gY[1] * hat[1] + gY[2] * hat[2];
+  for (int c = 0; c < 3; ++c) g[c] = R * (dRr * hat[c] + (gY[c] - hd * hat[c]) * ri);
 }
 
 template <typename T>
@@ -489,6 +575,12 @@ int make_atoms(AtomTable& at, int K, const double* pos, const double* Z, const d
   return GATO_OK;
 }
 
+// Shared memory for the coordinate tables of a potential or force kernel (a few KB; large grids opt in).
+int table_limit(const void* fn, size_t bytes) {
+  if (bytes > 200 * 1024) return fail(GATO_EUNSUPPORTED, "potential: grid too large for the coordinate table");
+  return bytes > 48 * 1024 ? raise_smem_limit(fn, bytes) : GATO_OK;
+}
+
 ProjParams proj_params(const Nonlocal& nl, const NlProj& p) {
   const NlChannel& ch = nl.ch[p.chan];
   ProjParams pp;
@@ -588,8 +680,10 @@ extern "C" int gato_softened_coulomb(int dtype, void* V, int N, double L, int K,
   cudaStream_t s = as_stream(stream);
   const double h = L / N;
   const int64_t n3 = (int64_t)N * N * N;
-  if (dtype == GATO_F64) k_softened<double><<<grid_for(n3, 256), 256, 0, s>>>((double*)V, N, L, h, at, eps);
-  else k_softened<float><<<grid_for(n3, 256), 256, 0, s>>>((float*)V, N, L, h, at, eps);
+  const size_t ctab = (size_t)N * sizeof(double);
+  GATO_TRY(table_limit(dtype == GATO_F64 ? (const void*)k_softened<double> : (const void*)k_softened<float>, ctab));
+  if (dtype == GATO_F64) k_softened<double><<<grid_for(n3, 256), 256, ctab, s>>>((double*)V, N, L, h, at, eps);
+  else k_softened<float><<<grid_for(n3, 256), 256, ctab, s>>>((float*)V, N, L, h, at, eps);
   GATO_LAUNCH_TRY();
   return GATO_OK;
 }
@@ -604,8 +698,10 @@ extern "C" int gato_hgh_local(int dtype, void* V, int N, double L, int K, const 
   cudaStream_t s = as_stream(stream);
   const double h = L / N;
   const int64_t n3 = (int64_t)N * N * N;
-  if (dtype == GATO_F64) k_hgh_local<double><<<grid_for(n3, 256), 256, 0, s>>>((double*)V, N, L, h, at);
-  else k_hgh_local<float><<<grid_for(n3, 256), 256, 0, s>>>((float*)V, N, L, h, at);
+  const size_t ctab = (size_t)N * sizeof(double);
+  GATO_TRY(table_limit(dtype == GATO_F64 ? (const void*)k_hgh_local<double> : (const void*)k_hgh_local<float>, ctab));
+  if (dtype == GATO_F64) k_hgh_local<double><<<grid_for(n3, 256), 256, ctab, s>>>((double*)V, N, L, h, at);
+  else k_hgh_local<float><<<grid_for(n3, 256), 256, ctab, s>>>((float*)V, N, L, h, at);
   GATO_LAUNCH_TRY();
   return GATO_OK;
 }
@@ -625,8 +721,10 @@ extern "C" int gato_hgh_local_grad(int dtype, const void* rho, int N, double L, 
   double* part = (double*)stream_scratch(s, (size_t)(3 * K * nblk + 3 * K) * sizeof(double));
   if (!part) return fail(GATO_ENOMEM, "scratch");
   double* res = part + 3 * K * nblk;
-  if (dtype == GATO_F64) k_local_grad<double><<<nblk, 256, 0, s>>>((const double*)rho, N, L, h, at, part);
-  else k_local_grad<float><<<nblk, 256, 0, s>>>((const float*)rho, N, L, h, at, part);
+  const size_t ctab = (size_t)3 * N * (dtype == GATO_F64 ? 8 : 4);
+  GATO_TRY(table_limit(dtype == GATO_F64 ? (const void*)k_local_grad<double> : (const void*)k_local_grad<float>, ctab));
+  if (dtype == GATO_F64) k_local_grad<double><<<dim3(nblk, K), 256, ctab, s>>>((const double*)rho, N, L, h, at, part);
+  else k_local_grad<float><<<dim3(nblk, K), 256, ctab, s>>>((const float*)rho, N, L, h, at, part);
   GATO_LAUNCH_TRY();
   GATO_TRY(finalize_sums(part, 3 * K, nblk, h * h * h, res, s));
   std::vector<double> g(3 * K);
@@ -649,10 +747,13 @@ extern "C" int gato_softened_coulomb_grad(int dtype, const void* rho, int N, dou
   double* part = (double*)stream_scratch(s, (size_t)(3 * K * nblk + 3 * K) * sizeof(double));
   if (!part) return fail(GATO_ENOMEM, "scratch");
   double* res = part + 3 * K * nblk;
+  const size_t ctab = (size_t)3 * N * (dtype == GATO_F64 ? 8 : 4);
+  GATO_TRY(table_limit(dtype == GATO_F64 ? (const void*)k_softened_grad<double> : (const void*)k_softened_grad<float>,
+                       ctab));
   if (dtype == GATO_F64)
-    k_softened_grad<double><<<nblk, 256, 0, s>>>((const double*)rho, N, L, h, at, eps, part);
+    k_softened_grad<double><<<dim3(nblk, K), 256, ctab, s>>>((const double*)rho, N, L, h, at, eps, part);
   else
-    k_softened_grad<float><<<nblk, 256, 0, s>>>((const float*)rho, N, L, h, at, eps, part);
+    k_softened_grad<float><<<dim3(nblk, K), 256, ctab, s>>>((const float*)rho, N, L, h, at, eps, part);
   GATO_LAUNCH_TRY();
   GATO_TRY(finalize_sums(part, 3 * K, nblk, h * h * h, res, s));
   std::vector<double> g(3 * K);
