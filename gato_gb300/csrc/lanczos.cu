@@ -644,15 +644,16 @@ __global__ void k_scale_copy(const T* __restrict__ src, T* dst, int64_t n, const
 // long. A zero minor takes the sign opposite to its predecessor (the LDL^T
 // form's q_i = 0 -> -pivmin convention), and the pair (p_i, p_{i-1}) is
 // rescaled by an exact power of two whenever p_i's exponent leaves [-480, 480].
-__device__ int sturm_count(const double* a, const double* e2, int m, double x) {
-  auto neg = [](double v, bool prev_neg) {
-    const int hi = __double2hiint(v);
-    const bool zero = ((hi & 0x7fffffff) | __double2loint(v)) == 0;
-    return zero ? !prev_neg : hi < 0;
-  };
+// The zero and exponent tests read the words of p (a compare would take the FP64 pipe). The exponent is
+// looked at every fourth step: four steps grow |p| by at most (2 nm)^4, so up to nm = 2^100 nothing
+// leaves the range in between; `wide` (nm beyond that) looks at every step.
+__device__ __forceinline__ int sturm_count(const double* a, const double* e2, int m, double x, bool wide) {
+  auto zero = [](double v) { return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0; };
+  auto neg = [&](double v, bool prev_neg) { return zero(v) ? !prev_neg : __double2hiint(v) < 0; };
   double pm = 1.0, p = a[0] - x;
   bool s = neg(p, false);
   int cnt = s;
+#pragma unroll 4
   for (int i = 1; i < m; ++i) {
     const double pn = fma(a[i] - x, p, -e2[i - 1] * pm);
     const bool sn = neg(pn, s);
@@ -660,13 +661,15 @@ __device__ int sturm_count(const double* a, const double* e2, int m, double x) {
     pm = p;
     p = pn;
     s = sn;
-    const int ex = (__double2hiint(p) >> 20) & 0x7ff;
-    if (ex > 1023 + 480) {
-      p *= 0x1p-480;
-      pm *= 0x1p-480;
-    } else if (ex < 1023 - 480 && p != 0.0) {
-      p *= 0x1p480;
-      pm *= 0x1p480;
+    if (wide || (i & 3) == 0) {
+      const int ex = (__double2hiint(p) >> 20) & 0x7ff;
+      if (ex > 1023 + 480) {
+        p *= 0x1p-480;
+        pm *= 0x1p-480;
+      } else if (ex < 1023 - 480 && !zero(p)) {
+        p *= 0x1p480;
+        pm *= 0x1p480;
+      }
     }
   }
   return cnt;
@@ -679,7 +682,7 @@ __device__ __forceinline__ void gershgorin(const double* a, const double* e, int
   lo = 1e300;
   hi = -1e300;
   nm = 0;
-  for (int i = threadIdx.x; i < m; i += 32) {
+  for (int i = threadIdx.x & 31; i < m; i += 32) {
     const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < m - 1 ? fabs(e[i]) : 0.0);
     lo = fmin(lo, a[i] - r);
     hi = fmax(hi, a[i] + r);
@@ -693,54 +696,58 @@ __device__ __forceinline__ void gershgorin(const double* a, const double* e, int
   }
 }
 
-// One warp per block, block k = eigenvalue k of T = diag(alpha) +
-// offdiag(beta[:m-1]) (ascending). Multisection on Sturm counts (33
-// sub-intervals a round), then inverse iteration: T - lambda_k I is factored
-// once with partial pivoting (the LAPACK dgttrf scheme: multipliers,
-// interchanges and reciprocal pivots kept in work) and the factors are applied
-// to the iterate four times (dgtts2). One eigenvalue per block spreads the FP64
-// work over K SMs: GB300's FP64 pipe is narrow, and a Sturm count is a chain
-// of m dependent FP64 divisions. The factorisation and the iterate live in shared memory (each
-// step of these sequential loops reads what the previous one wrote: in global memory every step
-// would wait on a round trip through L2); the final vector goes to work + k*7m + 6m. Dynamic
-// shared memory: a, e, e2 and d, du, du2, f, sw, rd, x, 10 m doubles.
-__global__ void __launch_bounds__(32) k_tridiag_eig(const double* alpha, const double* beta, int m, int K,
-                                                     double* lam_out, double* work, int* err) {
+// One block per eigenvalue, block k = eigenvalue k of T = diag(alpha) + offdiag(beta[:m-1]) (ascending).
+// Multisection on Sturm counts, then inverse iteration: T - lambda_k I is factored once with partial
+// pivoting (the LAPACK dgttrf scheme: multipliers, interchanges and reciprocal pivots) and the factors are
+// applied to the iterate four times (dgtts2). One eigenvalue per block spreads the FP64 work over K SMs.
+//
+// GB300's FP64 pipe takes 64 cycles of a scheduler per warp instruction, so a Sturm count, three
+// operations a row, is bound by that and not by latency: four warps, one per scheduler, take 129
+// sub-intervals a round (8 rounds to the last bit, 11 with one warp). What is elementwise (start vector,
+// reciprocals, scaled factors, norms, scaling) runs across the lanes of one warp; the chains that are
+// left, factorisation and the two substitutions, carry their value in registers at one multiply-add a
+// row (U is kept scaled by its reciprocal diagonal). m = 80: 531 us with one lane doing all of that
+// through shared memory, 220 us now. The final vector goes to work + k*7m + 6m. Dynamic shared
+// memory: a, e, e2 and d, du, du2, f, sw, rd, x, 10 m doubles.
+constexpr int kTriThreads = 128;
+__global__ void __launch_bounds__(kTriThreads) k_tridiag_eig(const double* alpha, const double* beta, int m, int K,
+                                                             double* lam_out, double* work, int* err) {
   extern __shared__ double sm[];
   double* a = sm;
   double* e = a + m;
   double* e2 = e + m;
-  const int lane = threadIdx.x, k = blockIdx.x;
-  for (int i = lane; i < m; i += 32) {
+  const int t = threadIdx.x, lane = t & 31, k = blockIdx.x;
+  for (int i = t; i < m; i += kTriThreads) {
     a[i] = alpha[i];
     e[i] = i < m - 1 ? beta[i] : 0.0;
     e2[i] = e[i] * e[i];
   }
-  __syncwarp();
+  __syncthreads();
   double glo, ghi, nm;
-  gershgorin(a, e, m, glo, ghi, nm);
+  gershgorin(a, e, m, glo, ghi, nm);   // every warp for itself, the same values
   const double pad = 2.2e-16 * nm * 4 + 1e-300;
   glo -= pad;
   ghi += pad;
   const double tnorm = nm > 0 ? nm : 1.0;
   const double pivmin = 1e-290 > 2.2e-16 * 2.2e-16 * tnorm ? 1e-290 : 1e-300;
+  const bool wide = !(nm < 0x1p100);
   double lo = glo, hi = ghi;
+  constexpr double kSec = kTriThreads + 1;
   for (int it = 0; it < 80; ++it) {
     const double width = hi - lo;
-    if (width <= 2.2e-16 * 2 * fmax(fabs(lo), fabs(hi)) + pivmin) break;
-    const double x = lo + width * (double)(lane + 1) / 33.0;
-    const int c = sturm_count(a, e2, m, x);
-    // bracket: eigenvalue k lies in [x_i, x_{i+1}) where count(x_i) <= k < count(x_{i+1})
-    const unsigned below = __ballot_sync(0xffffffffu, c <= k);   // lanes whose x is <= lambda_k
-    const int nb = __popc(below);  // counts are monotone: lanes 0..nb-1 have c <= k
-    const double nlo = nb > 0 ? lo + width * (double)nb / 33.0 : lo;
-    const double nhi = nb < 32 ? lo + width * (double)(nb + 1) / 33.0 : hi;
+    if (width <= 2.2e-16 * 2 * fmax(fabs(lo), fabs(hi)) + pivmin) break;   // the same in every thread
+    const double x = lo + width * (double)(t + 1) / kSec;
+    // bracket: eigenvalue k lies in [x_i, x_{i+1}) where count(x_i) <= k < count(x_{i+1}); the counts
+    // are monotone, so threads 0..nb-1 have count <= k
+    const int nb = __syncthreads_count(sturm_count(a, e2, m, x, wide) <= k);
+    const double nlo = nb > 0 ? lo + width * (double)nb / kSec : lo;
+    const double nhi = nb < kTriThreads ? lo + width * (double)(nb + 1) / kSec : hi;
     lo = nlo;
     hi = nhi;
   }
-  if (lane != 0) return;
+  if (t >= 32) return;
   const double shift = 0.5 * (lo + hi);
-  lam_out[k] = shift;
+  if (lane == 0) lam_out[k] = shift;
   double* d = e2 + m;
   double* du = d + m;
   double* du2 = du + m;
@@ -749,78 +756,106 @@ __global__ void __launch_bounds__(32) k_tridiag_eig(const double* alpha, const d
   double* rd = sw + m;     // 1 / d[i] of the final factor
   double* x = rd + m;
   const double tiny = 2.2e-16 * tnorm;
-  for (int i = 0; i < m; ++i) {
-    d[i] = a[i] - shift;
-    du[i] = e[i];
-    du2[i] = 0.0;
-  }
-  for (int i = 0; i < m - 1; ++i) {   // factor (dgttrf)
-    const double dli = e[i];
-    if (fabs(d[i]) >= fabs(dli)) {
-      if (d[i] == 0.0) d[i] = tiny;
-      f[i] = dli / d[i];
-      sw[i] = 0.0;
-      d[i + 1] -= f[i] * du[i];
-      du2[i] = 0.0;
-    } else {
-      f[i] = d[i] / dli;
-      sw[i] = 1.0;
-      d[i] = dli;
-      const double t = du[i];
-      du[i] = d[i + 1];
-      d[i + 1] = t - f[i] * d[i + 1];
-      if (i < m - 2) {
-        du2[i] = du[i + 1];
-        du[i + 1] = -f[i] * du[i + 1];
-      }
-    }
-  }
-  if (d[m - 1] == 0.0) d[m - 1] = tiny;
-  for (int i = 0; i < m; ++i) rd[i] = 1.0 / d[i];
-  for (int i = 0; i < m; ++i) x[i] = 1.0 + 0.25 * sin(0.7 * (i + 1) * (k + 1) + 0.3);   // start vector
-  for (int iter = 0; iter < 4; ++iter) {
-    for (int i = 0; i < m - 1; ++i) {   // forward: L^-1 P x
-      if (sw[i] == 0.0) {
-        x[i + 1] -= f[i] * x[i];
+  if (lane == 0) {   // factor (dgttrf): di, ui are the pivot row's entries, dn, un the next row's
+    double di = a[0] - shift, ui = e[0];
+    for (int i = 0; i < m - 1; ++i) {
+      const double dli = e[i], dn = a[i + 1] - shift, un = e[i + 1];
+      if (fabs(di) >= fabs(dli)) {
+        if (di == 0.0) di = tiny;
+        const double fi = dli / di;
+        f[i] = fi;
+        sw[i] = 0.0;
+        d[i] = di;
+        du[i] = ui;
+        du2[i] = 0.0;
+        di = dn - fi * ui;
+        ui = un;
       } else {
-        const double xt = x[i];
-        x[i] = x[i + 1];
-        x[i + 1] = xt - f[i] * x[i + 1];
+        const double fi = di / dli;
+        f[i] = fi;
+        sw[i] = 1.0;
+        d[i] = dli;
+        du[i] = dn;
+        du2[i] = i < m - 2 ? un : 0.0;
+        di = ui - fi * dn;
+        ui = -fi * un;
       }
     }
-    x[m - 1] *= rd[m - 1];   // back substitution with U (diagonal, du, du2)
-    if (m > 1) x[m - 2] = (x[m - 2] - du[m - 2] * x[m - 1]) * rd[m - 2];
-    for (int i = m - 3; i >= 0; --i) x[i] = (x[i] - du[i] * x[i + 1] - du2[i] * x[i + 2]) * rd[i];
+    if (di == 0.0) di = tiny;
+    d[m - 1] = di;
+    du[m - 1] = du2[m - 1] = 0.0;
+  }
+  __syncwarp();
+  for (int i = lane; i < m; i += 32) {
+    const double r = 1.0 / d[i];
+    rd[i] = r;
+    du[i] *= r;
+    du2[i] *= r;
+    x[i] = 1.0 + 0.25 * sin(0.7 * (i + 1) * (k + 1) + 0.3);   // start vector
+  }
+  __syncwarp();
+  for (int iter = 0; iter < 4; ++iter) {
+    if (lane == 0) {   // forward: L^-1 P x
+      double xc = x[0];
+#pragma unroll 4
+      for (int i = 0; i < m - 1; ++i) {
+        const double xn = x[i + 1];
+        const bool swap = sw[i] != 0.0;
+        const double up = swap ? xn : xc, lw = swap ? xc : xn;
+        x[i] = up;
+        xc = lw - f[i] * up;
+      }
+      x[m - 1] = xc;
+    }
+    __syncwarp();
+    for (int i = lane; i < m; i += 32) x[i] *= rd[i];
+    __syncwarp();
+    if (lane == 0) {   // back substitution with U scaled to a unit diagonal
+      double x1 = 0.0, x2 = 0.0;
+#pragma unroll 4
+      for (int i = m - 1; i >= 0; --i) {
+        const double xi = (x[i] - du2[i] * x2) - du[i] * x1;
+        x[i] = xi;
+        x2 = x1;
+        x1 = xi;
+      }
+    }
+    __syncwarp();
     double nrm = 0.0;
-    for (int i = 0; i < m; ++i) nrm += x[i] * x[i];
-    nrm = sqrt(nrm);
+    for (int i = lane; i < m; i += 32) nrm += x[i] * x[i];
+    nrm = sqrt(warp_sum(nrm));
     if (!(nrm > 0) || !isfinite(nrm)) {
-      if (err) atomicExch(err, 201);
+      if (lane == 0 && err) atomicExch(err, 201);
       nrm = 1.0;
     }
     const double inv = 1.0 / nrm;
-    for (int i = 0; i < m; ++i) x[i] *= inv;
+    for (int i = lane; i < m; i += 32) x[i] *= inv;
+    __syncwarp();
   }
   double* xo = work + (int64_t)k * 7 * m + 6 * m;   // read by k_tridiag_finish
-  for (int i = 0; i < m; ++i) xo[i] = x[i];
+  for (int i = lane; i < m; i += 32) xo[i] = x[i];
 }
 
 // Convergence flag (any beta_j < tol for j < max(m-1, 1), lanczos.py:199),
 // re-orthogonalisation of eigenvectors of clustered eigenvalues, and the sign
-// convention (largest component positive); writes evals and Y (column k at
-// Y + k*m). One thread: O(K^2 m) work at most.
-__global__ void k_tridiag_finish(const double* alpha, const double* beta, int m, int K, const double* lam,
-                                 double* work, double* evals, double* Y, int* flag, double tol) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int fl = 0;
+// convention (largest component positive, the first of equal ones); writes evals and Y (column k at
+// Y + k*m). One warp: O(K^2 m) work at most.
+__global__ void __launch_bounds__(32) k_tridiag_finish(const double* alpha, const double* beta, int m, int K,
+                                                       const double* lam, double* work, double* evals, double* Y,
+                                                       int* flag, double tol) {
+  const int lane = threadIdx.x;
   const int lim = m - 1 > 1 ? m - 1 : 1;
-  for (int j = 0; j < lim; ++j) fl |= beta[j] < tol;
-  flag[0] = fl;
+  bool fl = false;
+  for (int j = lane; j < lim; j += 32) fl |= beta[j] < tol;
+  fl = __any_sync(0xffffffffu, fl);
+  if (lane == 0) flag[0] = fl;
   double nm = 0;
-  for (int i = 0; i < m; ++i) {
+  for (int i = lane; i < m; i += 32) {
     const double r = (i > 0 ? fabs(beta[i - 1]) : 0.0) + (i < m - 1 ? fabs(beta[i]) : 0.0);
     nm = fmax(nm, fabs(alpha[i]) + r);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nm = fmax(nm, __shfl_xor_sync(0xffffffffu, nm, o));
   const double close = 1e-7 * (nm > 0 ? nm : 1.0);
   for (int k = 0; k < K; ++k) {
     double* xk = work + (int64_t)k * 7 * m + 6 * m;
@@ -828,19 +863,37 @@ __global__ void k_tridiag_finish(const double* alpha, const double* beta, int m,
       if (fabs(lam[k] - lam[l]) > close) continue;
       const double* xl = work + (int64_t)l * 7 * m + 6 * m;
       double dot = 0;
-      for (int i = 0; i < m; ++i) dot += xl[i] * xk[i];
-      for (int i = 0; i < m; ++i) xk[i] -= dot * xl[i];
+      for (int i = lane; i < m; i += 32) dot += xl[i] * xk[i];
+      dot = warp_sum(dot);
       double nrm = 0;
-      for (int i = 0; i < m; ++i) nrm += xk[i] * xk[i];
-      nrm = sqrt(nrm);
-      for (int i = 0; i < m; ++i) xk[i] /= nrm;
+      for (int i = lane; i < m; i += 32) {   // each lane reads and writes its own entries alone
+        const double v = xk[i] - dot * xl[i];
+        xk[i] = v;
+        nrm += v * v;
+      }
+      nrm = sqrt(warp_sum(nrm));
+      for (int i = lane; i < m; i += 32) xk[i] /= nrm;
     }
-    int imax = 0;
-    for (int i = 1; i < m; ++i)
-      if (fabs(xk[i]) > fabs(xk[imax])) imax = i;
-    const double sg = xk[imax] < 0 ? -1.0 : 1.0;
-    for (int i = 0; i < m; ++i) Y[(int64_t)k * m + i] = sg * xk[i];
-    evals[k] = lam[k];
+    double vmax = -1.0, sgn = 1.0;
+    int imax = m;
+    for (int i = lane; i < m; i += 32)
+      if (fabs(xk[i]) > vmax) {
+        vmax = fabs(xk[i]);
+        imax = i;
+        sgn = xk[i] < 0 ? -1.0 : 1.0;
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double v = __shfl_xor_sync(0xffffffffu, vmax, o), g = __shfl_xor_sync(0xffffffffu, sgn, o);
+      const int im = __shfl_xor_sync(0xffffffffu, imax, o);
+      if (v > vmax || (v == vmax && im < imax)) {
+        vmax = v;
+        sgn = g;
+        imax = im;
+      }
+    }
+    for (int i = lane; i < m; i += 32) Y[(int64_t)k * m + i] = sgn * xk[i];
+    if (lane == 0) evals[k] = lam[k];
   }
 }
 
@@ -1058,7 +1111,7 @@ int lz_finish(const T* Vb, int64_t n, int m, int K, double tol, const double* al
     return fail(GATO_EUNSUPPORTED, "lanczos: m = %d exceeds the tridiagonal eigensolver's shared memory", m);
   if (sme > 48 * 1024)
     GATO_TRY(raise_smem_limit(reinterpret_cast<const void*>(k_tridiag_eig), sme));
-  k_tridiag_eig<<<K, 32, sme, s>>>(alphas, betas, m, K, evals, z.work, device_error_word());
+  k_tridiag_eig<<<K, kTriThreads, sme, s>>>(alphas, betas, m, K, evals, z.work, device_error_word());
   GATO_LAUNCH_TRY();
   k_tridiag_finish<<<1, 32, 0, s>>>(alphas, betas, m, K, evals, z.work, evals, z.Y, flag, tol);
   GATO_LAUNCH_TRY();
@@ -1327,50 +1380,62 @@ __global__ void __maxnreg__(96)
 // with the sweep's projections reduced on the way in. part holds the sweep's block partials, rows
 // r <= j for a_k = dV <v_k, u_j> and rows j + 1 + k for d_k = dV <v_k, v_j>; a row sum is one warp
 // (lanes stride the G partials, then a fixed-order tree), the same sum wherever it runs. Every block
-// forms alpha_j = a_j - beta_{j-1} b_j (b_j = d_{j-1}); warps spread over the blocks form row j of Cm,
+// forms alpha_j = a_j - beta_{j-1} b_j (b_j = d_{j-1}); one warp of block k forms entry k of row j of Cm,
 // c_k = a_k - beta_{j-1} b_k - alpha_j d_k (b_k = <v_k, v_{j-1}> from the previous sweep for k < j,
-// d_{j-1} for k = j), and dprev <- d; block 0 records alpha_j.
-__global__ void k_fz_form(const float* __restrict__ U, const float* __restrict__ vm1, const float* __restrict__ vj,
+// d_{j-1} for k = j), and dprev <- d; block 0 records alpha_j. Bound by the latency of these reductions,
+// not by its 16 n bytes: the row sums run in four warps side by side, the first vectors are loaded before
+// them (64^3, warm: 10.6 -> 6.6 us). Launched with kFzFormThreads threads per block.
+constexpr int kFzFormThreads = 256;
+__global__ void __launch_bounds__(kFzFormThreads) k_fz_form(const float* __restrict__ U, const float* __restrict__ vm1, const float* __restrict__ vj,
                           float* wh, int64_t n, const double* part, int G, double dV, double* alphas,
                           const double* betas, double* dprev, double* Cm, int m, int j, double* partn) {
   __shared__ double sh[32];
-  __shared__ double s_ad[2];   // a_j, d_{j-1}
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  __shared__ double s_ad[4];   // a_j, d_{j-1}; this block's first Cm row: a_k, d_k
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t nv = n / 4, stride = (int64_t)gridDim.x * blockDim.x;
+  const float4* U4 = reinterpret_cast<const float4*>(U);
+  const float4* A4 = reinterpret_cast<const float4*>(j > 0 ? vm1 : vj);
+  const float4* B4 = reinterpret_cast<const float4*>(vj);
+  float4* W4 = reinterpret_cast<float4*>(wh);
+  // the first vectors are in flight while the row sums run
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  float4 u, a, b;
+  if (i < nv) {
+    u = U4[i];
+    a = A4[i];
+    b = B4[i];
+  }
   auto rowsum = [&](int r) {
     double v = 0.0;
+#pragma unroll 4
     for (int q = lane; q < G; q += 32) v += part[(int64_t)r * G + q];
     return warp_sum(v) * dV;
   };
-  if (warp == 0) {
-    const double aj = rowsum(j);
-    const double dj1 = j > 0 ? rowsum(2 * j) : 0.0;
-    if (lane == 0) {
-      s_ad[0] = aj;
-      s_ad[1] = dj1;
-    }
+  const int k0 = blockIdx.x;   // row k of Cm belongs to block k mod the grid
+  if (warp < 4) {              // four row sums side by side
+    const bool mine = warp < 2 || k0 <= j;
+    const int row = warp == 0 ? j : (warp == 1 ? 2 * j : (warp == 2 ? k0 : j + 1 + k0));
+    const double v = mine && (warp != 1 || j > 0) ? rowsum(row) : 0.0;
+    if (lane == 0) s_ad[warp] = v;
   }
   __syncthreads();
   const double beta = j > 0 ? betas[j - 1] : 0.0;
   const double ald = s_ad[0] - beta * s_ad[1];
   if (blockIdx.x == 0 && threadIdx.x == 0) alphas[j] = ald;
-  for (int k = blockIdx.x * nw + warp; k <= j; k += gridDim.x * nw) {
-    const double sak = rowsum(k), sdk = rowsum(j + 1 + k);
-    if (lane == 0) {
-      // the lane reads dprev[k] before it overwrites the same entry: no other thread touches it
-      const double bk = j == 0 ? 0.0 : (k < j ? dprev[k] : s_ad[1]);
-      Cm[(int64_t)j * m + k] = sak - beta * bk - ald * sdk;
-      dprev[k] = sdk;
+  if (warp == 4) {
+    for (int k = k0; k <= j; k += gridDim.x) {
+      const double sak = k == k0 ? s_ad[2] : rowsum(k), sdk = k == k0 ? s_ad[3] : rowsum(j + 1 + k);
+      if (lane == 0) {
+        // the lane reads dprev[k] before it overwrites the same entry: no other thread touches it
+        const double bk = j == 0 ? 0.0 : (k < j ? dprev[k] : s_ad[1]);
+        Cm[(int64_t)j * m + k] = sak - beta * bk - ald * sdk;
+        dprev[k] = sdk;
+      }
     }
   }
   const float be = (float)beta, al = (float)ald;
   Acc<float> acc;
-  const int64_t nv = n / 4;
-  const float4* U4 = reinterpret_cast<const float4*>(U);
-  const float4* A4 = reinterpret_cast<const float4*>(j > 0 ? vm1 : vj);
-  const float4* B4 = reinterpret_cast<const float4*>(vj);
-  float4* W4 = reinterpret_cast<float4*>(wh);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (int64_t)gridDim.x * blockDim.x) {
-    const float4 u = U4[i], a = A4[i], b = B4[i];
+  while (i < nv) {
     float4 w;
     w.x = u.x - be * a.x - al * b.x;
     w.y = u.y - be * a.y - al * b.y;
@@ -1381,6 +1446,12 @@ __global__ void k_fz_form(const float* __restrict__ U, const float* __restrict__
     acc.add_prod(w.y, w.y);
     acc.add_prod(w.z, w.z);
     acc.add_prod(w.w, w.w);
+    i += stride;
+    if (i < nv) {
+      u = U4[i];
+      a = A4[i];
+      b = B4[i];
+    }
   }
   const double v = block_sum(acc.value(), sh);
   if (threadIdx.x == 0) partn[blockIdx.x] = v;
@@ -1394,39 +1465,58 @@ constexpr int kFzPost2Threads = 256;
 __global__ void __launch_bounds__(kFzPost2Threads)
     k_fz_post2(const double* part, int nb, double dV, const double* Cm, int m, int j, const double* alphas,
                double* betas, double* binv, double* c_next, double* g_next) {
-  __shared__ double sh[32];
-  __shared__ double sc[kFzMaxM + 1];
-  double v = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) v += part[i];
-  const double wn = block_sum(v, sh);
-  double c2 = 0.0;
-  for (int k = threadIdx.x; k <= j; k += blockDim.x) {
-    const double ck = Cm[(int64_t)j * m + k];
-    sc[k] = ck;
-    c2 += ck * ck;
+  __shared__ double sh[2][32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const double* cj = Cm + (int64_t)j * m;
+  // everything the block reads is loaded before the first barrier
+  double v = 0.0, c2 = 0.0;
+#pragma unroll 4
+  for (int i = t; i < nb; i += kFzPost2Threads) v += part[i];
+  for (int k = t; k <= j; k += kFzPost2Threads) c2 += cj[k] * cj[k];
+  const int i = (int)((blockIdx.x * blockDim.x + t) >> 5);   // one warp per g_i
+  double gi = 0.0, ch = 0.0, bh = 0.0, cm = 0.0, am = 0.0, cl = 0.0;
+  if (i <= j + 1) {
+#pragma unroll 4
+    for (int k = i + lane; k <= j; k += 32) gi += cj[k] * Cm[(int64_t)k * m + i];
+    if (lane == 0) {
+      // the tridiagonal part of T~ row i: beta_i c_{i+1} + alpha_i c_i + beta_{i-1} c_{i-1}
+      if (i + 1 <= j) {
+        ch = cj[i + 1];
+        bh = betas[i];
+      }
+      if (i <= j) {
+        cm = cj[i];
+        am = alphas[i];
+      }
+      if (i >= 1) cl = cj[i - 1];
+    }
   }
-  const double cn = block_sum(c2, sh);   // its barriers also publish sc
+  const double bprev = i >= 1 && i - 1 < j ? betas[i - 1] : 0.0;
+  v = warp_sum(v);
+  c2 = warp_sum(c2);
+  gi = warp_sum(gi);
+  if (lane == 0) {
+    sh[0][warp] = v;
+    sh[1][warp] = c2;
+  }
+  __syncthreads();
+  // the block sums in block_sum's order, by every warp
+  constexpr int nw = kFzPost2Threads / 32;
+  const double wn = warp_sum(lane < nw ? sh[0][lane] : 0.0), cn = warp_sum(lane < nw ? sh[1][lane] : 0.0);
   const double b2 = wn * dV - cn;
   const double beta = b2 > 0.0 ? sqrt(b2) : 0.0;
   if (blockIdx.x == 0) {
-    if (threadIdx.x == 0) {
+    if (t == 0) {
       betas[j] = beta;
       binv[0] = beta;
       binv[1] = beta > 0.0 ? 1.0 / beta : 0.0;
     }
-    for (int k = threadIdx.x; k <= j; k += blockDim.x) c_next[k] = sc[k];
+    for (int k = t; k <= j; k += kFzPost2Threads) c_next[k] = cj[k];
   }
-  const int lane = threadIdx.x & 31;
-  const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (i > j + 1) return;
-  double gi = 0.0;
-  for (int k = i + lane; k <= j; k += 32) gi += sc[k] * Cm[(int64_t)k * m + i];
-  gi = warp_sum(gi);
-  if (lane == 0) {
-    // the tridiagonal part of T~ row i: beta_i c_{i+1} + alpha_i c_i + beta_{i-1} c_{i-1}
-    if (i + 1 <= j) gi += sc[i + 1] * betas[i];
-    if (i <= j) gi += sc[i] * alphas[i];
-    if (i >= 1) gi += sc[i - 1] * (i - 1 == j ? beta : betas[i - 1]);
+  if (i <= j + 1 && lane == 0) {
+    gi += ch * bh;
+    gi += cm * am;
+    gi += cl * (i - 1 == j ? beta : bprev);
     g_next[i] = gi;
   }
 }
@@ -1535,7 +1625,7 @@ int lanczos_fused(gato_operator& op, const void* psi0, int m, int K, double tol,
     k_fz_sweep<<<G, kFzThreads, smj, s>>>(*reinterpret_cast<const CUtensorMap*>(tm), Vb, n, j, ce, nst, wh, f.z,
                                           f.u, f.c, f.g, f.binv, f.part, device_error_word());
     GATO_LAUNCH_TRY();
-    k_fz_form<<<f.nbf, 256, 0, s>>>(f.u, j > 0 ? Vb + (int64_t)(j - 1) * n : nullptr, Vb + (int64_t)j * n, f.wh, n,
+    k_fz_form<<<f.nbf, kFzFormThreads, 0, s>>>(f.u, j > 0 ? Vb + (int64_t)(j - 1) * n : nullptr, Vb + (int64_t)j * n, f.wh, n,
                                     f.part, G, dV, alphas, betas, f.dprev, f.Cm, m, j, f.partn);
     GATO_LAUNCH_TRY();
     // beta_j and the next sweep's coefficients on the side stream, beside the operator apply to w^_j
