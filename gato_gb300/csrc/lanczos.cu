@@ -582,44 +582,289 @@ __global__ void __launch_bounds__(kBulkThreads)
   if (threadIdx.x == 0 && !*abort_v) part[blockIdx.x] = sum;
 }
 
-// nrm = dV * sum of the norm partials (the k_finalize_sums reduction order),
-// beta = sqrt(nrm) -> binv[0] and betas_out[0], 1 / beta (0 if beta = 0) ->
-// binv[1]: the FP64 square root and reciprocal once per step, in one thread.
-__global__ void k_beta_finalize(const double* partials, int nparts, double scale, double* binv,
-                                double* beta_out) {
-  __shared__ double sh[32];
-  double v = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) v += partials[i];
-  v = block_sum(v, sh);
-  if (threadIdx.x == 0) {
-    const double beta = sqrt(v * scale);
-    binv[0] = beta;
-    binv[1] = beta > 0 ? 1.0 / beta : 0.0;
-    beta_out[0] = beta;
+// ---- FP64 sweeps by warp shares --------------------------------------------------------
+// On an FP64 basis the coefficient sweep is bound by GB300's FP64 pipe (half a lane per clock and
+// scheduler): what counts is that every scheduler has the same number of FP64 instructions and few of
+// them are not multiply-adds of the sweep. Instructions whose lanes are predicated off or that reduce one
+// vector across the warp (five adds where a 64^3 block share has four multiply-adds) took more than half
+// of the block-share kernels' pipe time. Here the vector is cut into chunks of 64 elements (two a lane),
+// dealt in equal contiguous shares to one block of 8 to 12 warps per SM (ws_warps: the count whose largest
+// share is smallest); a warp keeps up to kWsChunks chunks of w in registers, streams kWsGroup vectors at a
+// time past them with 16-byte loads, and reduces the group together (multi_sum: nine adds for eight
+// vectors). 64^3, 40 vectors on average: 62 -> 33 us; the multiply-adds alone are 18 us.
+// VEC: 2 where every vector is 16-byte aligned (an even n), else 1 (two 8-byte loads).
+constexpr int kWsChunks = 3;
+constexpr int kWsGroup = 8;
+constexpr int kWsMaxWarps = 12;   // three a scheduler: 168 registers, which the two load buffers fit
+
+template <int VEC>
+__device__ __forceinline__ double2 ws_load(const double* p, int64_t base, int lane, int64_t n) {
+  double2 v = make_double2(0.0, 0.0);
+  if (VEC == 2) {
+    const int64_t i = base + 2 * lane;
+    if (i < n) v = *reinterpret_cast<const double2*>(p + i);
+  } else {
+    if (base + lane < n) v.x = p[base + lane];
+    if (base + lane + 32 < n) v.y = p[base + lane + 32];
+  }
+  return v;
+}
+template <int VEC>
+__device__ __forceinline__ void ws_store(double* p, int64_t base, int lane, int64_t n, double2 v) {
+  if (VEC == 2) {
+    const int64_t i = base + 2 * lane;
+    if (i < n) *reinterpret_cast<double2*>(p + i) = v;
+  } else {
+    if (base + lane < n) p[base + lane] = v.x;
+    if (base + lane + 32 < n) p[base + lane + 32] = v.y;
   }
 }
 
-// v = W / beta (or 0). The products run in the field type: an FP32 basis takes
-// the FP64 reciprocal rounded once to FP32, as FP64 products would put three
-// FP64-pipe operations on every element on GB300.
+// The warp sums of v[0..8): halving exchanges over lane bits 16, 8 and 4 leave each lane one value,
+// number lane >> 2, then the four lanes that share it add up.
+__device__ __forceinline__ double multi_sum(double* v, int lane) {
+  auto half = [&](int n, int o) {   // n values a lane -> n / 2, lanes with bit o keep the upper half
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < n / 2; ++i) {
+      const double send = up ? v[i] : v[i + n / 2], keep = up ? v[i + n / 2] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  };
+  half(8, 16);
+  half(4, 8);
+  half(2, 4);
+  double r = v[0];
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  return r;
+}
+
+// alpha of a step from its block partials, in every thread (k_finalize_sums for itself: one launch less);
+// block 0 stores it.
+struct WsAlpha {
+  const double* part = nullptr;   // null: the scalar is already in Pre
+  int n = 0;
+  double dv = 0.0;
+  double* out = nullptr;
+};
+
+__device__ __forceinline__ double2 ws_pre(double2 w, const double* u, int64_t base, int lane, int64_t n, double s,
+                                          bool vec2) {
+  const double2 x = vec2 ? ws_load<2>(u, base, lane, n) : ws_load<1>(u, base, lane, n);
+  w.x -= s * x.x;
+  w.y -= s * x.y;
+  return w;
+}
+
+// Four vectors' entries of CG chunks (q < cg) at p, p + ld, ...; vectors past nk and elements past n are zero.
+template <int VEC, int CG>
+__device__ __forceinline__ void ws_load4(double2 (&v)[4][CG], const double* p, int64_t ld, int left, int cg,
+                                         int64_t base, int lane, int64_t n) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int q = 0; q < CG; ++q) {
+      v[u][q] = make_double2(0.0, 0.0);
+      if (u < left && q < cg) v[u][q] = ws_load<VEC>(p + u * ld, base + 64 * q, lane, n);
+    }
+}
+
+// part[k * gridDim.x + block] = sum_i V_k[i] w[i], w = W - pre
+template <int VEC>
+__global__ void __launch_bounds__(32 * kWsMaxWarps, 1)
+    k_gemv_t_ws(const double* __restrict__ V, int64_t ld, int nk, const double* __restrict__ W, Pre<double> pre,
+                WsAlpha al, int64_t n, double* part) {
+  extern __shared__ double wacc[];   // [warp][k]
+  __shared__ double sh[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double sc[2];
+  pre_scalars(pre, sc);
+  if (al.part) {
+    double v = 0.0;
+    for (int i = threadIdx.x; i < al.n; i += blockDim.x) v += al.part[i];
+    sc[1] = block_sum(v, sh) * al.dv;
+    if (blockIdx.x == 0 && threadIdx.x == 0) al.out[0] = sc[1];
+  }
+  for (int i = threadIdx.x; i < nw * nk; i += blockDim.x) wacc[i] = 0.0;
+  __syncthreads();
+  const int64_t C = (n + 63) / 64, Wt = (int64_t)gridDim.x * nw, wid = (int64_t)blockIdx.x * nw + warp;
+  const int64_t c1 = C * (wid + 1) / Wt;
+  for (int64_t c = C * wid / Wt; c < c1; c += kWsChunks) {
+    const int cg = (int)(c1 - c < kWsChunks ? c1 - c : kWsChunks);
+    const int64_t base = c * 64;
+    double2 v[2][4][kWsChunks];   // the next four vectors load while these are multiplied
+    ws_load4<VEC, kWsChunks>(v[0], V, ld, nk, cg, base, lane, n);
+    double2 w[kWsChunks];
+#pragma unroll
+    for (int q = 0; q < kWsChunks; ++q) {
+      w[q] = make_double2(0.0, 0.0);
+      if (q >= cg) continue;
+      w[q] = ws_load<VEC>(W, base + 64 * q, lane, n);
+      if (pre.u[0]) w[q] = ws_pre(w[q], pre.u[0], base + 64 * q, lane, n, sc[0], VEC == 2);
+      if (pre.u[1]) w[q] = ws_pre(w[q], pre.u[1], base + 64 * q, lane, n, sc[1], VEC == 2);
+    }
+    const double* vp = V;
+    for (int k0 = 0; k0 < nk; k0 += kWsGroup) {
+      double sk[kWsGroup];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        vp += 4 * ld;
+        ws_load4<VEC, kWsChunks>(v[h ^ 1], vp, ld, nk - k0 - 4 * h - 4, cg, base, lane, n);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sk[4 * h + u] = v[h][u][0].x * w[0].x;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sk[4 * h + u] = fma(v[h][u][0].y, w[0].y, sk[4 * h + u]);
+#pragma unroll
+        for (int q = 1; q < kWsChunks; ++q) {
+          if (q >= cg) break;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) sk[4 * h + u] = fma(v[h][u][q].x, w[q].x, sk[4 * h + u]);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) sk[4 * h + u] = fma(v[h][u][q].y, w[q].y, sk[4 * h + u]);
+        }
+      }
+      const double d = multi_sum(sk, lane);
+      const int k = k0 + (lane >> 2);
+      if ((lane & 3) == 0 && k < nk) wacc[warp * nk + k] += d;
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += wacc[w * nk + k];
+    part[(int64_t)k * gridDim.x + blockIdx.x] = s;
+  }
+}
+
+// (float)v by integer arithmetic, round to nearest even: a conversion is an instruction of the FP64 pipe
+// (64 cycles a warp on GB300), this is nine of the integer units and no branch. Magnitudes below 2^-126
+// give 0; from 2^127 up (infinities and NaN among them) `big` is set and the value is not meaningful.
+__device__ __forceinline__ float to_float(double v, unsigned& big) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mag = hi & 0x7fffffffu;
+  const unsigned add = 0x0fffffffu + ((lo >> 29) & 1u);
+  const unsigned l2 = lo + add, m2 = mag + (l2 < lo);
+  big |= mag >= (1150u << 20);
+  const unsigned f = ((m2 - (896u << 20)) << 3) | (l2 >> 29);
+  return __uint_as_float((hi & 0x80000000u) | (mag < (897u << 20) ? 0u : f));
+}
+
+// W <- W - pre - sum_k c_k v_k, norm partial part[block]; the correction accumulates in FP32 as in
+// k_gemv_n<T, float>. No reduction per vector here, so the shares are single chunks over as many warps as
+// an SM takes (latency bound: 64^3, 40 vectors, 28 us with the block-share ring, 17.5 so).
+constexpr int kWsNWarps = 28;
+template <int VEC>
+__global__ void __launch_bounds__(32 * kWsNWarps, 1)
+    k_gemv_n_ws(const double* __restrict__ V, int64_t ld, int nk, double* __restrict__ W, Pre<double> pre,
+                const double* __restrict__ c_in, int64_t n, double* part) {
+  extern __shared__ double wacc[];
+  float* cs = reinterpret_cast<float*>(wacc);   // coefficients rounded once to FP32, zero up to a multiple of 4
+  __shared__ double sh[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double sc[2];
+  pre_scalars(pre, sc);
+  for (int i = threadIdx.x; i < (nk + 3) / 4 * 4; i += blockDim.x) cs[i] = i < nk ? (float)c_in[i] : 0.f;
+  __syncthreads();
+  const int64_t C = (n + 63) / 64, Wt = (int64_t)gridDim.x * nw, wid = (int64_t)blockIdx.x * nw + warp;
+  const int64_t c1 = C * (wid + 1) / Wt;
+  double acc = 0.0;
+  for (int64_t c = C * wid / Wt; c < c1; ++c) {
+    const int64_t base = c * 64;
+    double2 v[2][4][1];
+    ws_load4<VEC, 1>(v[0], V, ld, nk, 1, base, lane, n);
+    double2 w = ws_load<VEC>(W, base, lane, n);
+    if (pre.u[0]) w = ws_pre(w, pre.u[0], base, lane, n, sc[0], VEC == 2);
+    if (pre.u[1]) w = ws_pre(w, pre.u[1], base, lane, n, sc[1], VEC == 2);
+    float2 corr = make_float2(0.f, 0.f);
+    unsigned big = 0;
+    const double* vp = V;
+    for (int k0 = 0; k0 < nk; k0 += 8) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        vp += 4 * ld;
+        ws_load4<VEC, 1>(v[h ^ 1], vp, ld, nk - k0 - 4 * h - 4, 1, base, lane, n);
+        if (k0 + 4 * h >= nk) break;
+        const float4 ck = *reinterpret_cast<const float4*>(cs + k0 + 4 * h);
+        const float cu[4] = {ck.x, ck.y, ck.z, ck.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          corr.x = fmaf(cu[u], to_float(v[h][u][0].x, big), corr.x);
+          corr.y = fmaf(cu[u], to_float(v[h][u][0].y, big), corr.y);
+        }
+      }
+    }
+    if (big) {   // basis entries beyond FP32 (or not finite): the same sum by conversions
+      corr = make_float2(0.f, 0.f);
+      for (int k = 0; k < nk; ++k) {
+        const double2 x = ws_load<VEC>(V + (int64_t)k * ld, base, lane, n);
+        corr.x = fmaf(cs[k], (float)x.x, corr.x);
+        corr.y = fmaf(cs[k], (float)x.y, corr.y);
+      }
+    }
+    w.x -= (double)corr.x;
+    w.y -= (double)corr.y;
+    ws_store<VEC>(W, base, lane, n, w);
+    acc = fma(w.x, w.x, acc);   // elements past n are zero
+    acc = fma(w.y, w.y, acc);
+  }
+  const double sum = block_sum(acc, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = sum;
+}
+
+// Warps per block of the warp-share sweeps over nblk blocks: the largest share of an SM, in chunks, is
+// warps * ceil(chunks / (nblk warps)); the smallest such product, the fewest warps that reach it.
+inline int ws_warps(int64_t n, int nblk, int nk, int lo, int hi) {
+  const int64_t C = (n + 63) / 64;
+  int best = lo;
+  int64_t cost = INT64_MAX;
+  for (int w = lo; w <= hi; ++w) {
+    const int64_t share = w * ((C + (int64_t)nblk * w - 1) / ((int64_t)nblk * w));
+    if (share < cost && ((size_t)w * nk * sizeof(double) <= 200 * 1024 || w == lo)) {
+      cost = share;
+      best = w;
+    }
+  }
+  return best;
+}
+
+// beta = sqrt(dV * sum of the norm partials) and v = W / beta (or 0): every block sums the partials (in
+// k_finalize_sums' order, so all hold the same bits) while its first elements load, block 0 stores beta.
+// The products run in the field type: an FP32 basis takes the FP64 reciprocal rounded once to FP32, as
+// FP64 products would put three FP64-pipe operations on every element on GB300.
 template <typename T>
-__global__ void k_beta_scale(T* W, int64_t n, const double* binv) {
+__global__ void __launch_bounds__(256) k_beta_scale(T* W, int64_t n, const double* partials, int nparts, double scale,
+                                                    double* beta_out) {
   using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
   constexpr int VEC = 16 / (int)sizeof(T);
-  const bool pos = binv[0] > 0;
-  const T inv = (T)binv[1];
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  __shared__ double sh[32];
+  __shared__ double s_beta, s_inv;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nv = ((uintptr_t)W % 16) == 0 ? n / VEC : 0;   // 16-byte vectors
   V* W4 = reinterpret_cast<V*>(W);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride) {
-    V v = W4[i];
+  V v;
+  if (first < nv) v = W4[first];
+  double p = 0.0;
+  for (int i = threadIdx.x; i < nparts; i += blockDim.x) p += partials[i];
+  p = block_sum(p, sh);
+  if (threadIdx.x == 0) {
+    const double beta = sqrt(p * scale);
+    s_beta = beta;
+    s_inv = beta > 0 ? 1.0 / beta : 0.0;
+    if (blockIdx.x == 0) beta_out[0] = beta;
+  }
+  __syncthreads();
+  const bool pos = s_beta > 0;
+  const T inv = (T)s_inv;
+  for (int64_t i = first; i < nv;) {
     T* e = reinterpret_cast<T*>(&v);
 #pragma unroll
     for (int u = 0; u < VEC; ++u) e[u] = pos ? e[u] * inv : (T)0;
     W4[i] = v;
+    i += stride;
+    if (i < nv) v = W4[i];
   }
-  for (int64_t i = nv * VEC + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    W[i] = pos ? W[i] * inv : (T)0;
+  for (int64_t i = nv * VEC + first; i < n; i += stride) W[i] = pos ? W[i] * inv : (T)0;
 }
 
 template <typename T>
@@ -940,7 +1185,7 @@ __global__ void __launch_bounds__(256) k_ritz(const T* __restrict__ V, int64_t l
 }
 
 struct LzScratch {
-  double *part, *coef, *nrm, *Y, *work;
+  double *part, *coef, *nrm, *Y, *work, *apart;
   int nblk;     // k_gemv_n grid
   int nblk_t;   // k_gemv_t grid
   int nblk_b;   // bulk-streaming grid (both sweeps)
@@ -953,9 +1198,11 @@ inline int lz_nblk(int64_t n) { return (int)std::min<int64_t>((n + kChunk - 1) /
 inline int lz_nblk_t(int64_t n, bool fp64) {
   return (int)std::min<int64_t>((n + kChunk - 1) / kChunk, (fp64 ? 4 : 5) * 152);
 }
-// bulk-streaming kernels: 3 blocks per SM (their ring is 48 KB), at least one item each
+// FP32 bulk-streaming kernels: 3 blocks per SM (their ring is 48 KB), at least one item each. FP64
+// warp-share kernels: one block per SM, at least one chunk each.
 inline int lz_nblk_b(int64_t n, bool fp64) {
-  const int64_t ch = fp64 ? BulkGeom<double>::CH : BulkGeom<float>::CH;
+  if (fp64) return (int)std::max<int64_t>(1, std::min<int64_t>((n + 63) / 64, 152));
+  constexpr int64_t ch = BulkGeom<float>::CH;
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + ch - 1) / ch, 3 * 152));
 }
 
@@ -965,7 +1212,7 @@ int lz_scratch(cudaStream_t s, int64_t n, int m, int K, LzScratch& z, bool fp64)
   z.nblk_b = lz_nblk_b(n, fp64);
   const int np = std::max(std::max(z.nblk, z.nblk_t), z.nblk_b);
   // partials (m+1)*max(grids), coefficients (m+1), norm, Y (m*K), LU work 7*m*K
-  const size_t need = ((size_t)(m + 1) * np + (m + 1) + 8 + (size_t)m * K + (size_t)7 * m * K) *
+  const size_t need = ((size_t)(m + 1) * np + (m + 1) + 8 + (size_t)m * K + (size_t)7 * m * K + np) *
                       sizeof(double);
   z.part = (double*)stream_scratch(s, need, kSlotLanczos);
   if (!z.part) return fail(GATO_ENOMEM, "lanczos: scratch allocation failed");
@@ -973,6 +1220,7 @@ int lz_scratch(cudaStream_t s, int64_t n, int m, int K, LzScratch& z, bool fp64)
   z.nrm = z.coef + (m + 1);
   z.Y = z.nrm + 8;
   z.work = z.Y + (size_t)m * K;
+  z.apart = z.work + (size_t)7 * m * K;
   return GATO_OK;
 }
 
@@ -1045,6 +1293,29 @@ int gemv_n_bulk(const T* V, int64_t ld, int nk, T* W, const Pre<T>& pre, const d
   return GATO_OK;
 }
 
+bool ws_vec2(const double* V, int64_t n, const double* W, const Pre<double>& p) {
+  return n % 2 == 0 && (((uintptr_t)V | (uintptr_t)W | (uintptr_t)p.u[0] | (uintptr_t)p.u[1]) & 15u) == 0;
+}
+
+int gemv_t_ws(const double* V, int64_t ld, int nk, const double* W, const Pre<double>& pre, const WsAlpha& al,
+              int64_t n, int nblk, double* part, cudaStream_t s) {
+  const int nw = ws_warps(n, nblk, nk, 8, kWsMaxWarps);
+  const size_t sm = (size_t)nw * nk * sizeof(double);
+  auto kern = ws_vec2(V, n, W, pre) ? k_gemv_t_ws<2> : k_gemv_t_ws<1>;
+  if (sm > 48 * 1024) GATO_TRY(raise_smem_limit(reinterpret_cast<const void*>(kern), sm));
+  kern<<<nblk, 32 * nw, sm, s>>>(V, ld, nk, W, pre, al, n, part);
+  GATO_LAUNCH_TRY();
+  return GATO_OK;
+}
+
+int gemv_n_ws(const double* V, int64_t ld, int nk, double* W, const Pre<double>& pre, const double* c, int64_t n,
+              int nblk, double* part, cudaStream_t s) {
+  auto kern = ws_vec2(V, n, W, pre) ? k_gemv_n_ws<2> : k_gemv_n_ws<1>;
+  kern<<<nblk, 32 * ws_warps(n, nblk, 0, 16, kWsNWarps), (size_t)(nk + 3) / 4 * 16, s>>>(V, ld, nk, W, pre, c, n, part);
+  GATO_LAUNCH_TRY();
+  return GATO_OK;
+}
+
 template <typename T>
 int lz_step(T* Vb, int64_t n, double dV, int j, int passes, double* alphas, double* betas,
             const LzScratch& z, cudaStream_t s) {
@@ -1056,6 +1327,23 @@ int lz_step(T* Vb, int64_t n, double dV, int j, int passes, double* alphas, doub
     p1.s[0] = betas + (j - 1);
   }
   const int nk = j + 1;
+  if constexpr (sizeof(T) == 8) {
+    // alpha_j = dV <v_j, w'>: its partials stay in a row of their own, the coefficient sweep sums them
+    GATO_TRY(gemv_t_ws(vj, n, 1, W, p1, WsAlpha{}, n, z.nblk_b, z.apart, s));
+    Pre<T> p2 = p1;
+    p2.u[1] = vj;
+    p2.s[1] = alphas + j;
+    for (int p = 0; p < passes; ++p) {
+      const Pre<T> pp = p == 0 ? p2 : Pre<T>();
+      GATO_TRY(gemv_t_ws(Vb, n, nk, W, pp, p == 0 ? WsAlpha{z.apart, z.nblk_b, dV, alphas + j} : WsAlpha{}, n, z.nblk_b,
+                         z.part, s));
+      GATO_TRY(finalize_sums(z.part, nk, z.nblk_b, dV, z.coef, s));
+      GATO_TRY(gemv_n_ws(Vb, n, nk, W, pp, z.coef, n, z.nblk_b, z.part, s));
+    }
+    k_beta_scale<T><<<grid_for(n / 2 + 1, 256), 256, 0, s>>>(W, n, z.part, z.nblk_b, dV, betas + j);
+    GATO_LAUNCH_TRY();
+    return GATO_OK;
+  } else {
   if (bulk_ok(Vb, n)) {
     // alpha_j = dV <v_j, w'>
     GATO_TRY(gemv_t_bulk<T>(vj, n, 1, W, p1, n, z.nblk_b, z.part, s));
@@ -1069,9 +1357,8 @@ int lz_step(T* Vb, int64_t n, double dV, int j, int passes, double* alphas, doub
       GATO_TRY(finalize_sums(z.part, nk, z.nblk_b, dV, z.coef, s));
       GATO_TRY(gemv_n_bulk<T>(Vb, n, nk, W, pp, z.coef, n, z.nblk_b, z.part, s));
     }
-    k_beta_finalize<<<1, 256, 0, s>>>(z.part, z.nblk_b, dV, z.nrm, betas + j);
-    GATO_LAUNCH_TRY();
-    k_beta_scale<T><<<grid_for(n / (16 / (int64_t)sizeof(T)) + 1, 256), 256, 0, s>>>(W, n, z.nrm);
+    k_beta_scale<T><<<grid_for(n / (16 / (int64_t)sizeof(T)) + 1, 256), 256, 0, s>>>(W, n, z.part, z.nblk_b, dV,
+                                                                                      betas + j);
     GATO_LAUNCH_TRY();
     return GATO_OK;
   }
@@ -1095,11 +1382,11 @@ int lz_step(T* Vb, int64_t n, double dV, int j, int passes, double* alphas, doub
     k_gemv_n<T, float><<<z.nblk, kLzThreads, smn, s>>>(Vb, n, nk, W, pp, z.coef, n, z.part);
     GATO_LAUNCH_TRY();
   }
-  k_beta_finalize<<<1, 256, 0, s>>>(z.part, z.nblk, dV, z.nrm, betas + j);
-  GATO_LAUNCH_TRY();
-  k_beta_scale<T><<<grid_for(n / (16 / (int64_t)sizeof(T)) + 1, 256), 256, 0, s>>>(W, n, z.nrm);
+  k_beta_scale<T><<<grid_for(n / (16 / (int64_t)sizeof(T)) + 1, 256), 256, 0, s>>>(W, n, z.part, z.nblk, dV,
+                                                                                    betas + j);
   GATO_LAUNCH_TRY();
   return GATO_OK;
+  }
 }
 
 template <typename T>
