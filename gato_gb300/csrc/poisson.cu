@@ -344,7 +344,9 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
   // solve 1306 -> 736 us). FP64, arithmetic-bound, always gains. An FP32 lone field behind full ones
   // would cost a second set of launches, more than the half field it saves (exchange with three
   // orbitals, split against not: 68 against 47 us at 64^3, 88 against 73 us at 80^3, 203 against 192 us at
-  // 128^3), so FP32 takes them only where no full field rides along. Energies take them in the
+  // 128^3), so FP32 takes them only where no full field rides along, and from N = 64 up: below, their
+  // longer chain of barriers shows (helium matvec 21.3 against 24.2 us at N = 24, 27.2 and 27.0 at 40,
+  // 35.4 both at 64, 60.2 against 49.9 at 96). Energies take them in the
   // spectral pass only, and a lone field's epilogue writes its terms straight to the outputs, so
   // without accumulation it must be the call's one term.
   int nlone = 0;
@@ -352,7 +354,7 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
     while (nlone < args.nf && args.f[args.nf - 1 - nlone].p[1].a < 0) ++nlone;
     const PartDesc& d0 = args.f[args.nf - 1].p[0];
     if (epi == EPI_ACC && (nlone > 1 || (!accumulate && (args.nf > 1 || args.nout != 1 || d0.nt != 1)))) nlone = 0;
-    if (sizeof(T) == 4 && nlone < args.nf) nlone = 0;
+    if (sizeof(T) == 4 && (nlone < args.nf || N < 64)) nlone = 0;
   }
   const int nfull = args.nf - nlone;
   const int gfull = (nfull + group - 1) / group, ngroups = gfull + (nlone + group - 1) / group;
