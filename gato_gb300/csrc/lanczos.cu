@@ -794,16 +794,17 @@ __global__ void __launch_bounds__(32 * kWsNWarps, 1)
         }
       }
     }
-    if (big) {   // basis entries beyond FP32 (or not finite): the same sum by conversions
-      corr = make_float2(0.f, 0.f);
+    double2 cd = make_double2((double)corr.x, (double)corr.y);
+    if (big) {   // basis entries beyond FP32 (or not finite): the sum in FP64
+      cd = make_double2(0.0, 0.0);
       for (int k = 0; k < nk; ++k) {
         const double2 x = ws_load<VEC>(V + (int64_t)k * ld, base, lane, n);
-        corr.x = fmaf(cs[k], (float)x.x, corr.x);
-        corr.y = fmaf(cs[k], (float)x.y, corr.y);
+        cd.x = fma(c_in[k], x.x, cd.x);
+        cd.y = fma(c_in[k], x.y, cd.y);
       }
     }
-    w.x -= (double)corr.x;
-    w.y -= (double)corr.y;
+    w.x -= cd.x;
+    w.y -= cd.y;
     ws_store<VEC>(W, base, lane, n, w);
     acc = fma(w.x, w.x, acc);   // elements past n are zero
     acc = fma(w.y, w.y, acc);

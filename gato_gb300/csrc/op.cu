@@ -67,7 +67,7 @@ static int op_side(gato_operator& op) {
 static int local_part(gato_operator& op, const void* in, void* out, int nb, cudaStream_t ls) {
   const double coef = -0.5 / (op.h * op.h);
   GATO_TRY(stencil_apply(op.dtype, in, op.V, out, nb, op.N, op.N, op.N, op_n3(op), coef, op.boundary,
-                         op.order, nullptr, op.dV, ls));
+                         op.order, nullptr, op.dV, ls, ls == op.side && ls != nullptr));
   if (op.nl) GATO_TRY(nonlocal_apply(op.nl->n, in, out, nb, ls));
   return GATO_OK;
 }

@@ -51,7 +51,8 @@ __device__ __forceinline__ T lap_combine(T ctr, T s1, T s2, StencilCoef<T> c, in
     T d2 = (R == 2) ? (s2 - (T)6 * ctr) : (T)0;
     return c.c1 * d1 + c.c2 * d2;
   } else {
-    return c.c0 * ctr + c.c1 * s1 + c.c2 * s2;
+    const T v = c.c0 * ctr + c.c1 * s1;
+    return R == 2 ? v + c.c2 * s2 : v;
   }
 }
 
@@ -151,8 +152,10 @@ __device__ __forceinline__ bool run_slots(F& step, int qb, std::integer_sequence
 // a pair (8 bytes FP32, 16 bytes FP64), the z neighbours of both points come
 // from two pair loads (z - 2, z - 1) and (z + 2, z + 3), the y neighbours are
 // the thread's own queue centres plus 2R halo rows, and the output leaves as
-// one pair store per row.
-template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT>
+// one pair store per row. EDGE (ny not a multiple of the tile): warps whose rows
+// all lie past the grid's edge compute nothing (a third of an 80^3 grid's); where
+// there are none the test itself would cost up to a tenth.
+template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT, bool EDGE>
 __global__ void __launch_bounds__(kZP*(kBY / YPT))
     k_stencil_tma(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap vmap,
                   T* __restrict__ out, int nx, int ny, int nz, int cx, int tiles_z, int64_t bstride,
@@ -166,7 +169,12 @@ __global__ void __launch_bounds__(kZP*(kBY / YPT))
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSlots * G::SLOT_BYTES);
   __shared__ double sh[32];
 
-  const StencilCoef<T> c = coefs<T>(R == 1 ? 2 : 4);
+  StencilCoef<T> c = coefs<T>(R == 1 ? 2 : 4);
+  if constexpr (sizeof(T) == 8) {   // FP64: the prefactor in the coefficients, an operation a point less
+    c.c0 *= coef;
+    c.c1 *= coef;
+    c.c2 *= coef;
+  }
   const int tz = threadIdx.x, ty = threadIdx.y;
   const int tid = ty * kZP + tz;
   const int tile_z = blockIdx.x % tiles_z, tile_y = blockIdx.x / tiles_z;
@@ -232,7 +240,7 @@ __global__ void __launch_bounds__(kZP*(kBY / YPT))
       for (int r = 0; r < 2 * R; ++r) xq[k][r] = xq[k][r + 1];
       xq[k][2 * R] = ld2(pl + cidx + k * G::PW);
     }
-    if (q >= 2 * R) {
+    if (q >= 2 * R && (!EDGE || live)) {
       constexpr int CS = (J + kSlots - R) % kSlots;
       const T* pc = reinterpret_cast<const T*>(smem + CS * G::SLOT_BYTES);
       [[maybe_unused]] const T* pv = reinterpret_cast<const T*>(smem + CS * G::SLOT_BYTES + G::V_OFF);
@@ -258,8 +266,12 @@ __global__ void __launch_bounds__(kZP*(kBY / YPT))
           s2b = xq[k][0].y + xq[k][4].y + col[k].y + col[k + 4].y + lo.y + hi.y;
         }
         P2 val;
-        val.x = coef * lap_combine<T>(ctr.x, s1a, s2a, c, R);
-        val.y = coef * lap_combine<T>(ctr.y, s1b, s2b, c, R);
+        val.x = lap_combine<T>(ctr.x, s1a, s2a, c, R);
+        val.y = lap_combine<T>(ctr.y, s1b, s2b, c, R);
+        if constexpr (sizeof(T) == 4) {
+          val.x *= coef;
+          val.y *= coef;
+        }
         if constexpr (HAS_V) {
           const P2 v = ld2(pv + vidx + k * kBZ);
           val.x += v.x * ctr.x;
@@ -273,8 +285,9 @@ __global__ void __launch_bounds__(kZP*(kBY / YPT))
           }
         }
       }
-      if constexpr (STORE) op += pstride;
     }
+    if constexpr (STORE)
+      if (q >= 2 * R) op += pstride;
     // every thread is done with plane q - R; a timed-out wait anywhere stops the CTA
     fence_proxy_async_smem();   // its slot's reads precede the copy issued into it below
     if (__syncthreads_or(bad)) {
@@ -321,13 +334,13 @@ int resident_ctas(K kernel, int threads, int smem) {
   return per * sms;
 }
 
-template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT>
-int launch_tma_rows(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int nb, int nx, int ny,
+template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT, bool EDGE>
+int launch_tma_edge(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int nb, int nx, int ny,
                     int nz, int64_t bstride, double coef, double* dot_part, int* nparts,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool beside) {
   using G = TmaGeom<T, R>;
   constexpr int kThreads = kZP * (kBY / YPT);
-  auto kern = k_stencil_tma<T, R, YPT, HAS_V, STORE, DOT>;
+  auto kern = k_stencil_tma<T, R, YPT, HAS_V, STORE, DOT, EDGE>;
   // opt in to the large shared-memory carve-out once per device (the launch
   // itself then issues only stream work, so it can be graph-captured)
   static std::atomic<unsigned> attr_done{0};
@@ -340,12 +353,40 @@ int launch_tma_rows(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int
   }
   const int tiles_z = (nz + kBZ - 1) / kBZ, tiles_y = (ny + kBY - 1) / kBY;
   const int tiles = tiles_z * tiles_y;
-  // Split x into chunks so the grid is one full resident wave where the
-  // problem allows (every CTA streams at once, no tail wave); a chunk keeps at
-  // least 4 planes, since its 2R halo planes are re-read.
+  // Split x into chunks. FP32, bound by memory: one full resident wave where
+  // the problem allows (every CTA streams at once, no tail wave); a chunk keeps
+  // at least 4 planes, since its 2R halo planes are re-read, unless that leaves
+  // SMs without a CTA: a small grid waits for the march itself, and its halo
+  // planes come from L2 (13-point 16^3 3.6 us with 4 planes, 2.8 so, 64^3 3.7
+  // and 3.1; but four 64^3 fields, 256 CTAs of 4 planes, 4.5 us and in chunks
+  // of 3 planes 4.9). FP64, bound by the FP64 pipes: the chunk that gives the
+  // busiest SM the fewest planes, one plane's worth of march added per CTA
+  // (13-point 16^3 20.9 -> 4.9 us, 64^3 21.0 -> 11.4, 80^3 38.9 -> 25.0, 128^3
+  // 65.7 -> 63.0) -- except beside other kernels, where the same FP64 work
+  // on fewer SMs disturbs a one-wave kernel less (helium matvec at 64^3 198 us,
+  // spread out 202).
   static const int cap = resident_ctas(kern, kThreads, G::SMEM);   // one value per instantiation
-  int chunks = (int)std::max<int64_t>(1, cap / ((int64_t)tiles * nb));
-  chunks = std::min(chunks, std::max(1, nx / 4));
+  constexpr int kSms = 152;
+  int chunks;
+  if (sizeof(T) == 8 && !beside) {
+    // FP64 fields: the SM with the most planes on its FP64 pipe sets the time
+    int best = nx;
+    int64_t cost = INT64_MAX;
+    for (int c = 1; c <= nx; ++c) {
+      const int64_t ctas = (int64_t)tiles * nb * ((nx + c - 1) / c);
+      if (c < nx && ctas > (int64_t)4096 * nb) continue;   // the dot's partials per field
+      const int64_t load = (ctas + kSms - 1) / kSms * (c + 1);
+      if (load < cost) {
+        cost = load;
+        best = c;
+      }
+    }
+    chunks = (nx + best - 1) / best;
+  } else {
+    chunks = (int)std::max<int64_t>(1, cap / ((int64_t)tiles * nb));
+    const int fine = sizeof(T) == 8 ? 1 : (int)std::min<int64_t>(nx, kSms / ((int64_t)tiles * nb));
+    chunks = std::min(chunks, std::max(std::max(1, nx / 4), fine));
+  }
   const int cx = (nx + chunks - 1) / chunks;
   chunks = (nx + cx - 1) / cx;
   dim3 grid(tiles, chunks, nb), block(kZP, kBY / YPT);
@@ -356,20 +397,31 @@ int launch_tma_rows(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int
   return GATO_OK;
 }
 
+template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT>
+int launch_tma_rows(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int nb, int nx, int ny,
+                    int nz, int64_t bstride, double coef, double* dot_part, int* nparts,
+                    cudaStream_t s, bool beside) {
+  if (ny % kBY == 0)
+    return launch_tma_edge<T, R, YPT, HAS_V, STORE, DOT, false>(tm, vm, out, nb, nx, ny, nz, bstride, coef, dot_part,
+                                                                nparts, s, beside);
+  return launch_tma_edge<T, R, YPT, HAS_V, STORE, DOT, true>(tm, vm, out, nb, nx, ny, nz, bstride, coef, dot_part,
+                                                             nparts, s, beside);
+}
+
 template <typename T, int R, bool HAS_V, bool STORE, bool DOT>
 int launch_tma_mode(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int nb, int nx, int ny,
                     int nz, int64_t bstride, double coef, double* dot_part, int* nparts,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool beside) {
   const int rows = g_rows_per_thread.load() ? g_rows_per_thread.load() : kDefaultRows;
   if (rows == 2)
     return launch_tma_rows<T, R, 2, HAS_V, STORE, DOT>(tm, vm, out, nb, nx, ny, nz, bstride, coef,
-                                                       dot_part, nparts, s);
+                                                       dot_part, nparts, s, beside);
   return launch_tma_rows<T, R, 4, HAS_V, STORE, DOT>(tm, vm, out, nb, nx, ny, nz, bstride, coef,
-                                                     dot_part, nparts, s);
+                                                     dot_part, nparts, s, beside);
 }
 template <typename T, int R>
 int launch_tma(const void* psi, const void* V, void* out, int nb, int nx, int ny, int nz,
-               int64_t bstride, double coef, double* dot_part, int* nparts, cudaStream_t s) {
+               int64_t bstride, double coef, double* dot_part, int* nparts, cudaStream_t s, bool beside) {
   alignas(64) unsigned char tm[128];
   TmaBox box;
   box.rank = 4;
@@ -407,7 +459,7 @@ int launch_tma(const void* psi, const void* V, void* out, int nb, int nx, int ny
 #define GATO_TMA_MODE(M, HV, ST, DT)                                                          \
   case M:                                                                                    \
     return launch_tma_mode<T, R, HV, ST, DT>(T4, V3, out, nb, nx, ny, nz, bstride, coef,     \
-                                             dot_part, nparts, s);
+                                             dot_part, nparts, s, beside);
   switch (mode) {
     GATO_TMA_MODE(1, false, false, true)
     GATO_TMA_MODE(2, false, true, false)
@@ -424,7 +476,7 @@ int launch_tma(const void* psi, const void* V, void* out, int nb, int nx, int ny
 template <typename T>
 int stencil_typed(const void* psi, const void* V, void* out, int nb, int nx, int ny, int nz,
                   int64_t bstride, double coef, int boundary, int order, double* dot_dev,
-                  double dv, cudaStream_t s) {
+                  double dv, cudaStream_t s, bool beside) {
   const bool tma_ok = boundary == GATO_DIRICHLET && ((uint64_t)nz * sizeof(T)) % 16 == 0 &&
                       ((uint64_t)bstride * sizeof(T)) % 16 == 0 &&
                       ((uintptr_t)psi % 16) == 0 && ((uintptr_t)V % 16) == 0 &&
@@ -438,9 +490,9 @@ int stencil_typed(const void* psi, const void* V, void* out, int nb, int nx, int
   if (tma_ok) {
     int nparts = 0;
     if (order == 2)
-      GATO_TRY(launch_tma<T, 1>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s));
+      GATO_TRY(launch_tma<T, 1>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s, beside));
     else
-      GATO_TRY(launch_tma<T, 2>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s));
+      GATO_TRY(launch_tma<T, 2>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s, beside));
     if (dot_dev) {
       if (nparts > 4096) return fail(GATO_EUNSUPPORTED, "stencil: too many tiles for dot");
       GATO_TRY(finalize_sums(part, nb, nparts, dv, dot_dev, s));
@@ -471,7 +523,7 @@ int stencil_typed(const void* psi, const void* V, void* out, int nb, int nx, int
 
 int stencil_apply(int dtype, const void* psi, const void* V, void* out, int nb, int nx, int ny,
                   int nz, int64_t bstride, double coef, int boundary, int order, double* dot_dev,
-                  double dv, cudaStream_t s) {
+                  double dv, cudaStream_t s, bool beside) {
   if (order != 2 && order != 4)
     return fail(GATO_EBADARG, "Unknown order %d; expected 2 or 4.", order);
   if (boundary != GATO_DIRICHLET && boundary != GATO_PERIODIC)
@@ -480,10 +532,10 @@ int stencil_apply(int dtype, const void* psi, const void* V, void* out, int nb, 
     return fail(GATO_EBADARG, "stencil: bad arguments");
   if (dtype == GATO_F64)
     return stencil_typed<double>(psi, V, out, nb, nx, ny, nz, bstride, coef, boundary, order,
-                                 dot_dev, dv, s);
+                                 dot_dev, dv, s, beside);
   if (dtype == GATO_F32)
     return stencil_typed<float>(psi, V, out, nb, nx, ny, nz, bstride, coef, boundary, order,
-                                dot_dev, dv, s);
+                                dot_dev, dv, s, beside);
   return fail(GATO_EBADARG, "bad dtype %d", dtype);
 }
 

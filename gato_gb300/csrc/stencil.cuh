@@ -3,8 +3,9 @@
 #include "common.cuh"
 
 namespace gato {
-// out[b] = coef * L(psi[b]) + V * psi[b]; dot_dev[b] = dv * <psi[b], out[b]>.
+// out[b] = coef * L(psi[b]) + V * psi[b]; dot_dev[b] = dv * <psi[b], out[b]>. beside: other kernels run
+// on the GPU at the same time (a choice of tiles, not of results).
 int stencil_apply(int dtype, const void* psi, const void* V, void* out, int nb, int nx, int ny,
                   int nz, int64_t bstride, double coef, int boundary, int order, double* dot_dev,
-                  double dv, cudaStream_t s);
+                  double dv, cudaStream_t s, bool beside = false);
 }  // namespace gato
