@@ -478,6 +478,35 @@ int poisson_run(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate,
   return run_typed<float>(pl, args, epi, accumulate, energy_dev, s, join);
 }
 
+// Appends the FP64 stage-twiddle rows of an R-point second stage (see fft2.cuh), rows r < nrows:
+// (c, t = s / c) or (c, s) of exp(-2 pi i (a r / M + b / R)).
+static void stage_rows(std::vector<double2>& out, int nrows, int R, int M) {
+  const int A = fft2::tw_a(R), B = fft2::tw_b(R), stride = fft2::tw_row_stride(false, R);
+  const double floor_c = 0x1p-60;   // for c = 0: far below the rounding, c t = s
+  for (int r = 0; r < nrows; ++r) {
+    const size_t row = out.size();
+    auto add = [&](int a, int b, bool ratio) {
+      const int64_t den = (int64_t)M * R, num = ((int64_t)a * r * R + (int64_t)b * M) % den;
+      const long double ang = 2.0L * 3.14159265358979323846264338327950288L * (long double)num / (long double)den;
+      const long double c = cosl(ang), sn = -sinl(ang);
+      const bool zero = std::fabs((double)c) < floor_c;
+      if (ratio) out.push_back(make_double2(zero ? floor_c : (double)c, (double)(sn / (zero ? (long double)floor_c : c))));
+      else out.push_back(make_double2((double)c, (double)sn));
+    };
+    add(B, 0, true);
+    if (A == 4) add(2 * B, 0, true);
+    for (int k1 = 0; k1 < A && B > 1; ++k1) {
+      if (B == 2 || B == 4) {
+        add(1, k1, true);
+        if (B == 4) add(2, 2 * k1, true);
+      } else {
+        for (int n2 = 1; n2 < B; ++n2) add(n2, n2 * k1, false);
+      }
+    }
+    out.resize(row + stride, make_double2(1.0, 0.0));
+  }
+}
+
 static int plan_create(int dtype, int N, double h, double eps, int max_fields, PoissonPlan& pl,
                        cudaStream_t s) {
   if (dtype != GATO_F64 && dtype != GATO_F32) return fail(GATO_EBADARG, "bad dtype %d", dtype);
@@ -510,19 +539,20 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
   GATO_CUDA_TRY(cudaMemcpyAsync(pl.tw, dtype == GATO_F64 ? (void*)tw64.data() : (void*)tw32.data(),
                                 (size_t)M * 2 * ts, cudaMemcpyHostToDevice, s));
   if (const int R2 = fast::shape_r2(M)) {
-    // the register engine's stage twiddles: row k1 holds exp(-2 pi i n2 k1 / M)
-    // for n2 < R2, rows padded to the stride the kernels read them with
+    // the register engine's stage twiddles (fft2.cuh)
     const int R1 = M / R2;
-    const int S = fft2::tw_row_stride(dtype == GATO_F32, R2);
-    std::vector<double2> t64((size_t)R1 * S, make_double2(0.0, 0.0));
-    std::vector<float2> t32((size_t)R1 * S, make_float2(0.f, 0.f));
-    for (int k1 = 0; k1 < R1; ++k1)
-      for (int n2 = 0; n2 < R2; ++n2) {
-        const double2 w = tw64[(size_t)n2 * k1];   // n2 k1 < M
-        t64[(size_t)k1 * S + n2] = w;
-        t32[(size_t)k1 * S + n2] = make_float2((float)w.x, (float)w.y);
-      }
-    const size_t bytes = (size_t)R1 * S * 2 * ts;
+    std::vector<double2> t64;
+    std::vector<float2> t32;
+    if (dtype == GATO_F64) {
+      stage_rows(t64, R1, R2, M);
+      if (R1 != R2) stage_rows(t64, R2, R1, M);
+    } else {
+      const int S = fft2::tw_row_stride(true, R2);
+      t32.assign((size_t)R1 * S, make_float2(0.f, 0.f));
+      for (int k1 = 0; k1 < R1; ++k1)
+        for (int n2 = 0; n2 < R2; ++n2) t32[(size_t)k1 * S + n2] = tw32[(size_t)n2 * k1];   // n2 k1 < M
+    }
+    const size_t bytes = dtype == GATO_F64 ? t64.size() * sizeof(double2) : t32.size() * sizeof(float2);
     GATO_CUDA_TRY(cudaMalloc(&pl.tw2, bytes));
     GATO_CUDA_TRY(cudaMemcpyAsync(pl.tw2, dtype == GATO_F64 ? (void*)t64.data() : (void*)t32.data(), bytes,
                                   cudaMemcpyHostToDevice, s));

@@ -43,8 +43,7 @@ struct PoissonPlan {
   FftPlanDev fp{};
   void* ghat = nullptr;    // H^3 octant of the kernel spectrum, x dV / M^3
   void* tw = nullptr;      // M twiddles exp(-2 pi i k / M)
-  void* tw2 = nullptr;     // register engine: tw2[k1 S + n2] = exp(-2 pi i n2 k1 / M), M = R1 R2,
-                           // S = fft2::tw_row_stride
+  void* tw2 = nullptr;     // register engine: the stage-twiddle table(s) of fft2.cuh
   void* tw4 = nullptr;     // packed FP32 engine: tw4[k1 R2 + n2] = (c, c, s, s), (c, s) = exp(-2 pi i n2 k1 / M)
   void* ghat2 = nullptr;   // packed FP32 engine: kernel spectrum folded in x and y only, [kxo][kyo][kz < M]
   void* S1 = nullptr;      // max_fields x N x N x M complex

@@ -46,7 +46,11 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + M * LP;
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, L * Shape<R1, R2>::RMAX> twp(tw);
+  using Tab = TwTab<T2, R1, R2>;   // tws: F, I or both as the mode needs them
+  constexpr int TW0 = MODE == COL_INV ? Tab::OI : 0;
+  constexpr int TWN = MODE == COL_FMI ? Tab::N : (MODE == COL_FWD ? Tab::NF : Tab::NI);
+  const T2* twi = tws + (Tab::OI - TW0);
+  const TwPrefetch<T2, TWN, L * Shape<R1, R2>::RMAX> twp(tw + TW0);
   const int outer = blockIdx.x, col0 = blockIdx.y * L, f = blockIdx.z;
   const int t = threadIdx.x;
   const int line = t % L, q = t / L;   // q: n2 in stages 1/B, k1 in stages 2/A
@@ -79,7 +83,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
         else X[k2].x = X[k2].y = 0;
       }
     }
-    twp.store(tws);   // first read in inv_stageA, behind the barrier below
+    twp.store(tws);   // FP32: first read in inv_stageA, FP64 in inv_stageB, behind the barriers below
   }
   if (MODE == COL_FWD) {
     if (q < R1 && live) {
@@ -110,7 +114,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   __syncthreads();
   if (q < R2) {
     T2* b = dst + q * ops;
-    inv_stageB<T2, R1, R2, true>(buf, LP, line, q, [&](int pos, T2 v) {
+    inv_stageB<T2, R1, R2, true>(buf, LP, line, q, twi, [&](int pos, T2 v) {
       if (live) b[(pos - q) * ops] = v;
     });
   }
@@ -171,7 +175,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   __shared__ double sh[32];
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + M * LP;
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, L * Shape<R1, R2>::RMAX> twp(tw);
+  const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, L * Shape<R1, R2>::RMAX> twp(tw);
   const int outer = blockIdx.x, col0 = blockIdx.y * L, f = blockIdx.z;
   const int t = threadIdx.x;
   const int line = t % L, q = t / L;
@@ -262,7 +266,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, NT> twp(tw);
   const int p = blockIdx.y;
   const FieldDesc& fd = args.f[f0 + p];
   const int64_t nrows = (int64_t)N * N;
@@ -334,8 +338,8 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   __shared__ __align__(8) uint64_t sbar;
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
-  T* stage = reinterpret_cast<T*>(tws + R1 * TwRow<T2, R2>::S);   // [slot][line][z], rows of NP
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  T* stage = reinterpret_cast<T*>(tws + TwTab<T2, R1, R2>::NF);   // [slot][line][z], rows of NP
+  const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, NT> twp(tw);
   const int64_t row0 = (int64_t)blockIdx.x * L;
   const int64_t nrows = (int64_t)N * N;
   if constexpr (BULK) {
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   __shared__ int s_misaligned;
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
-  T* stage0 = reinterpret_cast<T*>(tws + R1 * TwRow<T2, R2>::S);   // [slot][input][line][z], rows of NP
+  T* stage0 = reinterpret_cast<T*>(tws + TwTab<T2, R1, R2>::NF);   // [slot][input][line][z], rows of NP
   const int SB = ri.nin * L * NP;                                    // floats per staging slot
   const int64_t nrows = (int64_t)N * N;
   const int nblk = (int)(nrows / L);
@@ -469,7 +473,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
     s_misaligned = bad_align;
     if (bad_align && err) atomicExch(err, 110);
   }
-  for (int i = threadIdx.x; i < R1 * TwRow<T2, R2>::S; i += NT) tws[i] = tw[i];
+  for (int i = threadIdx.x; i < TwTab<T2, R1, R2>::NF; i += NT) tws[i] = tw[i];
   __syncthreads();
   if (s_misaligned) return;
   auto issue = [&](int blk, int slot) {
@@ -559,7 +563,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX, (rows_inv_min_ctas<T,
   __shared__ double sh[32];
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  const TwPrefetch<T2, TwTab<T2, R1, R2>::NI, NT> twp(tw + TwTab<T2, R1, R2>::OI);
   const int64_t nrows = (int64_t)N * N;
   const RowMap<R1, R2, L> q;
   const int j = q.n2;
@@ -615,7 +619,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX, (rows_inv_min_ctas<T,
     if (own) {
       if constexpr (!PREFETCH) load_fac();
       T2 w[R1];
-      row_inv_stageB<T2, R1, R2>(buf, q.l1, j, w);
+      row_inv_stageB<T2, R1, R2>(buf, q.l1, j, tws, w);
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const int64_t gi = r * N + j + R2 * e;
@@ -686,7 +690,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * LS;
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, NT> twp(tw);
   const int p = blockIdx.y;
   const PartDesc& pd = args.f[f0 + p].p[0];
   const int64_t npair = (int64_t)N * N / 2;
@@ -743,7 +747,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  const TwPrefetch<T2, TwTab<T2, R1, R2>::NI, NT> twp(tw + TwTab<T2, R1, R2>::OI);
   const int p = blockIdx.y;
   const int64_t npair = (int64_t)N * N / 2;
   const RowMap<R1, R2, L> q;
@@ -773,7 +777,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   const int64_t l = l0 + q.l1;
   if (!q.a1 || l >= npair) return;
   T2 w[R1];
-  row_inv_stageB<T2, R1, R2>(buf, q.l1, q.n2, w);
+  row_inv_stageB<T2, R1, R2>(buf, q.l1, q.n2, tws, w);
   const int64_t g0 = 2 * l * N + q.n2;
   if constexpr (J) {
     T* o = reinterpret_cast<T*>(args.jbase) + (int64_t)(2 * (f0 + p)) * args.jstride + g0;
@@ -814,7 +818,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   extern __shared__ __align__(16) unsigned char smraw[];
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
-  const TwPrefetch<T2, R1 * TwRow<T2, R2>::S, NT> twp(tw);
+  const TwPrefetch<T2, TwTab<T2, R1, R2>::NI, NT> twp(tw + TwTab<T2, R1, R2>::OI);
   const int p = blockIdx.y;
   const int64_t nrows = (int64_t)N * N;
   const RowMap<R1, R2, L> q;
@@ -834,7 +838,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   __syncthreads();
   if (q.a1 && r < nrows) {
     T2 w[R1];
-    row_inv_stageB<T2, R1, R2>(buf, q.l1, q.n2, w);
+    row_inv_stageB<T2, R1, R2>(buf, q.l1, q.n2, tws, w);
     T* jre = jbase + (int64_t)(2 * (f0 + p)) * jstride + r * N + q.n2;
     T* jim = jre + jstride;
 #pragma unroll
@@ -855,9 +859,13 @@ template <typename T, int R1, int R2, int L>
 struct Launch {
   using T2 = typename Cplx<T>::type;
   static constexpr int M = R1 * R2, N = M / 2, NT = L * Shape<R1, R2>::RMAX;
-  static constexpr int TWN = R1 * TwRow<T2, R2>::S;   // stage-twiddle table entries
-  static size_t sm_cols() { return (size_t)(M * (L + 1) + TWN) * sizeof(T2); }
-  static size_t sm_rows() { return (size_t)(L * RowBuf<R1, R2>::LS + TWN) * sizeof(T2); }
+  using Tab = TwTab<T2, R1, R2>;   // stage-twiddle table entries
+  static size_t sm_cols(int mode) {
+    return (size_t)(M * (L + 1) + (mode == COL_FMI ? Tab::N : (mode == COL_FWD ? Tab::NF : Tab::NI))) * sizeof(T2);
+  }
+  static size_t sm_rows(bool fwd) {
+    return (size_t)(L * RowBuf<R1, R2>::LS + (fwd ? Tab::NF : Tab::NI)) * sizeof(T2);
+  }
   // Whole tiles only where L divides the M columns (the callers pass all of them, or a multiple of L
   // that is at most M).
   static constexpr bool FULL = M % L == 0;
@@ -865,7 +873,7 @@ struct Launch {
                   const T* ghat, int H, cudaStream_t s) {
     if (FULL && g.ncols % L != 0) return fail(GATO_EUNSUPPORTED, "column pass: whole tiles of %d columns", L);
     dim3 grid(outer, (g.ncols + L - 1) / L, nf);
-    const size_t sm = sm_cols();
+    const size_t sm = sm_cols(mode);
     if (mode == COL_FWD) {
       GATO_TRY(smem_attr(k_cols<T, R1, R2, L, COL_FWD, FULL>, sm));
       k_cols<T, R1, R2, L, COL_FWD, FULL><<<grid, NT, sm, s>>>(in, out, g, tw, ghat, H);
@@ -882,14 +890,14 @@ struct Launch {
   static int cols_fe(const T2* in, const ColGeom& g, int outer, int nf, const T2* tw, const T* ghat, int H,
                      const FeArgs& fa, cudaStream_t s) {
     dim3 grid(outer, (g.ncols + L - 1) / L, nf);
-    const size_t sm = sm_cols();
+    const size_t sm = sm_cols(COL_FWD);
     GATO_TRY(smem_attr(k_cols_fe<T, R1, R2, L, FULL>, sm));
     k_cols_fe<T, R1, R2, L, FULL><<<grid, NT, sm, s>>>(in, g, tw, ghat, H, fa);
     GATO_LAUNCH_TRY();
     return GATO_OK;
   }
   static int rows_fwd_real(const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw, cudaStream_t s) {
-    const size_t sm = sm_rows();
+    const size_t sm = sm_rows(true);
     GATO_TRY(smem_attr(k_rows_fwd_real<T, R1, R2, L>, sm));
     const unsigned nblk = (unsigned)(((int64_t)N * N / 2 + L - 1) / L);
     k_rows_fwd_real<T, R1, R2, L><<<dim3(nblk, nfg), NT, sm, s>>>(a, f0, S1, tw);
@@ -899,7 +907,7 @@ struct Launch {
   // j: potentials to the J fields (nfg fields at once), else one field's terms to the outputs
   static int rows_inv_real(const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,
                            bool j, cudaStream_t s) {
-    const size_t sm = sm_rows();
+    const size_t sm = sm_rows(false);
     const unsigned nblk = (unsigned)(((int64_t)N * N / 2 + L - 1) / L);
     if (j) {
       GATO_TRY(smem_attr(k_rows_inv_real<T, R1, R2, L, true>, sm));
@@ -937,7 +945,7 @@ struct Launch {
     constexpr int LM = L >= 16 ? L / 2 : L;
     const size_t stage_bytes = (size_t)ri.nin * LM * StageRow<R1, R2>::NP * sizeof(T);
     if (multi > 0 && nfg >= (multi == 1 ? 3 : 2) && stage_bytes <= 48 * 1024) {
-      const size_t sm = (size_t)(LM * RowBuf<R1, R2>::LS + TWN) * sizeof(T2) + stage_bytes;
+      const size_t sm = (size_t)(LM * RowBuf<R1, R2>::LS + Tab::NF) * sizeof(T2) + stage_bytes;
       const int64_t nrows = (int64_t)N * N;
       // a bulk copy needs 16-byte aligned source and destination rows and a
       // size that is a multiple of 16 bytes (the padded staged row included)
@@ -975,7 +983,7 @@ struct Launch {
       GATO_LAUNCH_TRY();
       return GATO_OK;
     }
-    const size_t sm = sm_rows();
+    const size_t sm = sm_rows(true);
     GATO_TRY(smem_attr(k_rows_fwd<T, R1, R2, L>, sm));
     const int64_t nrows = (int64_t)N * N;
     k_rows_fwd<T, R1, R2, L><<<dim3((unsigned)((nrows + L - 1) / L), nfg), NT, sm, s>>>(a, f0, S1, tw);
@@ -985,7 +993,7 @@ struct Launch {
   template <int NO>
   static int rows_inv_no(const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,
                          double* partials, int64_t slot_stride, cudaStream_t s) {
-    const size_t sm = sm_rows();
+    const size_t sm = sm_rows(false);
     const unsigned nblk = (unsigned)(((int64_t)N * N + L - 1) / L);
     GATO_TRY(smem_attr(k_rows_inv<T, R1, R2, L, NO>, sm));
     k_rows_inv<T, R1, R2, L, NO><<<nblk, NT, sm, s>>>(a, f0, nfg, S1, tw, accumulate, partials,
@@ -994,7 +1002,7 @@ struct Launch {
     return GATO_OK;
   }
   static int rows_inv_j(const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, cudaStream_t s) {
-    const size_t sm = sm_rows();
+    const size_t sm = sm_rows(false);
     const unsigned nblk = (unsigned)(((int64_t)N * N + L - 1) / L);
     GATO_TRY(smem_attr(k_rows_inv_j<T, R1, R2, L>, sm));
     k_rows_inv_j<T, R1, R2, L><<<dim3(nblk, nfg), NT, sm, s>>>((T*)a.jbase, a.jstride, f0, S1, tw);
