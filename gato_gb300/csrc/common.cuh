@@ -59,6 +59,38 @@ void release_stream_scratch(cudaStream_t s);
 // thread's allocation while those kernels still write it. Null entries are
 // skipped; nothing is waited for when all are null.
 void free_after_pending(std::initializer_list<void*> ptrs);
+// ---- kept resources ------------------------------------------------------------------
+// Device workspace of an operator. Freed workspace is kept for the next operator (an energy or gradient
+// call makes one operator each, and cudaMalloc and cudaFree, the latter with a device synchronisation,
+// cost it a millisecond): `ev` marks its last use, and whoever takes it makes its own stream wait for
+// that, so threads and streams never overlap on it. At most kWsKeep buffers and kWsKeepBytes are kept per
+// process; the rest is freed, as is everything kept when an allocation fails. Work captured into a CUDA
+// graph pins its buffer (the graph may replay after the operator is gone): it is never handed on.
+struct WsBuf {
+  void* p = nullptr;
+  size_t bytes = 0;
+  cudaEvent_t ev = nullptr;
+  int dev = 0;
+  bool captured = false;
+  bool open = false;    // taken for work whose end is not marked (yet): a call that failed in between
+};
+constexpr int kWsKeep = 8;
+constexpr size_t kWsKeepBytes = (size_t)1 << 30;
+int ws_get(WsBuf& b, size_t bytes, cudaStream_t s);   // b holds at least `bytes`, usable on s from here on
+int ws_used(WsBuf& b, cudaStream_t s);                // the work queued on s so far uses b
+void ws_put(WsBuf& b);                                // gives b back
+
+// A side stream with the events that fork work onto it and join it back. Kept like workspace (at most
+// kSideKeep): work left in the stream merely runs before its next owner's.
+struct SideStream {
+  cudaStream_t st = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  int dev = 0;
+};
+constexpr int kSideKeep = 16;
+int side_get(SideStream& x);
+void side_put(SideStream& x);
+
 // sum_i a_i b_i * scale into out[0] (device), FP64 / float-float accumulation.
 int dot_impl(int dtype, const void* a, const void* b, int64_t n, double scale, double* out,
              cudaStream_t s);

@@ -10,6 +10,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <vector>
 #include <string>
 #include <utility>
 
@@ -93,6 +94,134 @@ void free_after_pending(std::initializer_list<void*> ptrs) {
   cudaDeviceSynchronize();
   for (void* p : ptrs)
     if (p) cudaFree(p);
+}
+
+static std::mutex g_keep_mu;
+static std::vector<WsBuf> g_ws;
+static std::vector<SideStream> g_side;
+
+static bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
+static void ws_free(WsBuf& b) {
+  free_after_pending({b.p});
+  if (b.ev) cudaEventDestroy(b.ev);
+  b = WsBuf{};
+}
+
+int ws_get(WsBuf& b, size_t bytes, cudaStream_t s) {
+  if (b.p && b.bytes >= bytes) {
+    b.open = true;
+    return GATO_OK;
+  }
+  if (b.p) ws_put(b);
+  int dev = 0;
+  GATO_CUDA_TRY(cudaGetDevice(&dev));
+  const bool cap = is_capturing(s);   // a wait on work outside the capture would break it: fresh memory
+  if (!cap) {
+    std::lock_guard<std::mutex> lk(g_keep_mu);
+    int best = -1;
+    for (int i = 0; i < (int)g_ws.size(); ++i)
+      if (g_ws[i].dev == dev && g_ws[i].bytes >= bytes && (best < 0 || g_ws[i].bytes < g_ws[best].bytes)) best = i;
+    if (best >= 0) {
+      b = g_ws[best];
+      g_ws.erase(g_ws.begin() + best);
+    }
+  }
+  if (b.p) {
+    const cudaError_t e = cudaStreamWaitEvent(s, b.ev, 0);
+    if (e == cudaSuccess) {
+      b.open = true;
+      return GATO_OK;
+    }
+    ws_free(b);
+    GATO_CUDA_TRY(e);
+  }
+  cudaError_t e = cudaMalloc(&b.p, bytes);
+  if (e != cudaSuccess) {   // give back what is kept and try once more
+    cudaGetLastError();
+    std::vector<WsBuf> kept;
+    {
+      std::lock_guard<std::mutex> lk(g_keep_mu);
+      kept.swap(g_ws);
+    }
+    for (auto& k : kept) ws_free(k);
+    e = cudaMalloc(&b.p, bytes);
+  }
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    if (b.p) cudaFree(b.p);
+    b = WsBuf{};
+    GATO_CUDA_TRY(e);
+  }
+  b.bytes = bytes;
+  b.dev = dev;
+  b.open = true;
+  return GATO_OK;
+}
+
+int ws_used(WsBuf& b, cudaStream_t s) {
+  if (is_capturing(s)) {
+    b.captured = true;
+    return GATO_OK;
+  }
+  GATO_CUDA_TRY(cudaEventRecord(b.ev, s));
+  b.open = false;
+  return GATO_OK;
+}
+
+void ws_put(WsBuf& b) {
+  if (!b.p) return;
+  if (!b.captured && !b.open) {
+    std::lock_guard<std::mutex> lk(g_keep_mu);
+    size_t kept = b.bytes;
+    for (const auto& k : g_ws) kept += k.bytes;
+    if ((int)g_ws.size() < kWsKeep && kept <= kWsKeepBytes) {
+      g_ws.push_back(b);
+      b = WsBuf{};
+      return;
+    }
+  }
+  ws_free(b);
+}
+
+int side_get(SideStream& x) {
+  if (x.st) return GATO_OK;
+  int dev = 0;
+  GATO_CUDA_TRY(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lk(g_keep_mu);
+    for (size_t i = 0; i < g_side.size(); ++i)
+      if (g_side[i].dev == dev) {
+        x = g_side[i];
+        g_side.erase(g_side.begin() + i);
+        return GATO_OK;
+      }
+  }
+  GATO_CUDA_TRY(cudaStreamCreateWithFlags(&x.st, cudaStreamNonBlocking));
+  GATO_CUDA_TRY(cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming));
+  GATO_CUDA_TRY(cudaEventCreateWithFlags(&x.join, cudaEventDisableTiming));
+  x.dev = dev;
+  return GATO_OK;
+}
+
+void side_put(SideStream& x) {
+  if (!x.st) return;
+  if (x.fork && x.join) {
+    std::lock_guard<std::mutex> lk(g_keep_mu);
+    if ((int)g_side.size() < kSideKeep) {
+      g_side.push_back(x);
+      x = SideStream{};
+      return;
+    }
+  }
+  cudaStreamSynchronize(x.st);
+  cudaStreamDestroy(x.st);
+  if (x.fork) cudaEventDestroy(x.fork);
+  if (x.join) cudaEventDestroy(x.join);
+  x = SideStream{};
 }
 
 void release_stream_scratch(cudaStream_t s) {

@@ -1853,22 +1853,9 @@ __global__ void k_fz_init(double* g, double* binv) {
   binv[1] = 1.0;
 }
 
-// A stream of the Lanczos run's own, with the two events that fork work onto it and join it back
-// (released on every exit; pending work finishes first).
-struct FzSide {
-  cudaStream_t st = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-  int create() {
-    GATO_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    GATO_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-    GATO_CUDA_TRY(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-    return GATO_OK;
-  }
-  ~FzSide() {
-    if (join) cudaEventDestroy(join);
-    if (fork) cudaEventDestroy(fork);
-    if (st) cudaStreamDestroy(st);
-  }
+// The Lanczos run's own side stream (given back on every exit).
+struct FzSide : SideStream {
+  ~FzSide() { side_put(*this); }
 };
 
 int lanczos_fused(gato_operator& op, const void* psi0, int m, int K, double tol, float* Vb, double* evals,
@@ -1886,7 +1873,7 @@ int lanczos_fused(gato_operator& op, const void* psi0, int m, int K, double tol,
   GATO_TRY(raise_smem_limit(reinterpret_cast<const void*>(k_fz_sweep), kFzSmemCap));
   if (n > INT32_MAX) return fail(GATO_EUNSUPPORTED, "lanczos: field too large for the sweep's tensor map");
   FzSide side;
-  GATO_TRY(side.create());
+  GATO_TRY(side_get(side));
   for (int j = 0; j < m; ++j) {
     const float* wh = j == 0 ? Vb : f.wh;   // v_0 itself (beta = 1, c = g = 0) at the first step
     const int ce = fz_ce(j, n);

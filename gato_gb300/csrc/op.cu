@@ -27,6 +27,8 @@ int exchange_args(PassArgs& a, const void* psi, const void* orbitals, int n_orb,
 
 namespace {
 
+constexpr int kOpDoubles = 16;
+
 template <typename T>
 __global__ void k_vext_energy(const T* __restrict__ orb, int n, const T* __restrict__ V, int64_t npts,
                               double* part) {
@@ -54,20 +56,11 @@ __global__ void k_sum_scaled(const double* in, int n, double scale, double* out)
 
 }  // namespace
 
-// The operator's side stream and its fork/join events, created on first use.
-static int op_side(gato_operator& op) {
-  if (op.side) return GATO_OK;
-  GATO_CUDA_TRY(cudaStreamCreateWithFlags(&op.side, cudaStreamNonBlocking));
-  GATO_CUDA_TRY(cudaEventCreateWithFlags(&op.ev_fork, cudaEventDisableTiming));
-  GATO_CUDA_TRY(cudaEventCreateWithFlags(&op.ev_join, cudaEventDisableTiming));
-  return GATO_OK;
-}
-
 // out[b] = (-1/2 L + V) psi[b] (+ V_nl psi[b]) for nb fields, on stream ls.
 static int local_part(gato_operator& op, const void* in, void* out, int nb, cudaStream_t ls) {
   const double coef = -0.5 / (op.h * op.h);
   GATO_TRY(stencil_apply(op.dtype, in, op.V, out, nb, op.N, op.N, op.N, op_n3(op), coef, op.boundary,
-                         op.order, nullptr, op.dV, ls, ls == op.side && ls != nullptr));
+                         op.order, nullptr, op.dV, ls, ls == op.side.st && ls != nullptr));
   if (op.nl) GATO_TRY(nonlocal_apply(op.nl->n, in, out, nb, ls));
   return GATO_OK;
 }
@@ -78,12 +71,12 @@ static int fork_local(gato_operator& op, const void* in, void* out, int nb, cuda
                       cudaEvent_t* join) {
   *join = nullptr;
   if (!op.overlap) return local_part(op, in, out, nb, s);
-  GATO_TRY(op_side(op));
-  GATO_CUDA_TRY(cudaEventRecord(op.ev_fork, s));
-  GATO_CUDA_TRY(cudaStreamWaitEvent(op.side, op.ev_fork, 0));
-  GATO_TRY(local_part(op, in, out, nb, op.side));
-  GATO_CUDA_TRY(cudaEventRecord(op.ev_join, op.side));
-  *join = op.ev_join;
+  GATO_TRY(side_get(op.side));
+  GATO_CUDA_TRY(cudaEventRecord(op.side.fork, s));
+  GATO_CUDA_TRY(cudaStreamWaitEvent(op.side.st, op.side.fork, 0));
+  GATO_TRY(local_part(op, in, out, nb, op.side.st));
+  GATO_CUDA_TRY(cudaEventRecord(op.side.join, op.side.st));
+  *join = op.side.join;
   return GATO_OK;
 }
 
@@ -110,7 +103,7 @@ static void block_pairs(PassArgs& a, const gato_operator& op, void* out, bool en
     // The spectral energy pass sums both parts of a field with one weight: the diagonal pairs
     // (weight -1) and the off-diagonal ones (weight -2) pair up among themselves, and what is left
     // over rides alone at the end with the density (lone real fields cost half a field).
-    a.in[n] = op.rho;
+    a.in[n] = op.rho.p;
     int nf = 0, nl = 0;
     PartDesc lone[3];
     lone[nl].a = (int8_t)n;
@@ -137,7 +130,7 @@ static void block_pairs(PassArgs& a, const gato_operator& op, void* out, bool en
   }
   if (energy) {
     // the density rides first: E_H = 1/2 dV sum rho J[rho]
-    a.in[n] = op.rho;
+    a.in[n] = op.rho.p;
     PartDesc& d = a.f[0].p[0];
     d.a = (int8_t)n;
     d.ew = 0.5;
@@ -183,23 +176,15 @@ extern "C" int gato_op_create(int dtype, int N, double h, int order, int boundar
   op->dV = h * h * h;
   op->order = order;
   op->boundary = boundary;
-  if (cudaMalloc(&op->dscratch, 64 * sizeof(double)) != cudaSuccess) {
-    delete op;
-    return fail(GATO_ENOMEM, "gato_op_create: allocation failed");
-  }
   *out = op;
   return GATO_OK;
 }
 
 extern "C" int gato_op_destroy(gato_op_t op) {
   if (!op) return GATO_OK;
-  free_after_pending({op->dscratch, op->rho, op->jbuf});   // waits for the device first
-  if (op->side) {
-    cudaStreamSynchronize(op->side);
-    cudaStreamDestroy(op->side);
-    cudaEventDestroy(op->ev_fork);
-    cudaEventDestroy(op->ev_join);
-  }
+  ws_put(op->rho);
+  ws_put(op->jbuf);
+  side_put(op->side);
   delete op;
   return GATO_OK;
 }
@@ -249,18 +234,13 @@ extern "C" int gato_op_apply_block(gato_op_t op, void* out, void* stream) {
   if (jf && poisson_j_supported(op->pp->p)) {
     // pair potentials to J fields, then one elementwise pass: out_i -= sum_j phi_j J_ij
     const size_t need = (size_t)2 * a.nf * op_n3(*op) * op_esize(*op);
-    if (op->jbuf_bytes < need) {
-      free_after_pending({op->jbuf});
-      op->jbuf = nullptr;
-      op->jbuf_bytes = 0;
-      GATO_CUDA_TRY(cudaMalloc(&op->jbuf, need));
-      op->jbuf_bytes = need;
-    }
-    a.jbase = op->jbuf;
+    GATO_TRY(ws_get(op->jbuf, need, s));
+    a.jbase = op->jbuf.p;
     a.jstride = op_n3(*op);
     GATO_TRY(poisson_run(op->pp->p, a, EPI_J, false, nullptr, s));
     if (join) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
-    return pair_exchange(op->dtype, op->orbitals, op->n_orb, op->jbuf, out, op_n3(*op), s);
+    GATO_TRY(pair_exchange(op->dtype, op->orbitals, op->n_orb, op->jbuf.p, out, op_n3(*op), s));
+    return ws_used(op->jbuf, s);
   }
   return poisson_run(op->pp->p, a, EPI_ACC, true, nullptr, s, join);
 }
@@ -283,10 +263,12 @@ extern "C" int gato_op_energy_terms(gato_op_t op, const void* V_ext, double* ter
   cudaStream_t s = as_stream(stream);
   const int n = op->n_orb;
   const int64_t n3 = op_n3(*op);
-  double* ds = op->dscratch;   // [0..15] per-orbital kinetic, [16..] misc
+  if (n > kOpDoubles) return fail(GATO_EUNSUPPORTED, "energy terms: at most 16 orbitals");
+  const size_t rho_bytes = ((size_t)n3 * op_esize(*op) + 255) / 256 * 256;
+  GATO_TRY(ws_get(op->rho, rho_bytes + kOpDoubles * sizeof(double), s));
+  double* ds = (double*)((char*)op->rho.p + rho_bytes);   // per-orbital kinetic
   // kinetic: 2 sum_i <phi_i | T phi_i>, reduced inside the stencil (no store)
   const double coef = -0.5 / (op->h * op->h);
-  if (n > 16) return fail(GATO_EUNSUPPORTED, "energy terms: at most 16 orbitals");
   GATO_TRY(stencil_apply(op->dtype, op->orbitals, nullptr, nullptr, n, op->N, op->N, op->N, n3, coef,
                          op->boundary, op->order, ds, op->dV, s));
   k_sum_scaled<<<1, 32, 0, s>>>(ds, n, 2.0, terms + 0);
@@ -310,9 +292,9 @@ extern "C" int gato_op_energy_terms(gato_op_t op, const void* V_ext, double* ter
   else GATO_CUDA_TRY(cudaMemsetAsync(terms + 2, 0, sizeof(double), s));
   // hartree + exchange
   if (!op->pp) return fail(GATO_EBADARG, "energy terms need a Poisson plan");
-  if (!op->rho) GATO_CUDA_TRY(cudaMalloc(&op->rho, n3 * op_esize(*op)));
-  GATO_TRY(gato_density(op->dtype, op->orbitals, n, n3, op->rho, s));
+  GATO_TRY(gato_density(op->dtype, op->orbitals, n, n3, op->rho.p, s));
   PassArgs a;
   block_pairs(a, *op, nullptr, true);
-  return poisson_run(op->pp->p, a, EPI_ENERGY, false, terms + 3, s);
+  GATO_TRY(poisson_run(op->pp->p, a, EPI_ENERGY, false, terms + 3, s));
+  return ws_used(op->rho, s);
 }

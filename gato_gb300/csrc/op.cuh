@@ -14,16 +14,13 @@ struct gato_operator {
   gato_poisson_plan* pp = nullptr;
   const void* orbitals = nullptr;
   int n_orb = 0;
-  double* dscratch = nullptr;   // small device doubles
-  void* rho = nullptr;          // N^3 density scratch for the energy terms
-  void* jbuf = nullptr;         // pair potentials J_ij of the block apply
-  size_t jbuf_bytes = 0;
+  gato::WsBuf rho;              // energy terms: N^3 density, then kOpDoubles small doubles
+  gato::WsBuf jbuf;             // pair potentials J_ij of the block apply
   int block_epi = 0;            // block apply epilogue: 0 auto, 1 J fields + pair pass, 2 fused
   // The local part (stencil + V, non-local projectors) runs on a side stream beside the exchange's
   // transforms and joins before the first kernel that touches the outputs again.
   int overlap = 1;
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  gato::SideStream side;
 };
 
 namespace gato {

@@ -24,7 +24,7 @@ class Hamiltonian:
     def expectation(self, psi) -> torch.Tensor:
         """<psi|H|psi>, reduced inside the stencil kernel."""
         _, e = stencil(psi, self.grid.h, self.boundary, self.order, -0.5 / self.grid.h ** 2,
-                       V=self.V, dot=True)
+                       V=self.V, dot=True, store=False)
         return e
 
     def rayleigh(self, psi) -> torch.Tensor:

@@ -28,7 +28,7 @@ def kinetic_energy(psi, grid: Grid3D, boundary: str = "dirichlet", order: int = 
         return (kinetic_energy(psi.real.contiguous(), grid, boundary, order) * _real_norm(psi.real, grid)
                 + kinetic_energy(psi.imag.contiguous(), grid, boundary, order) * _real_norm(psi.imag, grid)
                 ) / _real_norm(psi, grid)
-    _, e = stencil(psi, grid.h, boundary, order, -0.5 / grid.h ** 2, dot=True)
+    _, e = stencil(psi, grid.h, boundary, order, -0.5 / grid.h ** 2, dot=True, store=False)
     return e / _real_norm(psi, grid)
 
 

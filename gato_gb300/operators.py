@@ -22,11 +22,12 @@ def _check(order: int, boundary: str) -> int:
 
 
 def stencil(psi, h: float, boundary: str, order: int, coef: float, V=None, out=None,
-            dot: bool = False):
+            dot: bool = False, store: bool = True):
     """out = coef * L(psi) + V * psi for psi of shape (nx, ny, nz) or (nb, nx, ny, nz).
 
     With dot=True also returns the per-field <psi, out> dV (the Hamiltonian
-    expectation) as float64 CUDA tensor(s).
+    expectation) as float64 CUDA tensor(s); store=False (with dot) computes
+    that alone and returns None in the place of out.
     """
     bcode = _check(order, boundary)
     psi = as_field(psi)
@@ -46,11 +47,12 @@ def stencil(psi, h: float, boundary: str, order: int, coef: float, V=None, out=N
         V = as_field(V, psi.dtype)
         if tuple(V.shape) != (nx, ny, nz):
             raise ValueError("potential shape does not match the field")
-    if out is None:
+    if out is None and (store or not dot):
         out = torch.empty_like(psi)
     dots = torch.empty(nb, dtype=torch.float64, device=psi.device) if dot else None
     _lib.call("gato_stencil_apply", _lib.dtype_code(psi), C.c_void_p(psi.data_ptr()),
-              C.c_void_p(V.data_ptr() if V is not None else None), C.c_void_p(out.data_ptr()),
+              C.c_void_p(V.data_ptr() if V is not None else None),
+              C.c_void_p(out.data_ptr() if out is not None else None),
               nb, nx, ny, nz, coef, bcode, order,
               C.c_void_p(dots.data_ptr() if dots is not None else None), h ** 3,
               C.c_void_p(_lib.stream()))

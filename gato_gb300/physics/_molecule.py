@@ -23,6 +23,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from ..geometry import Nuclei, _t, nuclear_repulsion
@@ -35,13 +36,13 @@ from ..solvers.poisson import get_plan
 
 def _coulomb_pair_grad(pos: torch.Tensor, Z) -> torch.Tensor:
     """d/dR of sum_{i<j} Z_i Z_j / |R_i - R_j|, (K, 3)."""
-    g = torch.zeros_like(pos)
-    for a in range(pos.shape[0]):
-        for b in range(pos.shape[0]):
-            if a != b:
-                d = pos[a] - pos[b]
-                g[a] -= Z[a] * Z[b] * d / torch.linalg.norm(d) ** 3
-    return g
+    p, z = pos.cpu().numpy(), np.asarray(Z, dtype=np.float64)
+    d = p[:, None, :] - p[None, :, :]
+    r = np.sqrt((d * d).sum(-1))
+    np.fill_diagonal(r, 1.0)   # d is 0 there
+    with np.errstate(divide="ignore", invalid="ignore"):   # coincident nuclei: nan, as the formula
+        g = -((z[:, None] * z[None, :] / r ** 3)[:, :, None] * d).sum(1)
+    return torch.from_numpy(g).to(pos.device)
 
 
 class HGHModel:

@@ -77,7 +77,7 @@ def _check_elements(nuclei: Nuclei, elements) -> None:
 
 
 def _pos_list(nuclei: Nuclei):
-    return [float(v) for v in _t(nuclei.positions).detach().reshape(-1)]
+    return _t(nuclei.positions).detach().to(torch.float64).reshape(-1).tolist()
 
 
 def hgh_local_potential(nuclei: Nuclei, elements, grid: Grid3D, dtype=torch.float64) -> torch.Tensor:
