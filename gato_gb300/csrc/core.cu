@@ -194,7 +194,7 @@ int side_get(SideStream& x) {
   {
     std::lock_guard<std::mutex> lk(g_keep_mu);
     for (size_t i = 0; i < g_side.size(); ++i)
-      if (g_side[i].dev == dev) {
+      if (g_side[i].dev == dev && !is_capturing(g_side[i].st)) {   // not in another's unfinished capture
         x = g_side[i];
         g_side.erase(g_side.begin() + i);
         return GATO_OK;
@@ -211,7 +211,7 @@ void side_put(SideStream& x) {
   if (!x.st) return;
   if (x.fork && x.join) {
     std::lock_guard<std::mutex> lk(g_keep_mu);
-    if ((int)g_side.size() < kSideKeep) {
+    if ((int)g_side.size() < kSideKeep || is_capturing(x.st)) {   // a stream in a capture is not destroyed
       g_side.push_back(x);
       x = SideStream{};
       return;

@@ -297,6 +297,16 @@ int launch_cols(int mode, const T2* in, T2* out, const ColGeom& g, int outer, in
   return GATO_OK;
 }
 
+// Whether a call's transforms run as two strands, half of the fields each on its own stream: every
+// pass has a last wave that leaves SMs idle and the passes have unlike bounds (memory, the FP64 or FP32
+// pipe, barriers), so one strand fills the other's gaps. Measured, one strand against two, exchange of
+// 3 / 4 / 5 / 8 orbitals, us. FP64: 71 / 41 / 77 / 60 against 52 / 43 / 58 / 54 at N = 16, 113 / 90 / 148 /
+// 151 against 78 / 81 / 115 / 138 at 32, 1076 / 1245 / 1682 / 2480 against 949 / 1168 / 1543 / 2331 at 80,
+// 3344 / 4304 / 5496 / 8456 against 3268 / 4225 / 5410 / 8513 at 128. FP32: 46 / 46 / 56 / 68 against 44 /
+// 42 / 54 / 65 at N = 64, 192 / 201 / 286 / 387 against 182 / 187 / 272 / 353 at 128; below, the fork and the
+// extra launches cost what the overlap gives (30 / 30 / 39 / 43 against 35 / 30 / 38 / 42 at N = 48).
+bool two_strands(size_t ts, int N) { return ts == 8 || N >= 64; }
+
 template <typename T>
 int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, double* energy_dev,
               cudaStream_t s, cudaEvent_t join) {
@@ -357,7 +367,7 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
     if (sizeof(T) == 4 && (nlone < args.nf || N < 64)) nlone = 0;
   }
   const int nfull = args.nf - nlone;
-  const int gfull = (nfull + group - 1) / group, ngroups = gfull + (nlone + group - 1) / group;
+  const int ngroups = (args.nf + group - 1) / group;
   if (epi == EPI_ENERGY && !fe && (int64_t)ngroups * 2 * nblk_i > pl.npart_cap)
     return fail(GATO_EUNSUPPORTED, "poisson: energy partials exceed plan capacity");
   if (Lf == 0) {
@@ -368,74 +378,87 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
   ColGeom gy{nrows * M, (int64_t)N * M * M, (int64_t)N * M, (int64_t)M * M, M, M, M, N, M};
   ColGeom gx{(int64_t)N * M * M, (int64_t)N * M * M, M, M, (int64_t)M * M, (int64_t)M * M, M, N, N};
   ColGeom gyi{(int64_t)N * M * M, nrows * M, (int64_t)M * M, (int64_t)N * M, M, M, M, M, N};
-  for (int g = 0; g < ngroups; ++g) {
-    const bool lone = g >= gfull;
-    const int f0 = lone ? nfull + (g - gfull) * group : g * group;
-    const int nfg = std::min(group, (lone ? args.nf : nfull) - f0);
+  if (Lf > 0) {
+    // register-resident two-pass engine: everything but the accumulating z inverse of n fields from
+    // f0, in the buffers from field `at` on
+    auto half = [&](ColGeom q, int tile) {   // the N + 1 columns of lone fields, rounded up to whole tiles
+      q.ncols = std::min(M, (N + tile) / tile * tile);
+      return q;
+    };
+    auto transform = [&](int f0, int n, int at, bool lone, cudaStream_t st) -> int {
+      T2* P1 = S1 + (int64_t)at * nrows * M;
+      T2* P2 = S2 + (int64_t)at * N * M * M;
+      // engine 0: multi-field z forward from two fields, 2: never, 3: from three
+      if (lone) GATO_TRY(fast::rows_fwd_real<T>(M, args, f0, n, P1, tw2, st));
+      else GATO_TRY(fast::rows_fwd<T>(M, args, f0, n, P1, tw2, pl.engine == 2 ? 0 : (pl.engine == 3 ? 1 : (pl.engine == 4 ? 3 : 2)), st));
+      if (packed) {
+        // FP32 column passes on the packed two-line engine (S2 in the split pair layout)
+        const float4* t4 = (const float4*)pl.tw4;
+        GATO_TRY(fast::packed_cols(M, COL_FWD, (const float2*)P1, (float2*)P2, lone ? half(gy, 16) : gy, N, n, t4,
+                                   nullptr, pl.H, st));
+        GATO_TRY(fast::packed_cols(M, COL_FMI, (const float2*)P2, (float2*)P2, lone ? half(gx, 16) : gx, M, n, t4,
+                                   (const float*)pl.ghat2, pl.H, st));
+        GATO_TRY(fast::packed_cols(M, COL_INV, (const float2*)P2, (float2*)P1, lone ? half(gyi, 16) : gyi, N, n, t4,
+                                   nullptr, pl.H, st));
+      } else {
+        GATO_TRY(fast::cols<T>(M, COL_FWD, P1, P2, lone ? half(gy, Lf) : gy, N, n, tw2, nullptr, pl.H, st));
+        if constexpr (sizeof(T) == 8) {
+          if (fe) {
+            fa.f0 = f0;
+            fa.half = lone;
+            return fast::cols_fe<T>(M, P2, gx, M, n, tw2, (const T*)pl.ghat, pl.H, fa, st);
+          }
+        }
+        GATO_TRY(fast::cols<T>(M, COL_FMI, P2, P2, lone ? half(gx, Lf) : gx, M, n, tw2, (const T*)pl.ghat, pl.H, st));
+        GATO_TRY(fast::cols<T>(M, COL_INV, P2, P1, lone ? half(gyi, Lf) : gyi, N, n, tw2, nullptr, pl.H, st));
+      }
+      if (epi != EPI_J) return GATO_OK;
+      return lone ? fast::rows_inv_real<T>(M, args, f0, n, P1, tw2, 0, true, st)
+                  : fast::rows_inv_j<T>(M, args, f0, n, P1, tw2, st);
+    };
+    for (int f0 = 0, g = 0; f0 < args.nf; ++g) {   // as many fields as the buffers hold
+      const int nf = std::min(group, std::max(nfull - f0, 0)), lf0 = f0 + nf;
+      const int nl = lf0 >= nfull ? std::min(group - nf, args.nf - lf0) : 0;
+      // two strands of about equal work, the second on the plan's own stream
+      int na = nf, la = nl;
+      if (two_strands(sizeof(T), N)) {
+        const int share = (2 * nf + nl + 1) / 2;
+        na = std::min(nf, (share + 1) / 2);
+        la = na == nf ? std::min(nl, std::max(share - 2 * nf, 0)) : 0;
+      }
+      const bool fork = na < nf || la < nl;
+      int rc = GATO_OK;
+      if (fork) {
+        GATO_CUDA_TRY(cudaEventRecord(pl.side.fork, s));
+        GATO_CUDA_TRY(cudaStreamWaitEvent(pl.side.st, pl.side.fork, 0));
+        if (rc == GATO_OK && na < nf) rc = transform(f0 + na, nf - na, na, false, pl.side.st);
+        if (rc == GATO_OK && la < nl) rc = transform(lf0 + la, nl - la, nf + la, true, pl.side.st);
+      }
+      if (rc == GATO_OK && na > 0) rc = transform(f0, na, 0, false, s);
+      if (rc == GATO_OK && la > 0) rc = transform(lf0, la, nf, true, s);
+      if (fork) {
+        GATO_CUDA_TRY(cudaEventRecord(pl.side.join, pl.side.st));
+        GATO_CUDA_TRY(cudaStreamWaitEvent(s, pl.side.join, 0));
+      }
+      if (rc != GATO_OK) return rc;
+      if (join && g == 0 && epi == EPI_ACC) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
+      if (epi != EPI_J && !fe) {
+        if (nf > 0)
+          GATO_TRY(fast::rows_inv<T>(M, args, f0, nf, S1, tw2, accumulate || f0 > 0 ? 1 : 0, epi == EPI_ENERGY,
+                                     pl.partials + (int64_t)g * nblk_i, (int64_t)ngroups * nblk_i, s));
+        if (nl > 0)
+          GATO_TRY(fast::rows_inv_real<T>(M, args, lf0, nl, S1 + (int64_t)nf * nrows * M, tw2,
+                                          accumulate || lf0 > 0 ? 1 : 0, false, s));
+      }
+      f0 = lf0 + nl;
+    }
+  }
+  for (int g = 0; g < ngroups && Lf == 0; ++g) {
+    const int f0 = g * group;
+    const int nfg = std::min(group, args.nf - f0);
     const bool acc_here = accumulate || g > 0;
     double* part = pl.partials + (int64_t)g * nblk_i;
     const int64_t sstride = (int64_t)ngroups * nblk_i;
-    if (Lf > 0) {
-      // register-resident two-pass engine
-      if (lone) {
-        auto half = [&](ColGeom q, int tile) {   // the N + 1 columns, rounded up to whole tiles
-          q.ncols = std::min(M, (N + tile) / tile * tile);
-          return q;
-        };
-        GATO_TRY(fast::rows_fwd_real<T>(M, args, f0, nfg, S1, tw2, s));
-        if (packed) {
-          const float4* t4 = (const float4*)pl.tw4;
-          GATO_TRY(fast::packed_cols(M, COL_FWD, (const float2*)S1, (float2*)S2, half(gy, 16), N, nfg, t4, nullptr, pl.H, s));
-          GATO_TRY(fast::packed_cols(M, COL_FMI, (const float2*)S2, (float2*)S2, half(gx, 16), M, nfg, t4,
-                                     (const float*)pl.ghat2, pl.H, s));
-          GATO_TRY(fast::packed_cols(M, COL_INV, (const float2*)S2, (float2*)S1, half(gyi, 16), N, nfg, t4, nullptr, pl.H, s));
-        } else {
-          GATO_TRY(fast::cols<T>(M, COL_FWD, S1, S2, half(gy, Lf), N, nfg, tw2, nullptr, pl.H, s));
-          if constexpr (sizeof(T) == 8) {
-            if (fe) {
-              fa.f0 = f0;
-              fa.half = 1;
-              GATO_TRY(fast::cols_fe<T>(M, S2, gx, M, nfg, tw2, (const T*)pl.ghat, pl.H, fa, s));
-              continue;
-            }
-          }
-          GATO_TRY(fast::cols<T>(M, COL_FMI, S2, S2, half(gx, Lf), M, nfg, tw2, (const T*)pl.ghat, pl.H, s));
-          GATO_TRY(fast::cols<T>(M, COL_INV, S2, S1, half(gyi, Lf), N, nfg, tw2, nullptr, pl.H, s));
-        }
-        if (join && g == 0 && epi == EPI_ACC) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
-        GATO_TRY(fast::rows_inv_real<T>(M, args, f0, nfg, S1, tw2, acc_here ? 1 : 0, epi == EPI_J, s));
-        continue;
-      }
-      // engine 0: multi-field z forward from two fields, 2: never, 3: from three
-      GATO_TRY(fast::rows_fwd<T>(M, args, f0, nfg, S1, tw2, pl.engine == 2 ? 0 : (pl.engine == 3 ? 1 : (pl.engine == 4 ? 3 : 2)), s));
-      if (packed) {
-        // FP32 column passes on the packed two-line engine (S2 in the split pair layout)
-        GATO_TRY(fast::packed_cols(M, COL_FWD, (const float2*)S1, (float2*)S2, gy, N, nfg,
-                                   (const float4*)pl.tw4, nullptr, pl.H, s));
-        GATO_TRY(fast::packed_cols(M, COL_FMI, (const float2*)S2, (float2*)S2, gx, M, nfg,
-                                   (const float4*)pl.tw4, (const float*)pl.ghat2, pl.H, s));
-        GATO_TRY(fast::packed_cols(M, COL_INV, (const float2*)S2, (float2*)S1, gyi, N, nfg,
-                                   (const float4*)pl.tw4, nullptr, pl.H, s));
-      } else {
-      GATO_TRY(fast::cols<T>(M, COL_FWD, S1, S2, gy, N, nfg, tw2, nullptr, pl.H, s));
-      if constexpr (sizeof(T) == 8) {
-        if (fe) {
-          fa.f0 = f0;
-          GATO_TRY(fast::cols_fe<T>(M, S2, gx, M, nfg, tw2, (const T*)pl.ghat, pl.H, fa, s));
-          continue;
-        }
-      }
-      GATO_TRY(fast::cols<T>(M, COL_FMI, S2, S2, gx, M, nfg, tw2, (const T*)pl.ghat, pl.H, s));
-      GATO_TRY(fast::cols<T>(M, COL_INV, S2, S1, gyi, N, nfg, tw2, nullptr, pl.H, s));
-      }
-      if (join && g == 0 && epi == EPI_ACC) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
-      if (epi == EPI_J)
-        GATO_TRY(fast::rows_inv_j<T>(M, args, f0, nfg, S1, tw2, s));
-      else
-        GATO_TRY(fast::rows_inv<T>(M, args, f0, nfg, S1, tw2, acc_here ? 1 : 0, epi == EPI_ENERGY, part,
-                                   sstride, s));
-      continue;
-    }
     if (epi == EPI_J) return fail(GATO_EUNSUPPORTED, "poisson: J output needs the register engine");
     // 1. z forward with the pair-density prologue
     k_rows_fwd<T><<<dim3((unsigned)((nrows + Lr - 1) / Lr), nfg), kFftThreads, sm_r, s>>>(
@@ -613,11 +636,12 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
   const int Lc = dtype == GATO_F64 ? fast::rows_L<double>(M) : 0;
   if (Lc > 0) pl.npart_cap = std::max(pl.npart_cap, 2 * 2 * max_fields * M * ((M + Lc - 1) / Lc));
   GATO_CUDA_TRY(cudaMalloc(&pl.partials, (size_t)pl.npart_cap * sizeof(double)));
-  return GATO_OK;
+  return side_get(pl.side);
 }
 
 static void plan_free(PoissonPlan& pl) {
   free_after_pending({pl.ghat, pl.tw, pl.tw2, pl.tw4, pl.ghat2, pl.S1, pl.S2, pl.partials});
+  side_put(pl.side);
   pl = PoissonPlan{};
 }
 
