@@ -80,6 +80,33 @@ int ws_get(WsBuf& b, size_t bytes, cudaStream_t s);   // b holds at least `bytes
 int ws_used(WsBuf& b, cudaStream_t s);                // the work queued on s so far uses b
 void ws_put(WsBuf& b);                                // gives b back
 
+// Launches a kernel that may begin while the one ahead of it in the stream drains: its launch latency and
+// the work it does before gdc_wait (ptx.cuh: barriers, constant tables) fall under the predecessor's end.
+// Every block calls gdc_wait before it reads or writes anything an earlier kernel touches, so a kernel
+// that has ended vouches for all before it; and it takes no const __restrict__ pointers, whose loads could
+// move ahead of the wait. Exchange of 3 / 8 orbitals, plain launches against these, us: FP32 24 / 30
+// against 14 / 18 at N = 16, 27 / 43 against 19 / 31 at 40, 42 / 66 against 35 / 56 at 64, 182 / 353
+// against 177 / 348 at 128; FP64 52 / 54 against 38 / 46 at N = 16, 80 / 136 against 71 / 130 at 32,
+// 1431 / 3656 against 1426 / 3655 at 96. No FFT kernel lets its successor begin earlier still (gdc_launch
+// at its start): the successor's waiting blocks take the places of a second strand's and land unevenly on
+// the SMs (FP32 block at 128^3 453 -> 488, FP64 exchange of 2 orbitals at 40^3 103 -> 188).
+template <typename... P, typename... A>
+int launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  GATO_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, P(a)...));
+  count_launch();
+  return GATO_OK;
+}
+
 // A side stream with the events that fork work onto it and join it back. Kept like workspace (at most
 // kSideKeep): work left in the stream merely runs before its next owner's.
 struct SideStream {

@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   constexpr int TWN = MODE == COL_FMI ? Tab::N : (MODE == COL_FWD ? Tab::NF : Tab::NI);
   const T2* twi = tws + (Tab::OI - TW0);
   const TwPrefetch<T2, TWN, L * Shape<R1, R2>::RMAX> twp(tw + TW0);
+  gdc_wait();
   const int outer = blockIdx.x, col0 = blockIdx.y * L, f = blockIdx.z;
   const int t = threadIdx.x;
   const int line = t % L, q = t / L;   // q: n2 in stages 1/B, k1 in stages 2/A
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + M * LP;
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, L * Shape<R1, R2>::RMAX> twp(tw);
+  gdc_wait();
   const int outer = blockIdx.x, col0 = blockIdx.y * L, f = blockIdx.z;
   const int t = threadIdx.x;
   const int line = t % L, q = t / L;
@@ -267,6 +269,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, NT> twp(tw);
+  gdc_wait();
   const int p = blockIdx.y;
   const FieldDesc& fd = args.f[f0 + p];
   const int64_t nrows = (int64_t)N * N;
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
   T* stage = reinterpret_cast<T*>(tws + TwTab<T2, R1, R2>::NF);   // [slot][line][z], rows of NP
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, NT> twp(tw);
+  gdc_wait();
   const int64_t row0 = (int64_t)blockIdx.x * L;
   const int64_t nrows = (int64_t)N * N;
   if constexpr (BULK) {
@@ -474,6 +478,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
     if (bad_align && err) atomicExch(err, 110);
   }
   for (int i = threadIdx.x; i < TwTab<T2, R1, R2>::NF; i += NT) tws[i] = tw[i];
+  gdc_wait();
   __syncthreads();
   if (s_misaligned) return;
   auto issue = [&](int blk, int slot) {
@@ -564,6 +569,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX, (rows_inv_min_ctas<T,
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NI, NT> twp(tw + TwTab<T2, R1, R2>::OI);
+  gdc_wait();
   const int64_t nrows = (int64_t)N * N;
   const RowMap<R1, R2, L> q;
   const int j = q.n2;
@@ -691,6 +697,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * LS;
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, NT> twp(tw);
+  gdc_wait();
   const int p = blockIdx.y;
   const PartDesc& pd = args.f[f0 + p].p[0];
   const int64_t npair = (int64_t)N * N / 2;
@@ -748,6 +755,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NI, NT> twp(tw + TwTab<T2, R1, R2>::OI);
+  gdc_wait();
   const int p = blockIdx.y;
   const int64_t npair = (int64_t)N * N / 2;
   const RowMap<R1, R2, L> q;
@@ -819,6 +827,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   T2* buf = reinterpret_cast<T2*>(smraw);
   T2* tws = buf + L * RowBuf<R1, R2>::LS;
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NI, NT> twp(tw + TwTab<T2, R1, R2>::OI);
+  gdc_wait();
   const int p = blockIdx.y;
   const int64_t nrows = (int64_t)N * N;
   const RowMap<R1, R2, L> q;
@@ -876,15 +885,14 @@ struct Launch {
     const size_t sm = sm_cols(mode);
     if (mode == COL_FWD) {
       GATO_TRY(smem_attr(k_cols<T, R1, R2, L, COL_FWD, FULL>, sm));
-      k_cols<T, R1, R2, L, COL_FWD, FULL><<<grid, NT, sm, s>>>(in, out, g, tw, ghat, H);
+      GATO_TRY(launch_chained(k_cols<T, R1, R2, L, COL_FWD, FULL>, grid, NT, sm, s, in, out, g, tw, ghat, H));
     } else if (mode == COL_INV) {
       GATO_TRY(smem_attr(k_cols<T, R1, R2, L, COL_INV, FULL>, sm));
-      k_cols<T, R1, R2, L, COL_INV, FULL><<<grid, NT, sm, s>>>(in, out, g, tw, ghat, H);
+      GATO_TRY(launch_chained(k_cols<T, R1, R2, L, COL_INV, FULL>, grid, NT, sm, s, in, out, g, tw, ghat, H));
     } else {
       GATO_TRY(smem_attr(k_cols<T, R1, R2, L, COL_FMI, FULL>, sm));
-      k_cols<T, R1, R2, L, COL_FMI, FULL><<<grid, NT, sm, s>>>(in, out, g, tw, ghat, H);
+      GATO_TRY(launch_chained(k_cols<T, R1, R2, L, COL_FMI, FULL>, grid, NT, sm, s, in, out, g, tw, ghat, H));
     }
-    GATO_LAUNCH_TRY();
     return GATO_OK;
   }
   static int cols_fe(const T2* in, const ColGeom& g, int outer, int nf, const T2* tw, const T* ghat, int H,
@@ -892,16 +900,14 @@ struct Launch {
     dim3 grid(outer, (g.ncols + L - 1) / L, nf);
     const size_t sm = sm_cols(COL_FWD);
     GATO_TRY(smem_attr(k_cols_fe<T, R1, R2, L, FULL>, sm));
-    k_cols_fe<T, R1, R2, L, FULL><<<grid, NT, sm, s>>>(in, g, tw, ghat, H, fa);
-    GATO_LAUNCH_TRY();
+    GATO_TRY(launch_chained(k_cols_fe<T, R1, R2, L, FULL>, grid, NT, sm, s, in, g, tw, ghat, H, fa));
     return GATO_OK;
   }
   static int rows_fwd_real(const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw, cudaStream_t s) {
     const size_t sm = sm_rows(true);
     GATO_TRY(smem_attr(k_rows_fwd_real<T, R1, R2, L>, sm));
     const unsigned nblk = (unsigned)(((int64_t)N * N / 2 + L - 1) / L);
-    k_rows_fwd_real<T, R1, R2, L><<<dim3(nblk, nfg), NT, sm, s>>>(a, f0, S1, tw);
-    GATO_LAUNCH_TRY();
+    GATO_TRY(launch_chained(k_rows_fwd_real<T, R1, R2, L>, dim3(nblk, nfg), NT, sm, s, a, f0, S1, tw));
     return GATO_OK;
   }
   // j: potentials to the J fields (nfg fields at once), else one field's terms to the outputs
@@ -911,12 +917,11 @@ struct Launch {
     const unsigned nblk = (unsigned)(((int64_t)N * N / 2 + L - 1) / L);
     if (j) {
       GATO_TRY(smem_attr(k_rows_inv_real<T, R1, R2, L, true>, sm));
-      k_rows_inv_real<T, R1, R2, L, true><<<dim3(nblk, nfg), NT, sm, s>>>(a, f0, S1, tw, 0);
+      GATO_TRY(launch_chained(k_rows_inv_real<T, R1, R2, L, true>, dim3(nblk, nfg), NT, sm, s, a, f0, S1, tw, 0));
     } else {
       GATO_TRY(smem_attr(k_rows_inv_real<T, R1, R2, L, false>, sm));
-      k_rows_inv_real<T, R1, R2, L, false><<<dim3(nblk, 1), NT, sm, s>>>(a, f0, S1, tw, accumulate);
+      GATO_TRY(launch_chained(k_rows_inv_real<T, R1, R2, L, false>, dim3(nblk, 1), NT, sm, s, a, f0, S1, tw, accumulate));
     }
-    GATO_LAUNCH_TRY();
     return GATO_OK;
   }
   // multi: 0 per-field CTAs, 1 multi-field CTAs from three fields up, 2 from two fields up
@@ -970,24 +975,20 @@ struct Launch {
           wave[ri.nin].store(w);
         }
         const unsigned pg = (unsigned)std::min<int64_t>(grid, (int64_t)w);
-        kern<<<pg, LM * Shape<R1, R2>::RMAX, smp, s>>>(a, ri, f0, nfg, S1, tw, device_error_word());
+        GATO_TRY(launch_chained(kern, pg, LM * Shape<R1, R2>::RMAX, smp, s, a, ri, f0, nfg, S1, tw, device_error_word()));
       } else if (bulk) {
         GATO_TRY(smem_attr(k_rows_fwd_multi<T, R1, R2, LM, true>, sm));
-        k_rows_fwd_multi<T, R1, R2, LM, true><<<grid, LM * Shape<R1, R2>::RMAX, sm, s>>>(
-            a, ri, f0, nfg, S1, tw, device_error_word());
+        GATO_TRY(launch_chained(k_rows_fwd_multi<T, R1, R2, LM, true>, grid, LM * Shape<R1, R2>::RMAX, sm, s, a, ri, f0, nfg, S1, tw, device_error_word()));
       } else {
         GATO_TRY(smem_attr(k_rows_fwd_multi<T, R1, R2, LM, false>, sm));
-        k_rows_fwd_multi<T, R1, R2, LM, false><<<grid, LM * Shape<R1, R2>::RMAX, sm, s>>>(
-            a, ri, f0, nfg, S1, tw, device_error_word());
+        GATO_TRY(launch_chained(k_rows_fwd_multi<T, R1, R2, LM, false>, grid, LM * Shape<R1, R2>::RMAX, sm, s, a, ri, f0, nfg, S1, tw, device_error_word()));
       }
-      GATO_LAUNCH_TRY();
       return GATO_OK;
     }
     const size_t sm = sm_rows(true);
     GATO_TRY(smem_attr(k_rows_fwd<T, R1, R2, L>, sm));
     const int64_t nrows = (int64_t)N * N;
-    k_rows_fwd<T, R1, R2, L><<<dim3((unsigned)((nrows + L - 1) / L), nfg), NT, sm, s>>>(a, f0, S1, tw);
-    GATO_LAUNCH_TRY();
+    GATO_TRY(launch_chained(k_rows_fwd<T, R1, R2, L>, dim3((unsigned)((nrows + L - 1) / L), nfg), NT, sm, s, a, f0, S1, tw));
     return GATO_OK;
   }
   template <int NO>
@@ -996,17 +997,14 @@ struct Launch {
     const size_t sm = sm_rows(false);
     const unsigned nblk = (unsigned)(((int64_t)N * N + L - 1) / L);
     GATO_TRY(smem_attr(k_rows_inv<T, R1, R2, L, NO>, sm));
-    k_rows_inv<T, R1, R2, L, NO><<<nblk, NT, sm, s>>>(a, f0, nfg, S1, tw, accumulate, partials,
-                                                       slot_stride);
-    GATO_LAUNCH_TRY();
+    GATO_TRY(launch_chained(k_rows_inv<T, R1, R2, L, NO>, nblk, NT, sm, s, a, f0, nfg, S1, tw, accumulate, partials, slot_stride));
     return GATO_OK;
   }
   static int rows_inv_j(const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, cudaStream_t s) {
     const size_t sm = sm_rows(false);
     const unsigned nblk = (unsigned)(((int64_t)N * N + L - 1) / L);
     GATO_TRY(smem_attr(k_rows_inv_j<T, R1, R2, L>, sm));
-    k_rows_inv_j<T, R1, R2, L><<<dim3(nblk, nfg), NT, sm, s>>>((T*)a.jbase, a.jstride, f0, S1, tw);
-    GATO_LAUNCH_TRY();
+    GATO_TRY(launch_chained(k_rows_inv_j<T, R1, R2, L>, dim3(nblk, nfg), NT, sm, s, (T*)a.jbase, a.jstride, f0, S1, tw));
     return GATO_OK;
   }
   static int rows_inv(const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,

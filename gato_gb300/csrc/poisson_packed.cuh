@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(PGeom<R1, R2, LPR, MODE>::NT)
     fence_barrier_init();
   }
   for (int i = t; i < R1 * R2; i += NT) tws[(i / R2) * G::TWS + i % R2] = tw4[i];
+  gdc_wait();
   __syncthreads();
   if (t == 0 && (int)blockIdx.x < ntiles) issue(blockIdx.x, 0);
   int it = 0;
@@ -212,9 +213,7 @@ struct LaunchP {
     }
     const int64_t ntiles = (int64_t)nf * outer * (g.ncols / CW);
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)w);
-    kern<<<grid, G::NT, G::SMEM, s>>>(tin, tg, out, g, outer, nf, tw4, device_error_word());
-    GATO_LAUNCH_TRY();
-    return GATO_OK;
+    return launch_chained(kern, grid, G::NT, G::SMEM, s, tin, tg, out, g, outer, nf, tw4, device_error_word());
   }
 
   // in: the pass's input buffer (S1 for the y forward, S2 otherwise), nfa fields allocated.

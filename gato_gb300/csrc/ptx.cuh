@@ -8,6 +8,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// Programmatic dependent launch: a kernel launched with launch_chained may begin once every block of the
+// kernel ahead of it in the stream has ended, and holds here until that kernel's writes are visible (at
+// once where there is nothing to wait for).
+__device__ __forceinline__ void gdc_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next chained kernel begin before this one's blocks have ended.
+__device__ __forceinline__ void gdc_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
                : "memory");

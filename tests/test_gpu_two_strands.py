@@ -12,7 +12,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 TOL = {torch.float64: 100 * 2.0 ** -53, torch.float32: 100 * 2.0 ** -24}
-CASES = [(torch.float64, 16), (torch.float64, 50), (torch.float32, 48), (torch.float32, 64), (torch.float32, 100)]
+CASES = [(torch.float64, 16), (torch.float64, 50), (torch.float32, 16), (torch.float32, 48), (torch.float32, 64), (torch.float32, 100)]
 
 
 def inputs(n, N, dtype, seed):
