@@ -1,6 +1,7 @@
 // Library core: error state, device error word, stream scratch, reductions,
 // TMA encoding, and the grid.py reductions of the C ABI.
 #include "common.cuh"
+#include "ptx.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -239,6 +240,7 @@ void release_stream_scratch(cudaStream_t s) {
 
 __global__ void k_finalize_sums(const double* partials, int nparts, double scale, double* out) {
   __shared__ double sh[32];
+  gdc_wait();
   const double* p = partials + (size_t)blockIdx.x * nparts;
   double v = 0.0;
   for (int i = threadIdx.x; i < nparts; i += blockDim.x) v += p[i];
@@ -246,12 +248,34 @@ __global__ void k_finalize_sums(const double* partials, int nparts, double scale
   if (threadIdx.x == 0) out[blockIdx.x] = v * scale;
 }
 
+// The same for many partials: one block's loads, latency after latency, so eight in flight a thread and 1024
+// threads (two sums of 49,152, the spectral energies of five fields at 128^3: 85 -> 19 us).
+constexpr int kManyParts = 4096, kManyThreads = 1024, kManyBatch = 8;
+__global__ void __launch_bounds__(kManyThreads) k_finalize_many(const double* partials, int nparts, double scale, double* out) {
+  __shared__ double sh[32];
+  gdc_wait();
+  const double* p = partials + (size_t)blockIdx.x * nparts;
+  double v = 0.0;
+  for (int i0 = threadIdx.x; i0 < nparts; i0 += kManyBatch * kManyThreads) {
+    double x[kManyBatch];
+#pragma unroll
+    for (int k = 0; k < kManyBatch; ++k) {
+      const int i = i0 + k * kManyThreads;
+      x[k] = i < nparts ? p[i] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kManyBatch; ++k) v += x[k];
+  }
+  v = block_sum(v, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = v * scale;
+}
+
 int finalize_sums(const double* partials, int nq, int nparts, double scale, double* out,
                   cudaStream_t s) {
   if (nq <= 0) return GATO_OK;
-  k_finalize_sums<<<nq, 256, 0, s>>>(partials, nparts, scale, out);
-  GATO_LAUNCH_TRY();
-  return GATO_OK;
+  if (nparts >= kManyParts)
+    return launch_chained(k_finalize_many, nq, kManyThreads, 0, s, partials, nparts, scale, out);
+  return launch_chained(k_finalize_sums, nq, 256, 0, s, partials, nparts, scale, out);
 }
 
 static PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
@@ -287,9 +311,9 @@ int encode_tma(void* out128, int dtype, const void* base, const TmaBox& b) {
 // ---- grid.py reductions --------------------------------------------------------
 
 template <typename T>
-__global__ void k_dot_partials(const T* __restrict__ a, const T* __restrict__ b, int64_t n,
-                               double* partials) {
+__global__ void k_dot_partials(const T* a, const T* b, int64_t n, double* partials) {
   __shared__ double sh[32];
+  gdc_wait();
   Acc<T> acc;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
