@@ -673,12 +673,13 @@ __device__ __forceinline__ void ws_load4(double2 (&v)[4][CG], const double* p, i
 // part[k * gridDim.x + block] = sum_i V_k[i] w[i], w = W - pre
 template <int VEC>
 __global__ void __launch_bounds__(32 * kWsMaxWarps, 1)
-    k_gemv_t_ws(const double* __restrict__ V, int64_t ld, int nk, const double* __restrict__ W, Pre<double> pre,
+    k_gemv_t_ws(const double* V, int64_t ld, int nk, const double* W, Pre<double> pre,
                 WsAlpha al, int64_t n, double* part) {
   extern __shared__ double wacc[];   // [warp][k]
   __shared__ double sh[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double sc[2];
+  gdc_wait();
   pre_scalars(pre, sc);
   if (al.part) {
     double v = 0.0;
@@ -756,13 +757,14 @@ __device__ __forceinline__ float to_float(double v, unsigned& big) {
 constexpr int kWsNWarps = 28;
 template <int VEC>
 __global__ void __launch_bounds__(32 * kWsNWarps, 1)
-    k_gemv_n_ws(const double* __restrict__ V, int64_t ld, int nk, double* __restrict__ W, Pre<double> pre,
-                const double* __restrict__ c_in, int64_t n, double* part) {
+    k_gemv_n_ws(const double* V, int64_t ld, int nk, double* W, Pre<double> pre, const double* c_in, int64_t n,
+                double* part) {
   extern __shared__ double wacc[];
   float* cs = reinterpret_cast<float*>(wacc);   // coefficients rounded once to FP32, zero up to a multiple of 4
   __shared__ double sh[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double sc[2];
+  gdc_wait();
   pre_scalars(pre, sc);
   for (int i = threadIdx.x; i < (nk + 3) / 4 * 4; i += blockDim.x) cs[i] = i < nk ? (float)c_in[i] : 0.f;
   __syncthreads();
@@ -840,6 +842,7 @@ __global__ void __launch_bounds__(256) k_beta_scale(T* W, int64_t n, const doubl
   constexpr int VEC = 16 / (int)sizeof(T);
   __shared__ double sh[32];
   __shared__ double s_beta, s_inv;
+  gdc_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nv = ((uintptr_t)W % 16) == 0 ? n / VEC : 0;   // 16-byte vectors
   V* W4 = reinterpret_cast<V*>(W);
@@ -1304,17 +1307,14 @@ int gemv_t_ws(const double* V, int64_t ld, int nk, const double* W, const Pre<do
   const size_t sm = (size_t)nw * nk * sizeof(double);
   auto kern = ws_vec2(V, n, W, pre) ? k_gemv_t_ws<2> : k_gemv_t_ws<1>;
   if (sm > 48 * 1024) GATO_TRY(raise_smem_limit(reinterpret_cast<const void*>(kern), sm));
-  kern<<<nblk, 32 * nw, sm, s>>>(V, ld, nk, W, pre, al, n, part);
-  GATO_LAUNCH_TRY();
-  return GATO_OK;
+  return launch_chained(kern, nblk, 32 * nw, sm, s, V, ld, nk, W, pre, al, n, part);
 }
 
 int gemv_n_ws(const double* V, int64_t ld, int nk, double* W, const Pre<double>& pre, const double* c, int64_t n,
               int nblk, double* part, cudaStream_t s) {
   auto kern = ws_vec2(V, n, W, pre) ? k_gemv_n_ws<2> : k_gemv_n_ws<1>;
-  kern<<<nblk, 32 * ws_warps(n, nblk, 0, 16, kWsNWarps), (size_t)(nk + 3) / 4 * 16, s>>>(V, ld, nk, W, pre, c, n, part);
-  GATO_LAUNCH_TRY();
-  return GATO_OK;
+  return launch_chained(kern, nblk, 32 * ws_warps(n, nblk, 0, 16, kWsNWarps), (size_t)(nk + 3) / 4 * 16, s, V, ld, nk, W,
+                        pre, c, n, part);
 }
 
 template <typename T>
@@ -1341,9 +1341,7 @@ int lz_step(T* Vb, int64_t n, double dV, int j, int passes, double* alphas, doub
       GATO_TRY(finalize_sums(z.part, nk, z.nblk_b, dV, z.coef, s));
       GATO_TRY(gemv_n_ws(Vb, n, nk, W, pp, z.coef, n, z.nblk_b, z.part, s));
     }
-    k_beta_scale<T><<<grid_for(n / 2 + 1, 256), 256, 0, s>>>(W, n, z.part, z.nblk_b, dV, betas + j);
-    GATO_LAUNCH_TRY();
-    return GATO_OK;
+    return launch_chained(k_beta_scale<T>, grid_for(n / 2 + 1, 256), 256, 0, s, W, n, z.part, z.nblk_b, dV, betas + j);
   } else {
   if (bulk_ok(Vb, n)) {
     // alpha_j = dV <v_j, w'>
@@ -1444,8 +1442,12 @@ int lz_finish(const T* Vb, int64_t n, int m, int K, double tol, const double* al
 // fz_stages). Only the FP32 basis takes this path: FP64 products would make
 // the sweep FP64-bound on GB300. After each sweep, k_fz_form sums the block
 // partials (one warp per row), forms alpha_j, the next correction row and w^_j;
-// k_fz_post2 forms beta_j and the next sweep's coefficients on the run's own
-// side stream while the operator is applied to w^_j.
+// k_fz_post2 forms beta_j and the next sweep's coefficients while the operator is
+// applied to w^_j. All are chained launches in one stream; k_fz_post2 lets a
+// local operator's stencil begin once k_fz_form is complete and run beside it
+// (64^3, m = 80, a run: post2 on a stream of its own, forked and joined by
+// events, 2937 us; chained in turn 2460; chained and beside 2329; 32^3 2224,
+// 1704, 1629; 128^3, m = 60, 6024, 5816, 5576).
 constexpr int kFzCE = 128;                  // the middle chunk width; n must be a multiple
 constexpr int kFzWarps = 8;                 // consumer warps
 constexpr int kFzThreads = 32 * (kFzWarps + 1);
@@ -1533,6 +1535,7 @@ __global__ void __maxnreg__(96)
     abort_flag = 0;
     fence_barrier_init();
   }
+  gdc_wait();
   for (int k = threadIdx.x; k <= j; k += blockDim.x) csg[k] = make_float2(k < j ? (float)c[k] : 0.f, (float)g[k]);
   __syncthreads();
   if (warp == kFzWarps) {   // producer
@@ -1674,11 +1677,11 @@ __global__ void __maxnreg__(96)
 // not by its 16 n bytes: the row sums run in four warps side by side, the first vectors are loaded before
 // them (64^3, warm: 10.6 -> 6.6 us). Launched with kFzFormThreads threads per block.
 constexpr int kFzFormThreads = 256;
-__global__ void __launch_bounds__(kFzFormThreads) k_fz_form(const float* __restrict__ U, const float* __restrict__ vm1, const float* __restrict__ vj,
-                          float* wh, int64_t n, const double* part, int G, double dV, double* alphas,
+__global__ void __launch_bounds__(kFzFormThreads) k_fz_form(const float* U, const float* vm1, const float* vj, float* wh, int64_t n, const double* part, int G, double dV, double* alphas,
                           const double* betas, double* dprev, double* Cm, int m, int j, double* partn) {
   __shared__ double sh[32];
   __shared__ double s_ad[4];   // a_j, d_{j-1}; this block's first Cm row: a_k, d_k
+  gdc_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t nv = n / 4, stride = (int64_t)gridDim.x * blockDim.x;
   const float4* U4 = reinterpret_cast<const float4*>(U);
@@ -1754,6 +1757,8 @@ __global__ void __launch_bounds__(kFzPost2Threads)
     k_fz_post2(const double* part, int nb, double dV, const double* Cm, int m, int j, const double* alphas,
                double* betas, double* binv, double* c_next, double* g_next) {
   __shared__ double sh[2][32];
+  gdc_wait();
+  gdc_launch();   // the operator apply runs beside: it reads w^_j alone, which is complete here
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const double* cj = Cm + (int64_t)j * m;
   // everything the block reads is loaded before the first barrier
@@ -1853,11 +1858,6 @@ __global__ void k_fz_init(double* g, double* binv) {
   binv[1] = 1.0;
 }
 
-// The Lanczos run's own side stream (given back on every exit).
-struct FzSide : SideStream {
-  ~FzSide() { side_put(*this); }
-};
-
 int lanczos_fused(gato_operator& op, const void* psi0, int m, int K, double tol, float* Vb, double* evals,
                   float* evecs, double* alphas, double* betas, int* flag, cudaStream_t s) {
   const int64_t n = op_n3(op);
@@ -1872,8 +1872,6 @@ int lanczos_fused(gato_operator& op, const void* psi0, int m, int K, double tol,
   GATO_LAUNCH_TRY();
   GATO_TRY(raise_smem_limit(reinterpret_cast<const void*>(k_fz_sweep), kFzSmemCap));
   if (n > INT32_MAX) return fail(GATO_EUNSUPPORTED, "lanczos: field too large for the sweep's tensor map");
-  FzSide side;
-  GATO_TRY(side_get(side));
   for (int j = 0; j < m; ++j) {
     const float* wh = j == 0 ? Vb : f.wh;   // v_0 itself (beta = 1, c = g = 0) at the first step
     const int ce = fz_ce(j, n);
@@ -1897,23 +1895,14 @@ int lanczos_fused(gato_operator& op, const void* psi0, int m, int K, double tol,
     }
     const int G = (int)std::min<int64_t>(std::min<int64_t>(n / ce, (int64_t)std::min(per_sm, 4) * f.sms),
                                          f.grid);
-    k_fz_sweep<<<G, kFzThreads, smj, s>>>(*reinterpret_cast<const CUtensorMap*>(tm), Vb, n, j, ce, nst, wh, f.z,
-                                          f.u, f.c, f.g, f.binv, f.part, device_error_word());
-    GATO_LAUNCH_TRY();
-    k_fz_form<<<f.nbf, kFzFormThreads, 0, s>>>(f.u, j > 0 ? Vb + (int64_t)(j - 1) * n : nullptr, Vb + (int64_t)j * n, f.wh, n,
-                                    f.part, G, dV, alphas, betas, f.dprev, f.Cm, m, j, f.partn);
-    GATO_LAUNCH_TRY();
-    // beta_j and the next sweep's coefficients on the side stream, beside the operator apply to w^_j
-    // (which reads neither); the next sweep, and the eigensolve after the last step, wait for them
-    GATO_CUDA_TRY(cudaEventRecord(side.fork, s));
-    GATO_CUDA_TRY(cudaStreamWaitEvent(side.st, side.fork, 0));
+    GATO_TRY(launch_chained(k_fz_sweep, G, kFzThreads, smj, s, *reinterpret_cast<const CUtensorMap*>(tm), Vb, n, j, ce,
+                            nst, wh, f.z, f.u, f.c, f.g, f.binv, f.part, device_error_word()));
+    GATO_TRY(launch_chained(k_fz_form, f.nbf, kFzFormThreads, 0, s, f.u, j > 0 ? Vb + (int64_t)(j - 1) * n : nullptr,
+                            Vb + (int64_t)j * n, f.wh, n, f.part, G, dV, alphas, betas, f.dprev, f.Cm, m, j, f.partn));
     constexpr int gpb = kFzPost2Threads / 32;   // g_i per block
-    k_fz_post2<<<(j + 2 + gpb - 1) / gpb, kFzPost2Threads, 0, side.st>>>(f.partn, f.nbf, dV, f.Cm, m, j, alphas,
-                                                                          betas, f.binv, f.c, f.g);
-    GATO_LAUNCH_TRY();
-    GATO_CUDA_TRY(cudaEventRecord(side.join, side.st));
-    if (j + 1 < m) GATO_TRY(op_apply(op, f.wh, f.z, s));
-    GATO_CUDA_TRY(cudaStreamWaitEvent(s, side.join, 0));
+    GATO_TRY(launch_chained(k_fz_post2, (j + 2 + gpb - 1) / gpb, kFzPost2Threads, 0, s, f.partn, f.nbf, dV, f.Cm, m, j,
+                            alphas, betas, f.binv, f.c, f.g));
+    if (j + 1 < m) GATO_TRY(op_apply(op, f.wh, f.z, s, true));
   }
   return lz_finish<float>(Vb, n, m, K, tol, alphas, betas, evals, evecs, flag, z, s);
 }

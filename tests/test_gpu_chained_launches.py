@@ -1,0 +1,63 @@
+"""Kernels chained by programmatic dependent launch: a Lanczos run, whose steps chain through every kernel
+of both forms, gives the same bits alone, back to back with other runs and beside them on another stream;
+sums of many partials match the same energies on the generic engine.
+
+The runs repeat the same kernels on the same inputs, so the comparison is exact. The energies are sums of
+the same terms, 25 levels of transform there and back and a factor of four for their accumulation: 100 eps.
+"""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def hamiltonian(N, dtype, seed):
+    from gato_gb300.grid import Grid3D
+    from gato_gb300.hamiltonian import Hamiltonian
+    g = torch.Generator().manual_seed(seed)
+    V = -torch.rand(N, N, N, generator=g, dtype=torch.float64)
+    H = Hamiltonian(Grid3D(N, 0.3 * N), V.to(dtype).cuda(), order=2)
+    return H, torch.rand(N, N, N, generator=g, dtype=torch.float64).to(dtype).cuda()
+
+
+@pytest.mark.parametrize("N,m", [(10, 8), (16, 40), (33, 24), (64, 40), (96, 12)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+def test_lanczos_alone_and_beside_others(N, m, dtype):
+    from gato_gb300.solvers.lanczos import lanczos
+    sets = [hamiltonian(N, dtype, s) for s in (1, 2)]
+
+    def run(k):
+        r = lanczos(sets[k][0], sets[k][1], n_iters=m, n_eigenstates=2)
+        return [x for x in (r if isinstance(r, (tuple, list)) else vars(r).values()) if torch.is_tensor(x)]
+    want = []
+    for k in range(2):
+        want.append(run(k))
+        torch.cuda.synchronize()
+    assert want[0] and all(torch.isfinite(x).all() for x in want[0] if x.is_floating_point())
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    got = []
+    for rep in range(4):
+        for k in range(2):
+            with torch.cuda.stream(streams[(k + rep) % 2]):
+                got.append((k, run(k)))
+        got += [(k, run(k)) for k in (1, 0)]
+    torch.cuda.synchronize()
+    for k, g in got:
+        assert all(torch.equal(a, b) for a, b in zip(g, want[k]))
+
+
+@pytest.mark.parametrize("N,n", [(64, 1), (64, 2), (64, 3), (100, 4)])
+def test_energies_of_many_partials(N, n):
+    from gato_gb300.autotune import set_plan
+    from gato_gb300.grid import Grid3D
+    from gato_gb300.scf import Operator, pair_fields
+    from gato_gb300.solvers.poisson import PoissonPlan
+    g = torch.Generator().manual_seed(N + n)
+    orb = torch.rand(n, N, N, N, generator=g, dtype=torch.float64).cuda()
+    plan = PoissonPlan(N, 0.2, 0.1, torch.float64, pair_fields(n))
+    op = Operator(Grid3D(N, 0.2 * N), torch.float64, 4)
+    op.set_exchange(plan, orb)
+    got = op.energy_terms(None)[3:].cpu()
+    set_plan(plan, 0, 1)
+    ref = op.energy_terms(None)[3:].cpu()
+    assert float(((got - ref) / ref).abs().max()) < 100 * 2.0 ** -53
