@@ -381,8 +381,15 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
   if (Lf > 0) {
     // register-resident two-pass engine: everything but the accumulating z inverse of n fields from
     // f0, in the buffers from field `at` on
-    auto half = [&](ColGeom q, int tile) {   // the N + 1 columns of lone fields, rounded up to whole tiles
-      q.ncols = std::min(M, (N + tile) / tile * tile);
+    // the N + 1 columns of lone fields: an edge tile for the last one where the others fill whole tiles
+    // (scalar passes), else rounded up to whole tiles
+    auto half = [&](ColGeom q, int tile) {
+      if (!packed && N % tile == 0) {
+        q.ncols = N;
+        q.edge = N / tile;
+      } else {
+        q.ncols = std::min(M, (N + tile) / tile * tile);
+      }
       return q;
     };
     auto transform = [&](int f0, int n, int at, bool lone, cudaStream_t st) -> int {
@@ -406,7 +413,9 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
           if (fe) {
             fa.f0 = f0;
             fa.half = lone;
-            return fast::cols_fe<T>(M, P2, gx, M, n, tw2, (const T*)pl.ghat, pl.H, fa, st);
+            ColGeom q = gx;
+            if (lone && N % Lf == 0) q.edge = N / Lf;
+            return fast::cols_fe<T>(M, P2, q, M, n, tw2, (const T*)pl.ghat, pl.H, fa, st);
           }
         }
         GATO_TRY(fast::cols<T>(M, COL_FMI, P2, P2, lone ? half(gx, Lf) : gx, M, n, tw2, (const T*)pl.ghat, pl.H, st));

@@ -67,6 +67,7 @@ struct ColGeom {
   int64_t in_ps, out_ps;   // position strides
   int ncols;               // contiguous columns (lines)
   int nin, nout;           // input positions, output positions kept
+  int edge = 0;            // > 0: tile `edge` holds the one column edge * L, its lines are outer indices
 };
 
 template <typename T>

@@ -35,6 +35,19 @@ struct TwPrefetch {
   }
 };
 
+// The last column of a lone real field's half spectrum (ColGeom::edge): a whole tile for it would do
+// L - 1 columns' work for nothing, and the FP64 passes are bound by just that work (72 columns instead
+// of 65 at N = 64; Hartree solve at 80^3 414 -> 358 us, 96^3 530 -> 497, 128^3 1163 -> 1123). So the lines of tile `edge` are L outer indices of that one
+// column (past the end: the last one again, which stores the same values). True: no such index.
+template <int L>
+__device__ __forceinline__ bool edge_tile(const ColGeom& g, int& outer, int& col, int line) {
+  if (g.edge == 0 || (int)blockIdx.y != g.edge) return false;
+  if (outer * L >= (int)gridDim.x) return true;
+  outer = min(outer * L + line, (int)gridDim.x - 1);
+  col = g.edge * L;
+  return false;
+}
+
 // Strided-line passes (y forward, x forward * kernel * x inverse, y inverse).
 // FULL: every CTA has L real columns (ncols % L == 0), so no per-access guard.
 template <typename T, int R1, int R2, int L, int MODE, bool FULL>
@@ -52,13 +65,14 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   const T2* twi = tws + (Tab::OI - TW0);
   const TwPrefetch<T2, TWN, L * Shape<R1, R2>::RMAX> twp(tw + TW0);
   gdc_wait();
-  const int outer = blockIdx.x, col0 = blockIdx.y * L, f = blockIdx.z;
-  const int t = threadIdx.x;
+  const int f = blockIdx.z, t = threadIdx.x;
   const int line = t % L, q = t / L;   // q: n2 in stages 1/B, k1 in stages 2/A
-  const bool live = FULL || line < g.ncols - col0;
+  int outer = blockIdx.x, col = blockIdx.y * L + line;
+  const bool live = FULL || col < g.ncols;
+  if (FULL && edge_tile<L>(g, outer, col, line)) return;
   // per-thread bases: element (pos, line) of this CTA's tile is base[pos * ps]
-  const T2* src = in + f * g.in_fs + outer * g.in_os + col0 + line;
-  T2* dst = out + f * g.out_fs + outer * g.out_os + col0 + line;
+  const T2* src = in + f * g.in_fs + outer * g.in_os + col;
+  T2* dst = out + f * g.out_fs + outer * g.out_os + col;
   const int64_t ips = g.in_ps, ops = g.out_ps;
   T2 X[R2];
   if (MODE != COL_INV) {
@@ -97,7 +111,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   if (MODE == COL_FMI && q < R1) {
     static_assert(R2 % 2 == 0, "the octant fold below splits k2 at R2 / 2");
     const int ky = outer, kyo = ky <= M - ky ? ky : M - ky;
-    const int kz = col0 + line, kzo = kz <= M - kz ? kz : M - kz;
+    const int kz = col, kzo = kz <= M - kz ? kz : M - kz;
     const int64_t HH = (int64_t)H * H, st = (int64_t)R1 * HH;
     // kx = q + R1 k2 (q < R1): k2 < R2/2 gives kx <= M/2, read at kx; the upper
     // half folds to M - kx = (M - q) - R1 k2.
@@ -178,18 +192,20 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   T2* tws = buf + M * LP;
   const TwPrefetch<T2, TwTab<T2, R1, R2>::NF, L * Shape<R1, R2>::RMAX> twp(tw);
   gdc_wait();
-  const int outer = blockIdx.x, col0 = blockIdx.y * L, f = blockIdx.z;
-  const int t = threadIdx.x;
+  const int f = blockIdx.z, t = threadIdx.x;
   const int line = t % L, q = t / L;
-  if (fa.half && col0 > M / 2) {   // no column of a lone real field's half spectrum
+  int outer = blockIdx.x, col = blockIdx.y * L + line;
+  const bool live = FULL || col < g.ncols;
+  // nothing to do: no column of a lone real field's half spectrum, or no outer index left
+  const bool none = fa.half && (int)blockIdx.y * L > M / 2;
+  if (none || (FULL && edge_tile<L>(g, outer, col, line))) {
     if (t == 0) {
       const int64_t b = ((int64_t)(fa.f0 + f) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
       fa.partials[b] = fa.partials[fa.slot_stride + b] = 0.0;
     }
     return;
   }
-  const bool live = FULL || line < g.ncols - col0;
-  const T2* src = in + f * g.in_fs + outer * g.in_os + col0 + line;
+  const T2* src = in + f * g.in_fs + outer * g.in_os + col;
   const int64_t ips = g.in_ps;
   if (q < R2) {
     const T2* b1 = src + q * ips;
@@ -208,7 +224,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
     fwd_stage2<T2, R1, R2>(buf, LP, line, q, tws, X);
     // kx = q + R1 k2, folded into the kernel-spectrum octant as in the x pass
     const int ky = outer, kyo = ky <= M - ky ? ky : M - ky;
-    const int kz = col0 + line, kzo = kz <= M - kz ? kz : M - kz;
+    const int kz = col, kzo = kz <= M - kz ? kz : M - kz;
     const int64_t HH = (int64_t)H * H, st = (int64_t)R1 * HH;
     const T* glo = ghat + (int64_t)q * HH + (int64_t)kyo * H + kzo;
     const T* ghi = ghat + (int64_t)(M - q) * HH + (int64_t)kyo * H + kzo;
@@ -220,6 +236,8 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
     // a lone real field's columns kz and M - kz carry the same power: 0 < kz < M/2 counts twice
     // (the sum is linear in the weight, so it scales the column's finished sum)
     if (fa.half) acc = scaled(acc, kz == 0 || kz == M / 2 ? 1 : (kz < M / 2 ? 2 : 0));
+    if (FULL && g.edge && (int)blockIdx.y == g.edge && (int)blockIdx.x * L + line >= (int)gridDim.x)
+      acc = scaled(acc, 0);   // a line past the last outer index
   }
   const double s = block_sum0(acc, sh);
   if (t == 0) {
@@ -881,7 +899,7 @@ struct Launch {
   static int cols(int mode, const T2* in, T2* out, const ColGeom& g, int outer, int nf, const T2* tw,
                   const T* ghat, int H, cudaStream_t s) {
     if (FULL && g.ncols % L != 0) return fail(GATO_EUNSUPPORTED, "column pass: whole tiles of %d columns", L);
-    dim3 grid(outer, (g.ncols + L - 1) / L, nf);
+    dim3 grid(outer, (g.ncols + L - 1) / L + (g.edge > 0), nf);
     const size_t sm = sm_cols(mode);
     if (mode == COL_FWD) {
       GATO_TRY(smem_attr(k_cols<T, R1, R2, L, COL_FWD, FULL>, sm));
