@@ -14,8 +14,10 @@
 #include <vector>
 
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "hgh.cuh"
+#include "ptx.cuh"
 
 namespace gato {
 
@@ -413,7 +415,8 @@ __global__ void k_nl_add(T* out, const T* __restrict__ vals, const double* coef,
 // rank order through distributed shared memory (the same sums in every CTA),
 // forms coef[q] = sum_j h_ij ov[block + j] and adds sum_q coef[q] p_q to out
 // over its share of each atom's box, atom by atom with a cluster barrier in
-// between. ov and coef of the vector are also left in global memory.
+// between. ov and coef of the vector are also left in global memory. Behind the stencil that writes
+// out, the overlaps (which read psi alone) run beside it (!wait_psi).
 namespace cg = cooperative_groups;
 constexpr int kNlCluster = 8;          // CTAs per vector (the portable cluster size)
 constexpr int kNlClThreads = 512;
@@ -425,10 +428,9 @@ struct NlAtomRange {
 
 template <typename T>
 __global__ void __cluster_dims__(kNlCluster, 1, 1) __launch_bounds__(kNlClThreads)
-    k_nl_apply_cluster(const T* __restrict__ psi, T* out, const T* __restrict__ vals, const int* q_atom,
-                       const int64_t* q_off, const int* boxes, const int* q_block, const int* q_n,
-                       const int* q_i, const double* q_h, int nq, int K, NlAtomRange ar, int N, double dV,
-                       double* ov_out, double* coef_out) {
+    k_nl_apply_cluster(const T* psi, T* out, const T* __restrict__ vals, const int64_t* q_off, const int* boxes,
+                       const int* q_block, const int* q_n, const int* q_i, const double* q_h, int nq, int K,
+                       NlAtomRange ar, int N, double dV, double* ov_out, double* coef_out, bool wait_psi) {
   cg::cluster_group cl = cg::this_cluster();
   __shared__ double wsum[kNlClMaxQ][kNlClThreads / 32];
   __shared__ double part[kNlClMaxQ];
@@ -439,6 +441,7 @@ __global__ void __cluster_dims__(kNlCluster, 1, 1) __launch_bounds__(kNlClThread
   const int start = rank * blockDim.x + threadIdx.x, stride = kNlCluster * blockDim.x;
   const T* ps = psi + (int64_t)b * N * N * N;
   T* o = out + (int64_t)b * N * N * N;
+  if (wait_psi) gdc_wait();
   // overlaps atom by atom, up to kNlQChunk projectors of one atom per pass over its box: a point's
   // index and psi value serve every projector of the pass (each projector's sum runs over the
   // thread's points in the same order as a pass of its own)
@@ -482,6 +485,7 @@ __global__ void __cluster_dims__(kNlCluster, 1, 1) __launch_bounds__(kNlClThread
     ovs[threadIdx.x] = v * dV;
   }
   cl.sync();   // the remote reads are done (no CTA leaves while another reads it); ovs is complete
+  gdc_wait();  // out holds the stencil's result, ov and coef have been read
   if (threadIdx.x < nq) {
     const int q = threadIdx.x, blk = q_block[q], n = q_n[q], i = q_i[q];
     double c = 0.0;
@@ -613,7 +617,7 @@ int nl_overlaps(Nonlocal& nl, const void* psi, int nb, cudaStream_t s) {
 
 }  // namespace
 
-int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_t s) {
+int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_t s, bool after_stencil) {
   if (nl.nq == 0) return GATO_OK;
   if (nb > Nonlocal::kMaxVec) return fail(GATO_EBADARG, "nonlocal: at most %d vectors", Nonlocal::kMaxVec);
   bool small_boxes = true;
@@ -626,16 +630,13 @@ int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_
       ar.nq[a] = nl.atom_nq[a];
     }
     dim3 g(kNlCluster, nb);
-    if (nl.dtype == GATO_F64)
-      k_nl_apply_cluster<double><<<g, kNlClThreads, 0, s>>>(
-          (const double*)psi, (double*)out, (const double*)nl.vals, nl.d_q_atom, nl.d_q_off, nl.d_box,
-          nl.d_q_block, nl.d_q_n, nl.d_q_i, nl.d_q_h, nl.nq, nl.K, ar, nl.N, nl.dV, nl.ov, nl.coef);
-    else
-      k_nl_apply_cluster<float><<<g, kNlClThreads, 0, s>>>(
-          (const float*)psi, (float*)out, (const float*)nl.vals, nl.d_q_atom, nl.d_q_off, nl.d_box,
-          nl.d_q_block, nl.d_q_n, nl.d_q_i, nl.d_q_h, nl.nq, nl.K, ar, nl.N, nl.dV, nl.ov, nl.coef);
-    GATO_LAUNCH_TRY();
-    return GATO_OK;
+    auto launch = [&](auto kern, auto* p, auto* o) {
+      using T = std::remove_pointer_t<decltype(o)>;
+      return launch_chained(kern, g, kNlClThreads, 0, s, p, o, (const T*)nl.vals, nl.d_q_off, nl.d_box, nl.d_q_block,
+                            nl.d_q_n, nl.d_q_i, nl.d_q_h, nl.nq, nl.K, ar, nl.N, nl.dV, nl.ov, nl.coef, !after_stencil);
+    };
+    if (nl.dtype == GATO_F64) return launch(k_nl_apply_cluster<double>, (const double*)psi, (double*)out);
+    return launch(k_nl_apply_cluster<float>, (const float*)psi, (float*)out);
   }
   GATO_TRY(nl_overlaps(nl, psi, nb, s));
   for (int a = 0; a < nl.K; ++a) {

@@ -54,7 +54,8 @@ struct Nonlocal {
   static constexpr int kChunks = 32;  // partial sums per projector box
 };
 
-int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_t s);
+// after_stencil: the launch ahead in the stream is the stencil that wrote out (kChainOpen).
+int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_t s, bool after_stencil = false);
 int nonlocal_energy(Nonlocal& nl, const void* psi, int nb, double* energy_dev, cudaStream_t s);
 
 }  // namespace gato

@@ -27,6 +27,7 @@
 #include <cuda.h>
 
 #include "op.cuh"
+#include "stencil.cuh"
 #include "ptx.cuh"
 
 namespace gato {
@@ -1902,7 +1903,7 @@ int lanczos_fused(gato_operator& op, const void* psi0, int m, int K, double tol,
     constexpr int gpb = kFzPost2Threads / 32;   // g_i per block
     GATO_TRY(launch_chained(k_fz_post2, (j + 2 + gpb - 1) / gpb, kFzPost2Threads, 0, s, f.partn, f.nbf, dV, f.Cm, m, j,
                             alphas, betas, f.binv, f.c, f.g));
-    if (j + 1 < m) GATO_TRY(op_apply(op, f.wh, f.z, s, true));
+    if (j + 1 < m) GATO_TRY(op_apply(op, f.wh, f.z, s, kChainLate));
   }
   return lz_finish<float>(Vb, n, m, K, tol, alphas, betas, evals, evecs, flag, z, s);
 }

@@ -57,11 +57,11 @@ __global__ void k_sum_scaled(const double* in, int n, double scale, double* out)
 }  // namespace
 
 // out[b] = (-1/2 L + V) psi[b] (+ V_nl psi[b]) for nb fields, on stream ls.
-static int local_part(gato_operator& op, const void* in, void* out, int nb, cudaStream_t ls, bool late = false) {
+static int local_part(gato_operator& op, const void* in, void* out, int nb, cudaStream_t ls, int chain = 0) {
   const double coef = -0.5 / (op.h * op.h);
   GATO_TRY(stencil_apply(op.dtype, in, op.V, out, nb, op.N, op.N, op.N, op_n3(op), coef, op.boundary,
-                         op.order, nullptr, op.dV, ls, ls == op.side.st && ls != nullptr, late));
-  if (op.nl) GATO_TRY(nonlocal_apply(op.nl->n, in, out, nb, ls));
+                         op.order, nullptr, op.dV, ls, ls == op.side.st && ls != nullptr, op.nl ? chain | kChainOpen : chain));
+  if (op.nl) GATO_TRY(nonlocal_apply(op.nl->n, in, out, nb, ls, true));
   return GATO_OK;
 }
 
@@ -80,8 +80,8 @@ static int fork_local(gato_operator& op, const void* in, void* out, int nb, cuda
   return GATO_OK;
 }
 
-int op_apply(gato_operator& op, const void* in, void* out, cudaStream_t s, bool late) {
-  if (op.n_orb <= 0) return local_part(op, in, out, 1, s, late);
+int op_apply(gato_operator& op, const void* in, void* out, cudaStream_t s, int chain) {
+  if (op.n_orb <= 0) return local_part(op, in, out, 1, s, chain);
   cudaEvent_t join = nullptr;
   GATO_TRY(fork_local(op, in, out, 1, s, &join));
   PassArgs a;

@@ -24,7 +24,7 @@ struct gato_operator {
 };
 
 namespace gato {
-int op_apply(gato_operator& op, const void* in, void* out, cudaStream_t s, bool late = false);   // late: see stencil_apply
+int op_apply(gato_operator& op, const void* in, void* out, cudaStream_t s, int chain = 0);   // chain: of stencil_apply
 inline size_t op_esize(const gato_operator& op) { return op.dtype == GATO_F64 ? 8 : 4; }
 inline int64_t op_n3(const gato_operator& op) { return (int64_t)op.N * op.N * op.N; }
 }  // namespace gato

@@ -159,7 +159,7 @@ template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT, bool EDG
 __global__ void __launch_bounds__(kZP*(kBY / YPT))
     k_stencil_tma(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap vmap,
                   T* __restrict__ out, int nx, int ny, int nz, int cx, int tiles_z, int64_t bstride,
-                  T coef, double* dot_part, int late, int* err) {
+                  T coef, double* dot_part, int chain, int* err) {
   using G = TmaGeom<T, R>;
   using P2 = typename Pair<T>::type;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(kZP*(kBY / YPT))
     for (int s = 0; s < kSlots; ++s) mbar_init(&bars[s], 1);
     fence_barrier_init();
   }
-  if (!late) gdc_wait();
+  if (!(chain & kChainLate)) gdc_wait();
+  if (chain & kChainOpen) gdc_launch();
   __syncthreads();
 
   // Only the centre planes R <= q < P - R carry a V tile.
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(kZP*(kBY / YPT))
   };
   for (int qb = 0; qb < P; qb += kSlots)
     if (!run_slots(step, qb, std::make_integer_sequence<int, kSlots>{})) break;
-  if (late) gdc_wait();   // whoever waits for this kernel waits for the one it ran beside
+  if (chain & kChainLate) gdc_wait();   // whoever waits for this kernel waits for the one it ran beside
   if (bad) {
     // drain the copies still in flight (bounded) before the CTA's shared memory goes away
     if (tid == 0)
@@ -339,7 +340,7 @@ int resident_ctas(K kernel, int threads, int smem) {
 template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT, bool EDGE>
 int launch_tma_edge(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int nb, int nx, int ny,
                     int nz, int64_t bstride, double coef, double* dot_part, int* nparts,
-                    cudaStream_t s, bool beside, bool late) {
+                    cudaStream_t s, bool beside, int chain) {
   using G = TmaGeom<T, R>;
   constexpr int kThreads = kZP * (kBY / YPT);
   auto kern = k_stencil_tma<T, R, YPT, HAS_V, STORE, DOT, EDGE>;
@@ -394,34 +395,34 @@ int launch_tma_edge(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int
   dim3 grid(tiles, chunks, nb), block(kZP, kBY / YPT);
   if (nparts) *nparts = tiles * chunks;
   return launch_chained(kern, grid, block, G::SMEM, s, tm, vm, (T*)out, nx, ny, nz, cx, tiles_z, bstride, (T)coef,
-                        dot_part, (int)late, device_error_word());
+                        dot_part, chain, device_error_word());
 }
 
 template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT>
 int launch_tma_rows(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int nb, int nx, int ny,
                     int nz, int64_t bstride, double coef, double* dot_part, int* nparts,
-                    cudaStream_t s, bool beside, bool late) {
+                    cudaStream_t s, bool beside, int chain) {
   if (ny % kBY == 0)
     return launch_tma_edge<T, R, YPT, HAS_V, STORE, DOT, false>(tm, vm, out, nb, nx, ny, nz, bstride, coef, dot_part,
-                                                                nparts, s, beside, late);
+                                                                nparts, s, beside, chain);
   return launch_tma_edge<T, R, YPT, HAS_V, STORE, DOT, true>(tm, vm, out, nb, nx, ny, nz, bstride, coef, dot_part,
-                                                             nparts, s, beside, late);
+                                                             nparts, s, beside, chain);
 }
 
 template <typename T, int R, bool HAS_V, bool STORE, bool DOT>
 int launch_tma_mode(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int nb, int nx, int ny,
                     int nz, int64_t bstride, double coef, double* dot_part, int* nparts,
-                    cudaStream_t s, bool beside, bool late) {
+                    cudaStream_t s, bool beside, int chain) {
   const int rows = g_rows_per_thread.load() ? g_rows_per_thread.load() : kDefaultRows;
   if (rows == 2)
     return launch_tma_rows<T, R, 2, HAS_V, STORE, DOT>(tm, vm, out, nb, nx, ny, nz, bstride, coef,
-                                                       dot_part, nparts, s, beside, late);
+                                                       dot_part, nparts, s, beside, chain);
   return launch_tma_rows<T, R, 4, HAS_V, STORE, DOT>(tm, vm, out, nb, nx, ny, nz, bstride, coef,
-                                                     dot_part, nparts, s, beside, late);
+                                                     dot_part, nparts, s, beside, chain);
 }
 template <typename T, int R>
 int launch_tma(const void* psi, const void* V, void* out, int nb, int nx, int ny, int nz,
-               int64_t bstride, double coef, double* dot_part, int* nparts, cudaStream_t s, bool beside, bool late) {
+               int64_t bstride, double coef, double* dot_part, int* nparts, cudaStream_t s, bool beside, int chain) {
   alignas(64) unsigned char tm[128];
   TmaBox box;
   box.rank = 4;
@@ -459,7 +460,7 @@ int launch_tma(const void* psi, const void* V, void* out, int nb, int nx, int ny
 #define GATO_TMA_MODE(M, HV, ST, DT)                                                          \
   case M:                                                                                    \
     return launch_tma_mode<T, R, HV, ST, DT>(T4, V3, out, nb, nx, ny, nz, bstride, coef,     \
-                                             dot_part, nparts, s, beside, late);
+                                             dot_part, nparts, s, beside, chain);
   switch (mode) {
     GATO_TMA_MODE(1, false, false, true)
     GATO_TMA_MODE(2, false, true, false)
@@ -476,7 +477,7 @@ int launch_tma(const void* psi, const void* V, void* out, int nb, int nx, int ny
 template <typename T>
 int stencil_typed(const void* psi, const void* V, void* out, int nb, int nx, int ny, int nz,
                   int64_t bstride, double coef, int boundary, int order, double* dot_dev,
-                  double dv, cudaStream_t s, bool beside, bool late) {
+                  double dv, cudaStream_t s, bool beside, int chain) {
   const bool tma_ok = boundary == GATO_DIRICHLET && ((uint64_t)nz * sizeof(T)) % 16 == 0 &&
                       ((uint64_t)bstride * sizeof(T)) % 16 == 0 &&
                       ((uintptr_t)psi % 16) == 0 && ((uintptr_t)V % 16) == 0 &&
@@ -490,9 +491,9 @@ int stencil_typed(const void* psi, const void* V, void* out, int nb, int nx, int
   if (tma_ok) {
     int nparts = 0;
     if (order == 2)
-      GATO_TRY(launch_tma<T, 1>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s, beside, late));
+      GATO_TRY(launch_tma<T, 1>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s, beside, chain));
     else
-      GATO_TRY(launch_tma<T, 2>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s, beside, late));
+      GATO_TRY(launch_tma<T, 2>(psi, V, out, nb, nx, ny, nz, bstride, coef, part, &nparts, s, beside, chain));
     if (dot_dev) {
       if (nparts > 4096) return fail(GATO_EUNSUPPORTED, "stencil: too many tiles for dot");
       GATO_TRY(finalize_sums(part, nb, nparts, dv, dot_dev, s));
@@ -523,7 +524,7 @@ int stencil_typed(const void* psi, const void* V, void* out, int nb, int nx, int
 
 int stencil_apply(int dtype, const void* psi, const void* V, void* out, int nb, int nx, int ny,
                   int nz, int64_t bstride, double coef, int boundary, int order, double* dot_dev,
-                  double dv, cudaStream_t s, bool beside, bool late) {
+                  double dv, cudaStream_t s, bool beside, int chain) {
   if (order != 2 && order != 4)
     return fail(GATO_EBADARG, "Unknown order %d; expected 2 or 4.", order);
   if (boundary != GATO_DIRICHLET && boundary != GATO_PERIODIC)
@@ -532,10 +533,10 @@ int stencil_apply(int dtype, const void* psi, const void* V, void* out, int nb, 
     return fail(GATO_EBADARG, "stencil: bad arguments");
   if (dtype == GATO_F64)
     return stencil_typed<double>(psi, V, out, nb, nx, ny, nz, bstride, coef, boundary, order,
-                                 dot_dev, dv, s, beside, late);
+                                 dot_dev, dv, s, beside, chain);
   if (dtype == GATO_F32)
     return stencil_typed<float>(psi, V, out, nb, nx, ny, nz, bstride, coef, boundary, order,
-                                dot_dev, dv, s, beside, late);
+                                dot_dev, dv, s, beside, chain);
   return fail(GATO_EBADARG, "bad dtype %d", dtype);
 }
 

@@ -61,3 +61,39 @@ def test_energies_of_many_partials(N, n):
     set_plan(plan, 0, 1)
     ref = op.energy_terms(None)[3:].cpu()
     assert float(((got - ref) / ref).abs().max()) < 100 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("N", [18, 40, 64])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+def test_projectors_beside_the_stencil(N, dtype):
+    """A chain of applies, each on the result of the one before, against the same applies one at a time, exactly;
+    and one apply against its two parts by themselves, which add the stencil's value and two atoms' projectors in
+    another order: at most four roundings of either part's size."""
+    from gato_gb300.grid import Grid3D
+    from gato_gb300.geometry import Nuclei
+    from gato_gb300.pseudopotentials import HGH_TABLE, HGHNonlocal
+    from gato_gb300.scf import Operator
+    g = torch.Generator().manual_seed(N)
+    grid = Grid3D(N, 9.0)
+    nl = HGHNonlocal(Nuclei(torch.tensor([[0.1, -0.2, 0.3], [0.5, 0.4, -0.6]], dtype=torch.float64),
+                            torch.tensor([6.0, 6.0], dtype=torch.float64)), [HGH_TABLE["O"]] * 2, grid, dtype)
+    psi = torch.rand(N, N, N, generator=g, dtype=torch.float64).to(dtype).cuda()
+    op, bare = Operator(grid, dtype, 4), Operator(grid, dtype, 4)
+    for o in (op, bare):
+        o.set_potential(-psi)
+    op.set_nonlocal(nl)
+    eps = 2.0 ** -53 if dtype == torch.float64 else 2.0 ** -24
+    both, local, far = op.apply(psi).double(), bare.apply(psi).double(), nl(psi).double()
+    assert float((both - local - far).norm()) < 4 * eps * float(local.norm() + far.norm())
+    bufs = [psi.clone(), torch.empty_like(psi)]
+    want = []
+    for k in range(6):
+        op.apply(bufs[k % 2], bufs[1 - k % 2])
+        torch.cuda.synchronize()
+        want.append(bufs[1 - k % 2].clone())
+        torch.cuda.synchronize()
+    for _ in range(3):
+        bufs = [psi.clone(), torch.empty_like(psi)]
+        for k in range(6):
+            op.apply(bufs[k % 2], bufs[1 - k % 2])
+        assert torch.equal(bufs[1], want[4]) and torch.equal(bufs[0], want[5])
