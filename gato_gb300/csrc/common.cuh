@@ -90,21 +90,28 @@ void ws_put(WsBuf& b);                                // gives b back
 // 1431 / 3656 against 1426 / 3655 at 96. No FFT kernel lets its successor begin earlier still (gdc_launch
 // at its start): the successor's waiting blocks take the places of a second strand's and land unevenly on
 // the SMs (FP32 block at 128^3 453 -> 488, FP64 exchange of 2 orbitals at 40^3 103 -> 188).
+// launch_cluster: the same with clusters of `cluster` blocks along x.
 template <typename... P, typename... A>
-int launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... a) {
+int launch_cluster(int cluster, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... a) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim = {(unsigned)cluster, 1, 1};
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   GATO_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, P(a)...));
   count_launch();
   return GATO_OK;
+}
+template <typename... P, typename... A>
+int launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... a) {
+  return launch_cluster(1, k, grid, block, smem, s, static_cast<A&&>(a)...);
 }
 
 // A side stream with the events that fork work onto it and join it back. Kept like workspace (at most

@@ -408,17 +408,17 @@ __global__ void k_nl_add(T* out, const T* __restrict__ vals, const double* coef,
   }
 }
 
-// The whole apply for one vector b in one cluster of kNlCluster CTAs (grid
-// (kNlCluster, nb)): each CTA takes every kNlCluster-th stretch of every box,
-// reduces its partial overlaps per projector in shared memory, and after a
-// cluster barrier every CTA sums the kNlCluster partials of each projector in
-// rank order through distributed shared memory (the same sums in every CTA),
+// The whole apply for one vector b in one cluster of C CTAs (grid (C, nb)):
+// each CTA takes every C-th stretch of every box, reduces its partial overlaps
+// per projector in shared memory, and after a cluster barrier every CTA sums
+// the C partials of each projector in rank order through distributed shared memory (the same sums in every CTA),
 // forms coef[q] = sum_j h_ij ov[block + j] and adds sum_q coef[q] p_q to out
 // over its share of each atom's box, atom by atom with a cluster barrier in
 // between. ov and coef of the vector are also left in global memory. Behind the stencil that writes
 // out, the overlaps (which read psi alone) run beside it (!wait_psi).
 namespace cg = cooperative_groups;
 constexpr int kNlCluster = 8;          // CTAs per vector (the portable cluster size)
+constexpr int kNlClusterBig = 16;      // large boxes (big_boxes)
 constexpr int kNlClThreads = 512;
 constexpr int kNlClMaxQ = 64;          // projectors of all atoms
 constexpr int kNlQChunk = 8;           // projectors of one atom accumulated per pass over its box
@@ -427,7 +427,7 @@ struct NlAtomRange {
 };
 
 template <typename T>
-__global__ void __cluster_dims__(kNlCluster, 1, 1) __launch_bounds__(kNlClThreads)
+__global__ void __launch_bounds__(kNlClThreads)
     k_nl_apply_cluster(const T* psi, T* out, const T* __restrict__ vals, const int64_t* q_off, const int* boxes,
                        const int* q_block, const int* q_n, const int* q_i, const double* q_h, int nq, int K,
                        NlAtomRange ar, int N, double dV, double* ov_out, double* coef_out, bool wait_psi) {
@@ -438,7 +438,8 @@ __global__ void __cluster_dims__(kNlCluster, 1, 1) __launch_bounds__(kNlClThread
   __shared__ T cf[kNlClMaxQ];
   const int rank = (int)cl.block_rank(), b = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int start = rank * blockDim.x + threadIdx.x, stride = kNlCluster * blockDim.x;
+  const int ncl = (int)cl.num_blocks();
+  const int start = rank * blockDim.x + threadIdx.x, stride = ncl * blockDim.x;
   const T* ps = psi + (int64_t)b * N * N * N;
   T* o = out + (int64_t)b * N * N * N;
   if (wait_psi) gdc_wait();
@@ -481,7 +482,7 @@ __global__ void __cluster_dims__(kNlCluster, 1, 1) __launch_bounds__(kNlClThread
   cl.sync();   // every CTA's partial overlaps are in its shared memory
   if (threadIdx.x < nq) {
     double v = 0.0;
-    for (int r = 0; r < kNlCluster; ++r) v += cl.map_shared_rank(part, r)[threadIdx.x];
+    for (int r = 0; r < ncl; ++r) v += cl.map_shared_rank(part, r)[threadIdx.x];
     ovs[threadIdx.x] = v * dV;
   }
   cl.sync();   // the remote reads are done (no CTA leaves while another reads it); ovs is complete
@@ -617,6 +618,38 @@ int nl_overlaps(Nonlocal& nl, const void* psi, int nb, cudaStream_t s) {
 
 }  // namespace
 
+// Boxes whose walk is worth twice the SMs: the apply takes the time of one CTA's share of the projector values.
+// On a cluster of 8 / 16 CTAs, us, apply alone and FP32 matvec: LiH (boxes up to the whole grid) 22 / 16 and
+// 32.0 / 27.7 at 32^3, 102 / 54 and 119 / 72 at 64^3, 242 / 125 and 267 / 150 at 96^3; HCl 24 / 19 and 44.0 / 39.9
+// at 64^3. Where the boxes are a small part of the grid the exchange transforms hide the apply and the wider
+// cluster only takes their SMs: HCl matvec 94.7 / 95.9 at 96^3, 193 / 195 at 128^3. FP64 transforms mind more
+// (LiH matvec at 32^3 45 / 52, 48^3 106 / 108, 64^3 187 / 168).
+static bool big_boxes(const Nonlocal& nl) {
+  return nl.nvals >= (nl.dtype == GATO_F64 ? 1 << 19 : 1 << 17) && 4 * nl.nvals >= (int64_t)nl.N * nl.N * nl.N;
+}
+
+// Whether the GPU takes clusters of kNlClusterBig CTAs of this kernel (more than the portable size).
+template <typename K>
+static bool big_clusters(K kern) {
+  static const bool ok = [kern] {   // one kernel per instantiation of K's type
+    const void* f = reinterpret_cast<const void*>(kern);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kNlClusterBig);
+    cfg.blockDim = dim3(kNlClThreads);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {kNlClusterBig, 1, 1};
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool fits = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                      cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    return fits;
+  }();
+  return ok;
+}
+
 int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_t s, bool after_stencil) {
   if (nl.nq == 0) return GATO_OK;
   if (nb > Nonlocal::kMaxVec) return fail(GATO_EBADARG, "nonlocal: at most %d vectors", Nonlocal::kMaxVec);
@@ -629,10 +662,10 @@ int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_
       ar.q0[a] = nl.atom_q0[a];
       ar.nq[a] = nl.atom_nq[a];
     }
-    dim3 g(kNlCluster, nb);
     auto launch = [&](auto kern, auto* p, auto* o) {
       using T = std::remove_pointer_t<decltype(o)>;
-      return launch_chained(kern, g, kNlClThreads, 0, s, p, o, (const T*)nl.vals, nl.d_q_off, nl.d_box, nl.d_q_block,
+      const int C = big_boxes(nl) && big_clusters(kern) ? kNlClusterBig : kNlCluster;
+      return launch_cluster(C, kern, dim3(C, nb), kNlClThreads, 0, s, p, o, (const T*)nl.vals, nl.d_q_off, nl.d_box, nl.d_q_block,
                             nl.d_q_n, nl.d_q_i, nl.d_q_h, nl.nq, nl.K, ar, nl.N, nl.dV, nl.ov, nl.coef, !after_stencil);
     };
     if (nl.dtype == GATO_F64) return launch(k_nl_apply_cluster<double>, (const double*)psi, (double*)out);

@@ -64,11 +64,13 @@ def test_energies_of_many_partials(N, n):
 
 
 @pytest.mark.parametrize("N", [18, 40, 64])
+@pytest.mark.parametrize("element", ["O", "Cl", "Li"])   # small boxes, middle ones, boxes as large as the grid
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
-def test_projectors_beside_the_stencil(N, dtype):
+def test_projectors_beside_the_stencil(N, element, dtype):
     """A chain of applies, each on the result of the one before, against the same applies one at a time, exactly;
     and one apply against its two parts by themselves, which add the stencil's value and two atoms' projectors in
-    another order: at most four roundings of either part's size."""
+    another order, at most four roundings of either part's size (a point's sum has ten projectors' terms at most,
+    formed alike on both sides)."""
     from gato_gb300.grid import Grid3D
     from gato_gb300.geometry import Nuclei
     from gato_gb300.pseudopotentials import HGH_TABLE, HGHNonlocal
@@ -76,7 +78,7 @@ def test_projectors_beside_the_stencil(N, dtype):
     g = torch.Generator().manual_seed(N)
     grid = Grid3D(N, 9.0)
     nl = HGHNonlocal(Nuclei(torch.tensor([[0.1, -0.2, 0.3], [0.5, 0.4, -0.6]], dtype=torch.float64),
-                            torch.tensor([6.0, 6.0], dtype=torch.float64)), [HGH_TABLE["O"]] * 2, grid, dtype)
+                            torch.tensor([6.0, 6.0], dtype=torch.float64)), [HGH_TABLE[element]] * 2, grid, dtype)
     psi = torch.rand(N, N, N, generator=g, dtype=torch.float64).to(dtype).cuda()
     op, bare = Operator(grid, dtype, 4), Operator(grid, dtype, 4)
     for o in (op, bare):
