@@ -86,7 +86,7 @@ int op_apply(gato_operator& op, const void* in, void* out, cudaStream_t s, int c
   GATO_TRY(fork_local(op, in, out, 1, s, &join));
   PassArgs a;
   GATO_TRY(exchange_args(a, in, op.orbitals, op.n_orb, op_esize(op), op_n3(op), out, -1.0));
-  return poisson_run(op.pp->p, a, EPI_ACC, true, nullptr, s, join);
+  return poisson_run(op.pp->p, a, EPI_ACC, true, nullptr, s, join, op.overlap);
 }
 
 static void block_pairs(PassArgs& a, const gato_operator& op, void* out, bool energy) {
@@ -237,12 +237,12 @@ extern "C" int gato_op_apply_block(gato_op_t op, void* out, void* stream) {
     GATO_TRY(ws_get(op->jbuf, need, s));
     a.jbase = op->jbuf.p;
     a.jstride = op_n3(*op);
-    GATO_TRY(poisson_run(op->pp->p, a, EPI_J, false, nullptr, s));
+    GATO_TRY(poisson_run(op->pp->p, a, EPI_J, false, nullptr, s, nullptr, op->overlap));
     if (join) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
     GATO_TRY(pair_exchange(op->dtype, op->orbitals, op->n_orb, op->jbuf.p, out, op_n3(*op), s));
     return ws_used(op->jbuf, s);
   }
-  return poisson_run(op->pp->p, a, EPI_ACC, true, nullptr, s, join);
+  return poisson_run(op->pp->p, a, EPI_ACC, true, nullptr, s, join, op->overlap);
 }
 
 extern "C" int gato_op_overlap(gato_op_t op, int on) {

@@ -309,7 +309,7 @@ bool two_strands(size_t ts, int N) { return ts == 8 || N >= 64; }
 
 template <typename T>
 int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, double* energy_dev,
-              cudaStream_t s, cudaEvent_t join) {
+              cudaStream_t s, cudaEvent_t join, bool strands) {
   using T2 = typename Cplx<T>::type;
   const int N = pl.N, M = pl.M;
   const int64_t nrows = (int64_t)N * N;
@@ -430,7 +430,7 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
       const int nl = lf0 >= nfull ? std::min(group - nf, args.nf - lf0) : 0;
       // two strands of about equal work, the second on the plan's own stream
       int na = nf, la = nl;
-      if (two_strands(sizeof(T), N)) {
+      if (strands && two_strands(sizeof(T), N)) {
         const int share = (2 * nf + nl + 1) / 2;
         na = std::min(nf, (share + 1) / 2);
         la = na == nf ? std::min(nl, std::max(share - 2 * nf, 0)) : 0;
@@ -500,14 +500,14 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
 }  // namespace
 
 int poisson_run(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate,
-                double* energy_dev, cudaStream_t s, cudaEvent_t join) {
+                double* energy_dev, cudaStream_t s, cudaEvent_t join, bool strands) {
   if (args.nf <= 0) {
     if (join) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
     return GATO_OK;
   }
   if (args.nf > kMaxFields) return fail(GATO_EBADARG, "poisson: too many fields (%d)", args.nf);
-  if (pl.dtype == GATO_F64) return run_typed<double>(pl, args, epi, accumulate, energy_dev, s, join);
-  return run_typed<float>(pl, args, epi, accumulate, energy_dev, s, join);
+  if (pl.dtype == GATO_F64) return run_typed<double>(pl, args, epi, accumulate, energy_dev, s, join, strands);
+  return run_typed<float>(pl, args, epi, accumulate, energy_dev, s, join, strands);
 }
 
 // Appends the FP64 stage-twiddle rows of an R-point second stage (see fft2.cuh), rows r < nrows:

@@ -195,9 +195,10 @@ bool poisson_fe_supported(const PoissonPlan& pl);
 // (two slots).
 // join (EPI_ACC only, may be null): the stream waits on it before the first z-inverse epilogue,
 // the first kernel that reads or writes the outputs (work on another stream that also writes them,
-// ordered before the accumulation without holding up the transforms).
+// ordered before the accumulation without holding up the transforms). strands: the transforms may run as
+// two strands, one on the plan's stream; else all stays in order on s.
 int poisson_run(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate,
-                double* energy_dev, cudaStream_t s, cudaEvent_t join = nullptr);
+                double* energy_dev, cudaStream_t s, cudaEvent_t join = nullptr, bool strands = true);
 
 }  // namespace gato
 
