@@ -135,32 +135,39 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
   }
 }
 
-// Block sum of a per-thread accumulator, valid in thread 0 only: float-float
-// through the shuffles for FP32 (the FP64 pipe is used once per CTA), double
-// for FP64. `sh` holds 32 doubles.
-__device__ __forceinline__ double block_sum0(const Acc<float>& a, double* sh) {
-  FF s = a.s;
+// Block sums, valid in thread 0 only, of a block of NT threads: some shapes' blocks (L * RMAX threads) are
+// not whole warps, and a shuffle may name only lanes that exist. A short last warp exchanges among its
+// own lanes, a lane without a partner adds nothing. `sh` holds 32 doubles; NT <= 1024.
+template <int NT>
+__device__ __forceinline__ double block_total(double v, double* sh) {
+  constexpr int TAIL = NT % 32, NW = (NT + 31) / 32;
+  if constexpr (TAIL == 0) {
+    return block_sum(v, sh);
+  } else {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < NW - 1) {
+      v = warp_sum(v);
+    } else {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float hi = __shfl_xor_sync(0xffffffffu, s.hi, o);
-    const float lo = __shfl_xor_sync(0xffffffffu, s.lo, o);
-    ff_add(s, hi);
-    s.lo += lo;
+      for (int o = 16; o > 0; o >>= 1) {
+        const bool has = lane + o < TAIL;
+        const double x = __shfl_sync((1u << TAIL) - 1, v, has ? lane + o : lane);
+        if (has) v += x;
+      }
+    }
+    __syncthreads();   // sh may still be read from a sum before
+    if (lane == 0) sh[warp] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+      for (int w = 0; w < NW; ++w) t += sh[w];
+    return t;
   }
-  float2* shf = reinterpret_cast<float2*>(sh);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  if (lane == 0) shf[warp] = make_float2(s.hi, s.lo);
-  __syncthreads();
-  if (threadIdx.x != 0) return 0.0;
-  FF t{0.f, 0.f};
-  for (int w = 0; w < nw; ++w) {
-    ff_add(t, shf[w].x);
-    t.lo += shf[w].y;
-  }
-  return ff_value(t);
 }
+// Of a per-thread accumulator.
+template <int NT>
 __device__ __forceinline__ double block_sum0(const Acc<double>& a, double* sh) {
-  return block_sum(a.value(), sh);
+  return block_total<NT>(a.value(), sh);
 }
 
 // acc times a small whole number w (exact for 0, 1 and 2).
@@ -239,7 +246,7 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX)
     if (FULL && g.edge && (int)blockIdx.y == g.edge && (int)blockIdx.x * L + line >= (int)gridDim.x)
       acc = scaled(acc, 0);   // a line past the last outer index
   }
-  const double s = block_sum0(acc, sh);
+  const double s = block_sum0<L * Shape<R1, R2>::RMAX>(acc, sh);
   if (t == 0) {
     const int fg = fa.f0 + f;
     const int64_t b = ((int64_t)fg * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
@@ -675,8 +682,8 @@ __global__ void __launch_bounds__(L * Shape<R1, R2>::RMAX, (rows_inv_min_ctas<T,
     }
   }
   if constexpr (ENERGY) {
-    const double s0 = block_sum(e0.value(), sh);
-    const double s1 = block_sum(e1.value(), sh);
+    const double s0 = block_total<NT>(e0.value(), sh);
+    const double s1 = block_total<NT>(e1.value(), sh);
     if (threadIdx.x == 0) {
       partials[blockIdx.x] = s0;
       partials[slot_stride + blockIdx.x] = s1;
