@@ -580,10 +580,11 @@ int make_atoms(AtomTable& at, int K, const double* pos, const double* Z, const d
   return GATO_OK;
 }
 
-// Shared memory for the coordinate tables of a potential or force kernel (a few KB; large grids opt in).
+// Shared memory for the coordinate tables of a potential or force kernel (a few KB; large grids opt in:
+// the tables and the kernels' own arrays share the 48 KB that a launch gets without).
 int table_limit(const void* fn, size_t bytes) {
   if (bytes > 200 * 1024) return fail(GATO_EUNSUPPORTED, "potential: grid too large for the coordinate table");
-  return bytes > 48 * 1024 ? raise_smem_limit(fn, bytes) : GATO_OK;
+  return bytes > 47 * 1024 ? raise_smem_limit(fn, bytes) : GATO_OK;
 }
 
 ProjParams proj_params(const Nonlocal& nl, const NlProj& p) {
