@@ -29,6 +29,7 @@ struct AtomTable {
   int K;
   double x[kMaxAtoms], y[kMaxAtoms], z[kMaxAtoms];
   double Z[kMaxAtoms], rloc[kMaxAtoms], c[kMaxAtoms][4];
+  double far[kMaxAtoms];   // radius of far_radius
 };
 
 __device__ __forceinline__ double axis_coord(int i, double L, double h) {
@@ -100,8 +101,9 @@ __global__ void k_softened(T* V, int N, double L, double h, AtomTable at, double
 // From 8 sqrt(2) r_loc outwards erf(r / (sqrt(2) r_loc)) is 1 in FP64 and exp(-r^2 / (2 r_loc^2)) < 2e-28
 // is far below the last bit of anything it is added to: only the Coulomb tail is left there. That is
 // all but a sphere of 2 to 9 bohr around each centre, and the erf, the exp and the divisions are most
-// of the FP64 work (64^3 water, V_loc: 180 -> 50 us; its force integral 304 -> 73).
-constexpr double kFar = 8.0 * 1.4142135623730951;
+// of the FP64 work (64^3 water, V_loc: 180 -> 50 us; its force integral 304 -> 73). The FP32 force takes
+// 6 sqrt(2) r_loc (erf is 1, the exponentials below 2^-30 of the rest). far_radius says where it holds.
+constexpr double kFar = 8.0 * 1.4142135623730951, kFarF32 = 0.75 * kFar;
 
 // V_loc of one centre at distance r (pseudopotentials.py:214-227).
 __device__ __forceinline__ double hgh_vloc(double r, double Z, double rloc, const double* c) {
@@ -122,7 +124,7 @@ __global__ void k_hgh_local(T* V, int N, double L, double h, AtomTable at) {
     double v = 0.0;
     for (int k = 0; k < at.K; ++k) {
       const double dx = ctab[w.x] - at.x[k], dy = ctab[w.y] - at.y[k], dz = ctab[w.z] - at.z[k];
-      const double r2 = dx * dx + dy * dy + dz * dz + 1e-30, rf = kFar * at.rloc[k];
+      const double r2 = dx * dx + dy * dy + dz * dz + 1e-30, rf = at.far[k];
       if (r2 > rf * rf) v -= at.Z[k] * rsqrt(r2);
       else v += hgh_vloc(sqrt(r2), at.Z[k], at.rloc[k], at.c[k]);
     }
@@ -157,8 +159,7 @@ __device__ __forceinline__ T norm2(T dx, T dy, T dz, T e) {
   return fma(dz, dz, fma(dy, dy, dx * dx)) + e;
 }
 
-// rho dV_k/dR is w d with w = -rho (dV/dr) / r; in the far region (kFar; FP32: 6 sqrt(2) r_loc, where
-// erf is 1 and the exponentials are below 2^-30 of the rest) dV/dr = Z / r^2.
+// rho dV_k/dR is w d with w = -rho (dV/dr) / r; in the far region (far_radius) dV/dr = Z / r^2.
 template <typename T>
 __device__ __forceinline__ T local_grad_weight(T rho, T r2, T far2, T Z, T rloc, const double* c) {
   if (r2 > far2) {
@@ -188,7 +189,7 @@ __global__ void k_local_grad(const T* __restrict__ rho, int N, double L, double 
     const int k = blockIdx.y;
     axis_table(d, N, L, h, at.x[k], at.y[k], at.z[k]);
     __syncthreads();
-    const T rf = (T)((sizeof(T) == 8 ? kFar : 0.75 * kFar) * at.rloc[k]), far2 = rf * rf;
+    const T rf = (T)at.far[k], far2 = rf * rf;
     Acc<T> g[3];
     for (PointWalk w(N); w.i < n3; w.next(N)) {
       const T dx = d[w.x], dy = d[N + w.y], dz = d[2 * N + w.z];
@@ -565,8 +566,26 @@ __global__ void k_nl_grad_combine(const double* coef, const double* dov, const i
         grad[3 * q_atom[q] + c] += 4.0 * coef[b * nq + q] * dov[((int64_t)b * nq + q) * 3 + c];
 }
 
+// The radius from which a centre's potential, or its force, is the Coulomb tail alone. The parameters are the
+// caller's: where the Gaussian terms at kFar r_loc are not below half an ulp of the tail (those of the
+// table's elements are, 2^-13 times and less) it is the radius at which their exponential underflows to zero, and with
+// parameters that the tail's formula does not cover (not finite, r_loc <= 0) there is none.
+enum LocalPart { kNoLocal, kPotential, kForceF64, kForceF32 };
+double far_radius(LocalPart part, double Z, double rloc, const double* c) {
+  const bool force = part != kPotential;
+  bool plain = rloc > 0 && std::isfinite(rloc) && std::isfinite(Z);
+  for (int i = 0; i < 4; ++i) plain = plain && std::isfinite(c[i]);
+  if (!plain) return INFINITY;
+  const double rho = part == kForceF32 ? kFarF32 : kFar, q = rho * rho, half_ulp = part == kForceF32 ? 0x1p-25 : 0x1p-54;
+  const double poly = fabs(c[0]) + q * (fabs(c[1]) + q * (fabs(c[2]) + q * fabs(c[3])));
+  const double dpoly = fabs(c[1]) + q * (2 * fabs(c[2]) + q * 3 * fabs(c[3]));
+  const double gauss = exp(-0.5 * q) * (force ? (0.5 * poly + dpoly) * 2 * rho / rloc : poly);
+  const double tail = fabs(Z) / (force ? q * rloc * rloc : rho * rloc);
+  return (gauss <= half_ulp * tail ? rho : 40.0) * rloc;
+}
+
 int make_atoms(AtomTable& at, int K, const double* pos, const double* Z, const double* rloc,
-               const double* c) {
+               const double* c, LocalPart part = kNoLocal) {
   if (K < 0 || K > kMaxAtoms) return fail(GATO_EBADARG, "at most %d atoms (got %d)", kMaxAtoms, K);
   at.K = K;
   for (int k = 0; k < K; ++k) {
@@ -576,6 +595,7 @@ int make_atoms(AtomTable& at, int K, const double* pos, const double* Z, const d
     at.Z[k] = Z ? Z[k] : 0.0;
     at.rloc[k] = rloc ? rloc[k] : 1.0;
     for (int i = 0; i < 4; ++i) at.c[k][i] = c ? c[4 * k + i] : 0.0;
+    at.far[k] = part == kNoLocal ? INFINITY : far_radius(part, at.Z[k], at.rloc[k], at.c[k]);
   }
   return GATO_OK;
 }
@@ -729,7 +749,7 @@ extern "C" int gato_hgh_local(int dtype, void* V, int N, double L, int K, const 
   if (!V || N < 1 || L <= 0 || (K > 0 && (!pos_host || !Zion_host || !rloc_host || !c_host)))
     return fail(GATO_EBADARG, "gato_hgh_local: bad arguments");
   AtomTable at;
-  GATO_TRY(make_atoms(at, K, pos_host, Zion_host, rloc_host, c_host));
+  GATO_TRY(make_atoms(at, K, pos_host, Zion_host, rloc_host, c_host, kPotential));
   cudaStream_t s = as_stream(stream);
   const double h = L / N;
   const int64_t n3 = (int64_t)N * N * N;
@@ -749,7 +769,7 @@ extern "C" int gato_hgh_local_grad(int dtype, const void* rho, int N, double L, 
       !grad_host)
     return fail(GATO_EBADARG, "gato_hgh_local_grad: bad arguments");
   AtomTable at;
-  GATO_TRY(make_atoms(at, K, pos_host, Zion_host, rloc_host, c_host));
+  GATO_TRY(make_atoms(at, K, pos_host, Zion_host, rloc_host, c_host, dtype == GATO_F64 ? kForceF64 : kForceF32));
   cudaStream_t s = as_stream(stream);
   const double h = L / N;
   const int nblk = kRedBlocks;
