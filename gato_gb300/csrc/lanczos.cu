@@ -895,8 +895,10 @@ __global__ void k_scale_copy(const T* __restrict__ src, T* dst, int64_t n, const
 // form's q_i = 0 -> -pivmin convention), and the pair (p_i, p_{i-1}) is
 // rescaled by an exact power of two whenever p_i's exponent leaves [-480, 480].
 // The zero and exponent tests read the words of p (a compare would take the FP64 pipe). The exponent is
-// looked at every fourth step: four steps grow |p| by at most (2 nm)^4, so up to nm = 2^100 nothing
-// leaves the range in between; `wide` (nm beyond that) looks at every step.
+// looked at every fourth step: four steps grow |p| by at most (2 nm)^4, and with |x| >= 2^-60 a row's a_i - x
+// is 0 or at least 2^-54 |x|, so four shrink it by at most 2^-456: between two looks nothing leaves the range
+// for nm up to 2^100. `wide` (larger norms, smaller x: small norms, or a bracket that closes in on an
+// eigenvalue 0 such as the zero rows after a breakdown have) looks at every step.
 __device__ __forceinline__ int sturm_count(const double* a, const double* e2, int m, double x, bool wide) {
   auto zero = [](double v) { return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0; };
   auto neg = [&](double v, bool prev_neg) { return zero(v) ? !prev_neg : __double2hiint(v) < 0; };
@@ -980,13 +982,14 @@ __global__ void __launch_bounds__(kTriThreads) k_tridiag_eig(const double* alpha
   ghi += pad;
   const double tnorm = nm > 0 ? nm : 1.0;
   const double pivmin = 1e-290 > 2.2e-16 * 2.2e-16 * tnorm ? 1e-290 : 1e-300;
-  const bool wide = !(nm < 0x1p100);
-  double lo = glo, hi = ghi;
+    double lo = glo, hi = ghi;
   constexpr double kSec = kTriThreads + 1;
+  const double least = fmax(pivmin, 0x1p-200 * tnorm);   // a bracket around 0: 1 / shift, squared, is finite
   for (int it = 0; it < 80; ++it) {
     const double width = hi - lo;
-    if (width <= 2.2e-16 * 2 * fmax(fabs(lo), fabs(hi)) + pivmin) break;   // the same in every thread
+    if (width <= 2.2e-16 * 2 * fmax(fabs(lo), fabs(hi)) + least) break;   // the same in every thread
     const double x = lo + width * (double)(t + 1) / kSec;
+    const bool wide = !(nm < 0x1p100) || !(fabs(x) >= 0x1p-60);
     // bracket: eigenvalue k lies in [x_i, x_{i+1}) where count(x_i) <= k < count(x_{i+1}); the counts
     // are monotone, so threads 0..nb-1 have count <= k
     const int nb = __syncthreads_count(sturm_count(a, e2, m, x, wide) <= k);
