@@ -295,6 +295,6 @@ extern "C" int gato_op_energy_terms(gato_op_t op, const void* V_ext, double* ter
   GATO_TRY(gato_density(op->dtype, op->orbitals, n, n3, op->rho.p, s));
   PassArgs a;
   block_pairs(a, *op, nullptr, true);
-  GATO_TRY(poisson_run(op->pp->p, a, EPI_ENERGY, false, terms + 3, s));
+  GATO_TRY(poisson_run(op->pp->p, a, EPI_ENERGY, false, terms + 3, s, nullptr, op->overlap));
   return ws_used(op->rho, s);
 }

@@ -78,8 +78,8 @@ class Operator:
         self.block_epilogue = int(block_epilogue)
 
     def overlap(self, on: bool):
-        """Run the stencil and non-local part beside the exchange transforms (True, the default) or
-        in order on the caller's stream (False); results are the same either way."""
+        """Run the stencil and non-local part beside the exchange transforms, and those as two strands (True,
+        the default), or everything in order on the caller's stream (False); the same results either way."""
         _lib.call("gato_op_overlap", self.handle, int(bool(on)))
 
     def set_potential(self, V: torch.Tensor | None):
