@@ -740,16 +740,20 @@ __global__ void __launch_bounds__(32 * kWsMaxWarps, 1)
 }
 
 // (float)v by integer arithmetic, round to nearest even: a conversion is an instruction of the FP64 pipe
-// (64 cycles a warp on GB300), this is nine of the integer units and no branch. Magnitudes below 2^-126
-// give 0; from 2^127 up (infinities and NaN among them) `big` is set and the value is not meaningful.
-__device__ __forceinline__ float to_float(double v, unsigned& big) {
+// (64 cycles a warp on GB300), this is ten of the integer units and no branch. From 2^127 up (infinities
+// and NaN among them) `big` is set and the value is not meaningful. Magnitudes below 2^-126 give 0, and `small`
+// the largest of their high words: kSmall and more stand for results that are subnormal, not 0.
+constexpr unsigned kSmall = 873u << 20;   // 2^-150
+__device__ __forceinline__ float to_float(double v, unsigned& big, unsigned& small) {
   const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
   const unsigned mag = hi & 0x7fffffffu;
   const unsigned add = 0x0fffffffu + ((lo >> 29) & 1u);
   const unsigned l2 = lo + add, m2 = mag + (l2 < lo);
   big |= mag >= (1150u << 20);
+  const bool tiny = mag < (897u << 20);
+  if (tiny) small = max(small, mag);
   const unsigned f = ((m2 - (896u << 20)) << 3) | (l2 >> 29);
-  return __uint_as_float((hi & 0x80000000u) | (mag < (897u << 20) ? 0u : f));
+  return __uint_as_float((hi & 0x80000000u) | (tiny ? 0u : f));
 }
 
 // W <- W - pre - sum_k c_k v_k, norm partial part[block]; the correction accumulates in FP32 as in
@@ -780,7 +784,7 @@ __global__ void __launch_bounds__(32 * kWsNWarps, 1)
     if (pre.u[0]) w = ws_pre(w, pre.u[0], base, lane, n, sc[0], VEC == 2);
     if (pre.u[1]) w = ws_pre(w, pre.u[1], base, lane, n, sc[1], VEC == 2);
     float2 corr = make_float2(0.f, 0.f);
-    unsigned big = 0;
+    unsigned big = 0, small = 0;
     const double* vp = V;
     for (int k0 = 0; k0 < nk; k0 += 8) {
 #pragma unroll
@@ -792,9 +796,17 @@ __global__ void __launch_bounds__(32 * kWsNWarps, 1)
         const float cu[4] = {ck.x, ck.y, ck.z, ck.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          corr.x = fmaf(cu[u], to_float(v[h][u][0].x, big), corr.x);
-          corr.y = fmaf(cu[u], to_float(v[h][u][0].y, big), corr.y);
+          corr.x = fmaf(cu[u], to_float(v[h][u][0].x, big, small), corr.x);
+          corr.y = fmaf(cu[u], to_float(v[h][u][0].y, big, small), corr.y);
         }
+      }
+    }
+    if (small >= kSmall) {   // tails of decaying vectors: the conversions after all
+      corr = make_float2(0.f, 0.f);
+      for (int k = 0; k < nk; ++k) {
+        const double2 x = ws_load<VEC>(V + (int64_t)k * ld, base, lane, n);
+        corr.x = fmaf(cs[k], (float)x.x, corr.x);
+        corr.y = fmaf(cs[k], (float)x.y, corr.y);
       }
     }
     double2 cd = make_double2((double)corr.x, (double)corr.y);
