@@ -35,6 +35,7 @@ P_i32 = C.POINTER(C.c_int)
 _SIGS = {
     "gato_version": [],
     "gato_last_error": [C.c_char_p, C.c_size_t],
+    "gato_workspace_release": [],
     "gato_device_status": [P_i32, vp],
     "gato_dot": [i32, vp, vp, i64, f64, vp, vp],
     "gato_dot_noalloc": [i32, vp, vp, i64, f64, vp, vp],

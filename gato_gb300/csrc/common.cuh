@@ -76,6 +76,13 @@ struct WsBuf {
 };
 constexpr int kWsKeep = 8;
 constexpr size_t kWsKeepBytes = (size_t)1 << 30;
+// cudaMalloc for everything the library allocates: out of memory, it gives back what is kept and tries once more.
+cudaError_t device_malloc(void** p, size_t bytes);
+template <typename T>
+cudaError_t device_malloc(T** p, size_t bytes) {
+  return device_malloc(reinterpret_cast<void**>(p), bytes);
+}
+void ws_release();                                    // frees all kept workspace
 int ws_get(WsBuf& b, size_t bytes, cudaStream_t s);   // b holds at least `bytes`, usable on s from here on
 int ws_used(WsBuf& b, cudaStream_t s);                // the work queued on s so far uses b
 void ws_put(WsBuf& b);                                // gives b back

@@ -66,7 +66,7 @@ void* stream_scratch(cudaStream_t s, size_t bytes, int slot) {
   }
   size_t sz = bytes < (1u << 20) ? (1u << 20) : bytes;
   void* p = nullptr;
-  if (cudaMalloc(&p, sz) != cudaSuccess) {
+  if (device_malloc(&p, sz) != cudaSuccess) {
     e = {nullptr, 0};
     return nullptr;
   }
@@ -112,6 +112,26 @@ static void ws_free(WsBuf& b) {
   b = WsBuf{};
 }
 
+void ws_release() {
+  std::vector<WsBuf> kept;
+  {
+    std::lock_guard<std::mutex> lk(g_keep_mu);
+    kept.swap(g_ws);
+  }
+  for (auto& k : kept) ws_free(k);
+}
+
+cudaError_t device_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    ws_release();
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) cudaGetLastError();   // reported here, not by the next launch's check
+  return e;
+}
+
 int ws_get(WsBuf& b, size_t bytes, cudaStream_t s) {
   if (b.p && b.bytes >= bytes) {
     b.open = true;
@@ -140,17 +160,7 @@ int ws_get(WsBuf& b, size_t bytes, cudaStream_t s) {
     ws_free(b);
     GATO_CUDA_TRY(e);
   }
-  cudaError_t e = cudaMalloc(&b.p, bytes);
-  if (e != cudaSuccess) {   // give back what is kept and try once more
-    cudaGetLastError();
-    std::vector<WsBuf> kept;
-    {
-      std::lock_guard<std::mutex> lk(g_keep_mu);
-      kept.swap(g_ws);
-    }
-    for (auto& k : kept) ws_free(k);
-    e = cudaMalloc(&b.p, bytes);
-  }
+  cudaError_t e = device_malloc(&b.p, bytes);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     if (b.p) cudaFree(b.p);
@@ -373,6 +383,11 @@ __global__ void k_mix(T* rho, const T* __restrict__ rnew, int64_t npts, double a
 using namespace gato;
 
 extern "C" int gato_version(void) { return 1; }
+
+extern "C" int gato_workspace_release(void) {
+  ws_release();
+  return GATO_OK;
+}
 
 extern "C" long long gato_launch_count(void) { return g_launches.load(); }
 

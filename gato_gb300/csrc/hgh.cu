@@ -910,7 +910,7 @@ extern "C" int gato_nonlocal_create(int dtype, int N, double L, int K, const dou
   int st = GATO_OK;
   auto alloc = [&](void** p, size_t bytes) {
     if (st != GATO_OK) return;
-    if (cudaMalloc(p, bytes < 8 ? 8 : bytes) != cudaSuccess)
+    if (device_malloc(p, bytes < 8 ? 8 : bytes) != cudaSuccess)
       st = fail(GATO_ENOMEM, "nonlocal: allocation of %zu bytes failed", bytes);
   };
   auto up = [&](void* d, const void* h, size_t bytes) {

@@ -564,7 +564,7 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
     tw64[k] = make_double2(cos(a), -sin(a));
     tw32[k] = make_float2((float)tw64[k].x, (float)tw64[k].y);
   }
-  GATO_CUDA_TRY(cudaMalloc(&pl.tw, (size_t)M * 2 * ts));
+  GATO_CUDA_TRY(device_malloc(&pl.tw, (size_t)M * 2 * ts));
   // uploads go on s: a blocking cudaMemcpy from pageable memory may return before its DMA lands
   // and is not ordered against a non-blocking s, whose kernels read these tables next (a pageable
   // cudaMemcpyAsync returns once the host data is staged, so the vectors may go out of scope)
@@ -585,7 +585,7 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
         for (int n2 = 0; n2 < R2; ++n2) t32[(size_t)k1 * S + n2] = tw32[(size_t)n2 * k1];   // n2 k1 < M
     }
     const size_t bytes = dtype == GATO_F64 ? t64.size() * sizeof(double2) : t32.size() * sizeof(float2);
-    GATO_CUDA_TRY(cudaMalloc(&pl.tw2, bytes));
+    GATO_CUDA_TRY(device_malloc(&pl.tw2, bytes));
     GATO_CUDA_TRY(cudaMemcpyAsync(pl.tw2, dtype == GATO_F64 ? (void*)t64.data() : (void*)t32.data(), bytes,
                                   cudaMemcpyHostToDevice, s));
   }
@@ -598,16 +598,16 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
         const float c = (float)tw64[(size_t)n2 * k1].x, sn = (float)tw64[(size_t)n2 * k1].y;
         t4[(size_t)k1 * R2 + n2] = make_float4(c, c, sn, sn);
       }
-    GATO_CUDA_TRY(cudaMalloc(&pl.tw4, t4.size() * sizeof(float4)));
+    GATO_CUDA_TRY(device_malloc(&pl.tw4, t4.size() * sizeof(float4)));
     GATO_CUDA_TRY(cudaMemcpyAsync(pl.tw4, t4.data(), t4.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
   }
   double2* tw_d = nullptr;
-  GATO_CUDA_TRY(cudaMalloc(&tw_d, (size_t)M * sizeof(double2)));
+  GATO_CUDA_TRY(device_malloc(&tw_d, (size_t)M * sizeof(double2)));
   GATO_CUDA_TRY(cudaMemcpyAsync(tw_d, tw64.data(), (size_t)M * sizeof(double2), cudaMemcpyHostToDevice, s));
   // kernel spectrum in FP64 on an M^3 complex scratch
   double2* X = nullptr;
   const size_t xbytes = (size_t)M * M * M * sizeof(double2);
-  GATO_CUDA_TRY(cudaMalloc(&X, xbytes));
+  GATO_CUDA_TRY(device_malloc(&X, xbytes));
   const int L = pick_L<double2>(M, 0, 8);
   const size_t sm = fft_smem<double2>(M, L);
   GATO_TRY(set_smem(k_ghat_rows, sm));
@@ -619,7 +619,7 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
   ColGeom gx{0, 0, M, M, (int64_t)M * M, (int64_t)M * M, M, M, M};
   GATO_TRY(launch_cols<double2>(COL_FWD, X, X, gx, M, 1, pl.fp, tw_d, nullptr, pl.H, s));
   const int64_t oct = (int64_t)pl.H * pl.H * pl.H;
-  GATO_CUDA_TRY(cudaMalloc(&pl.ghat, oct * ts));
+  GATO_CUDA_TRY(device_malloc(&pl.ghat, oct * ts));
   const double scale = pl.dV / ((double)M * M * M);
   if (dtype == GATO_F64)
     k_ghat_extract<double><<<grid_for(oct, 256), 256, 0, s>>>(X, (double*)pl.ghat, M, pl.H, scale);
@@ -628,7 +628,7 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
   GATO_LAUNCH_TRY();
   if (pl.tw4) {
     const int64_t n2 = (int64_t)pl.H * pl.H * M;
-    GATO_CUDA_TRY(cudaMalloc(&pl.ghat2, n2 * sizeof(float)));
+    GATO_CUDA_TRY(device_malloc(&pl.ghat2, n2 * sizeof(float)));
     k_ghat_unfold_z<<<grid_for(n2, 256), 256, 0, s>>>((const float*)pl.ghat, (float*)pl.ghat2, M, pl.H);
     GATO_LAUNCH_TRY();
   }
@@ -637,14 +637,14 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
   cudaFree(tw_d);
   // spectral buffers
   const size_t cs = 2 * ts;
-  GATO_CUDA_TRY(cudaMalloc(&pl.S1, (size_t)max_fields * N * N * M * cs));
-  GATO_CUDA_TRY(cudaMalloc(&pl.S2, (size_t)max_fields * N * M * M * cs));
+  GATO_CUDA_TRY(device_malloc(&pl.S1, (size_t)max_fields * N * N * M * cs));
+  GATO_CUDA_TRY(device_malloc(&pl.S2, (size_t)max_fields * N * M * M * cs));
   // energy partials: 2 slots x (groups of a 40-field call) x row blocks (L >= 1);
   // the FP64 spectral pass needs 2 slots x fields x x-pass CTAs (room for 2 max_fields)
   pl.npart_cap = 2 * ((kMaxFields + max_fields - 1) / max_fields) * N * N;
   const int Lc = dtype == GATO_F64 ? fast::rows_L<double>(M) : 0;
   if (Lc > 0) pl.npart_cap = std::max(pl.npart_cap, 2 * 2 * max_fields * M * ((M + Lc - 1) / Lc));
-  GATO_CUDA_TRY(cudaMalloc(&pl.partials, (size_t)pl.npart_cap * sizeof(double)));
+  GATO_CUDA_TRY(device_malloc(&pl.partials, (size_t)pl.npart_cap * sizeof(double)));
   return side_get(pl.side);
 }
 

@@ -53,6 +53,12 @@ def pair_fields(n: int) -> int:
     return (n * (n + 1) // 2 + 2) // 2
 
 
+def release_workspace() -> None:
+    """Free the device memory that the library keeps from operators that are gone for later ones (at most
+    1 GB), after waiting for the device: for a program whose torch allocations run out."""
+    _lib.call("gato_workspace_release")
+
+
 class Operator:
     """Handle on a libgato_cuda operator: F = -1/2 L + V [+ V_nl] [- K]."""
 

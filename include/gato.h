@@ -58,6 +58,10 @@ typedef struct gato_operator* gato_op_t;
  * status and this message).                                                */
 int gato_version(void);
 int gato_last_error(char* buf, size_t len);
+/* Frees the device workspace kept from operators that are gone (at most 1 GB,
+ * reused by later ones), after waiting for the device: for a caller whose own
+ * allocator runs out. The library's own allocations do so by themselves.   */
+int gato_workspace_release(void);
 /* Reads and clears the device error word set by bounded spin-waits. */
 int gato_device_status(int* status_out, void* stream);
 /* Kernel launches issued by this library since it was loaded (all threads). */
