@@ -62,14 +62,17 @@ void free_after_pending(std::initializer_list<void*> ptrs);
 // ---- kept resources ------------------------------------------------------------------
 // Device workspace of an operator. Freed workspace is kept for the next operator (an energy or gradient
 // call makes one operator each, and cudaMalloc and cudaFree, the latter with a device synchronisation,
-// cost it a millisecond): `ev` marks its last use, and whoever takes it makes its own stream wait for
-// that, so threads and streams never overlap on it. At most kWsKeep buffers and kWsKeepBytes are kept per
-// process; the rest is freed, as is everything kept when an allocation fails. Work captured into a CUDA
-// graph pins its buffer (the graph may replay after the operator is gone): it is never handed on.
+// cost it a millisecond): `ev` marks its last use, on stream `last`. It goes to work of the same stream, which
+// comes after it anyway, or, once that use has ended, to any other: threads and streams neither overlap on it
+// nor wait for one another; where no kept buffer is free, one is allocated. At most kWsKeep buffers and
+// kWsKeepBytes are kept per process; the rest is freed, as is everything kept when an allocation fails. A
+// buffer in work captured into a CUDA graph is never handed on, only freed: with the operator, or when a later
+// call of it needs more. So a graph may replay as long as its operator lives and has not outgrown the capture.
 struct WsBuf {
   void* p = nullptr;
   size_t bytes = 0;
   cudaEvent_t ev = nullptr;
+  cudaStream_t last = nullptr;
   int dev = 0;
   bool captured = false;
   bool open = false;    // taken for work whose end is not marked (yet): a call that failed in between
@@ -122,14 +125,16 @@ int launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStre
 }
 
 // A side stream with the events that fork work onto it and join it back. Kept like workspace (at most
-// kSideKeep): work left in the stream merely runs before its next owner's.
+// kSideKeep): it goes to whoever forks from the stream it was forked from last, or to any other once its work
+// has ended. side_get is called before each fork from s.
 struct SideStream {
   cudaStream_t st = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  cudaStream_t last = nullptr;
   int dev = 0;
 };
 constexpr int kSideKeep = 16;
-int side_get(SideStream& x);
+int side_get(SideStream& x, cudaStream_t s);
 void side_put(SideStream& x);
 
 // sum_i a_i b_i * scale into out[0] (device), FP64 / float-float accumulation.

@@ -106,6 +106,18 @@ static bool is_capturing(cudaStream_t s) {
   return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
 }
 
+// A query of an event or a stream would end a capture of the global mode that another thread has under way,
+// unless the asking thread is in the relaxed mode.
+struct RelaxedQueries {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedQueries() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedQueries() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+static bool ended(cudaError_t query) {
+  if (query != cudaSuccess) cudaGetLastError();   // not ready
+  return query == cudaSuccess;
+}
+
 static void ws_free(WsBuf& b) {
   free_after_pending({b.p});
   if (b.ev) cudaEventDestroy(b.ev);
@@ -142,10 +154,14 @@ int ws_get(WsBuf& b, size_t bytes, cudaStream_t s) {
   GATO_CUDA_TRY(cudaGetDevice(&dev));
   const bool cap = is_capturing(s);   // a wait on work outside the capture would break it: fresh memory
   if (!cap) {
+    const RelaxedQueries relaxed;
     std::lock_guard<std::mutex> lk(g_keep_mu);
     int best = -1;
-    for (int i = 0; i < (int)g_ws.size(); ++i)
-      if (g_ws[i].dev == dev && g_ws[i].bytes >= bytes && (best < 0 || g_ws[i].bytes < g_ws[best].bytes)) best = i;
+    for (int i = 0; i < (int)g_ws.size(); ++i) {
+      const WsBuf& k = g_ws[i];
+      if (k.dev != dev || k.bytes < bytes || (best >= 0 && k.bytes >= g_ws[best].bytes)) continue;
+      if (k.last == s || ended(cudaEventQuery(k.ev))) best = i;
+    }
     if (best >= 0) {
       b = g_ws[best];
       g_ws.erase(g_ws.begin() + best);
@@ -179,6 +195,7 @@ int ws_used(WsBuf& b, cudaStream_t s) {
     return GATO_OK;
   }
   GATO_CUDA_TRY(cudaEventRecord(b.ev, s));
+  b.last = s;
   b.open = false;
   return GATO_OK;
 }
@@ -198,23 +215,31 @@ void ws_put(WsBuf& b) {
   ws_free(b);
 }
 
-int side_get(SideStream& x) {
-  if (x.st) return GATO_OK;
+int side_get(SideStream& x, cudaStream_t s) {
+  if (x.st) {
+    x.last = s;
+    return GATO_OK;
+  }
   int dev = 0;
   GATO_CUDA_TRY(cudaGetDevice(&dev));
   {
+    const RelaxedQueries relaxed;
     std::lock_guard<std::mutex> lk(g_keep_mu);
-    for (size_t i = 0; i < g_side.size(); ++i)
-      if (g_side[i].dev == dev && !is_capturing(g_side[i].st)) {   // not in another's unfinished capture
-        x = g_side[i];
-        g_side.erase(g_side.begin() + i);
-        return GATO_OK;
-      }
+    for (size_t i = 0; i < g_side.size(); ++i) {
+      const SideStream& k = g_side[i];
+      if (k.dev != dev || is_capturing(k.st)) continue;   // not in another's unfinished capture
+      if (k.last != s && !ended(cudaStreamQuery(k.st))) continue;
+      x = k;
+      x.last = s;
+      g_side.erase(g_side.begin() + i);
+      return GATO_OK;
+    }
   }
   GATO_CUDA_TRY(cudaStreamCreateWithFlags(&x.st, cudaStreamNonBlocking));
   GATO_CUDA_TRY(cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming));
   GATO_CUDA_TRY(cudaEventCreateWithFlags(&x.join, cudaEventDisableTiming));
   x.dev = dev;
+  x.last = s;
   return GATO_OK;
 }
 

@@ -71,7 +71,7 @@ static int fork_local(gato_operator& op, const void* in, void* out, int nb, cuda
                       cudaEvent_t* join) {
   *join = nullptr;
   if (!op.overlap) return local_part(op, in, out, nb, s);
-  GATO_TRY(side_get(op.side));
+  GATO_TRY(side_get(op.side, s));
   GATO_CUDA_TRY(cudaEventRecord(op.side.fork, s));
   GATO_CUDA_TRY(cudaStreamWaitEvent(op.side.st, op.side.fork, 0));
   GATO_TRY(local_part(op, in, out, nb, op.side.st));

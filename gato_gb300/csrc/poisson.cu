@@ -438,6 +438,7 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
       const bool fork = na < nf || la < nl;
       int rc = GATO_OK;
       if (fork) {
+        GATO_TRY(side_get(pl.side, s));
         GATO_CUDA_TRY(cudaEventRecord(pl.side.fork, s));
         GATO_CUDA_TRY(cudaStreamWaitEvent(pl.side.st, pl.side.fork, 0));
         if (rc == GATO_OK && na < nf) rc = transform(f0 + na, nf - na, na, false, pl.side.st);
@@ -645,7 +646,7 @@ static int plan_create(int dtype, int N, double h, double eps, int max_fields, P
   const int Lc = dtype == GATO_F64 ? fast::rows_L<double>(M) : 0;
   if (Lc > 0) pl.npart_cap = std::max(pl.npart_cap, 2 * 2 * max_fields * M * ((M + Lc - 1) / Lc));
   GATO_CUDA_TRY(device_malloc(&pl.partials, (size_t)pl.npart_cap * sizeof(double)));
-  return side_get(pl.side);
+  return side_get(pl.side, s);
 }
 
 static void plan_free(PoissonPlan& pl) {
