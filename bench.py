@@ -261,8 +261,8 @@ def e2e_pipelined(st, st_b, host_in, steps):
     ops, bufs, outs = [st["op"], st_b["op"]], [st["fields"], st_b["fields"]], [st["out"], st_b["out"]]
     hosts = [torch.empty_like(host_in).pin_memory() for _ in range(2)]
     ev = lambda: torch.cuda.Event()   # noqa: E731
-    try:   # each operator's block apply as a graph replay, as in the headline
-        graphs = [op.block_graph(o) for op, o in zip(ops, outs)]
+    try:   # each operator's block apply as a graph replay, its transforms in one strand beside the other's
+        graphs = [op.block_graph(o, strands=False) for op, o in zip(ops, outs)]
         steps_fn = [g.replay for g in graphs]
     except Exception:
         steps_fn = [lambda b=b: ops[b].apply_block(outs[b]) for b in range(2)]
@@ -489,7 +489,8 @@ def run_gato(args):
     # (no L2 flush between steps here: each step streams ~2.4 GB, far more than L2 holds)
     two_streams = None
     if graph is not None:
-        graph_b = s32b["op"].block_graph(s32b["out"])
+        graph_a = op32.block_graph(s32["out"], strands=False)
+        graph_b = s32b["op"].block_graph(s32b["out"], strands=False)
         sb = torch.cuda.Stream()
 
         def two(n):
@@ -498,7 +499,7 @@ def run_gato(args):
             e0.record(cur)
             sb.wait_stream(cur)
             for _ in range(n // 2):
-                graph.replay()
+                graph_a.replay()
                 with torch.cuda.stream(sb):
                     graph_b.replay()
             cur.wait_stream(sb)
@@ -509,7 +510,7 @@ def run_gato(args):
         n2 = 2 * max(3, args.steps // 2)
         two_streams = {"value": n2 / two(n2), "steps": n2,
                        "mode": "two operators, each step a graph replay on its own stream"}
-        del graph_b
+        del graph_a, graph_b
 
     # ---- plain FP64 and matvec rates ----------------------------------------------
     k64 = max(2, args.steps // 4)

@@ -55,6 +55,7 @@ _SIGS = {
     "gato_hartree_energy": [vp, vp, vp, vp],
     "gato_poisson_stage": [vp, i32, i32, vp],
     "gato_poisson_tune": [vp, i32, i32],
+    "gato_poisson_strands": [vp, i32],
     "gato_op_tune": [vp, i32],
     "gato_op_overlap": [vp, i32],
     "gato_density": [i32, vp, i32, i64, vp, vp],

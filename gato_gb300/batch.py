@@ -31,6 +31,7 @@ from .grid import Grid3D
 from .physics import _molecule as mol
 from .physics.water import water_initial_geometry
 from .pseudopotentials import lookup
+from .solvers.poisson import thread_strands
 
 SPECIES = ("H2", "LiH", "HCl", "H2O")
 GRIDS = (64, 96, 128, 160)
@@ -117,6 +118,9 @@ def solve_batch(specs, *, precision: str = "mixed", streams: int = 8, max_iters:
 
     def worker(k: int):
         torch.cuda.set_device(dev)
+        # several workers' systems fill one another's gaps: second strands only add to the streams that contend
+        # (48 systems, 12 SCF iterations each, 8 workers: 39.0 s with them, 38.1 without)
+        thread_strands(streams <= 1)
         s = torch.cuda.Stream(device=dev)
         with torch.cuda.stream(s):
             while not errors:

@@ -430,7 +430,7 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
       const int nl = lf0 >= nfull ? std::min(group - nf, args.nf - lf0) : 0;
       // two strands of about equal work, the second on the plan's own stream
       int na = nf, la = nl;
-      if (strands && two_strands(sizeof(T), N)) {
+      if (strands && pl.strands && two_strands(sizeof(T), N)) {
         const int share = (2 * nf + nl + 1) / 2;
         na = std::min(nf, (share + 1) / 2);
         la = na == nf ? std::min(nl, std::max(share - 2 * nf, 0)) : 0;
@@ -801,6 +801,12 @@ extern "C" int gato_poisson_stage(gato_poisson_t plan, int stage, int nf, void* 
 // with the multi-field z forward from three fields; 4: as 0, with the scalar
 // FP32 column passes instead of the packed two-line ones and the z forward
 // staging once per CTA instead of persistent CTAs with double-buffered staging).
+extern "C" int gato_poisson_strands(gato_poisson_t plan, int on) {
+  if (!plan) return fail(GATO_EBADARG, "null plan");
+  plan->p.strands = on ? 1 : 0;
+  return GATO_OK;
+}
+
 extern "C" int gato_poisson_tune(gato_poisson_t plan, int group, int engine) {
   if (!plan || group < 0 || group > plan->p.max_fields || engine < 0 || engine > 4)
     return fail(GATO_EBADARG, "gato_poisson_tune: bad arguments");

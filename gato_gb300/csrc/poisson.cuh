@@ -51,6 +51,7 @@ struct PoissonPlan {
   double* partials = nullptr;
   int npart_cap = 0;
   SideStream side;         // second strand of the transforms
+  int strands = 1;         // 0: every transform on the caller's stream
   int group = 0;           // fields per launch group (0: max_fields)
   int engine = 0;          // 0: register two-pass kernels where M allows, 1: generic Stockham
                            // (2, 3: z-forward variants; 4: as 0 with the scalar column passes)

@@ -117,8 +117,11 @@ class Operator:
         _lib.call("gato_op_apply_block", self.handle, C.c_void_p(out.data_ptr()), C.c_void_p(_lib.stream()))
         return out
 
-    def block_graph(self, out: torch.Tensor) -> torch.cuda.CUDAGraph:
+    def block_graph(self, out: torch.Tensor, strands: bool | None = None) -> torch.cuda.CUDAGraph:
         """``apply_block(out)`` captured once as a CUDA graph; ``replay()`` re-runs its launches.
+
+        ``strands`` is the plan's ``strands`` setting in the graph (None: as the plan has it); a graph that
+        replays beside another operator's runs faster without them.
 
         The graph holds the addresses of the orbitals, potential, projectors, plan
         buffers and ``out``: their values may change between replays, their
@@ -127,14 +130,22 @@ class Operator:
         allocate its pair-potential buffer, so nothing allocates inside the graph;
         the block apply uses no per-stream scratch. Replays on one stream at a
         time: the plan's spectral buffers and the projector object are shared."""
-        g = torch.cuda.CUDAGraph()
-        side = torch.cuda.Stream()
-        side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):
-            self.apply_block(out)
-        torch.cuda.current_stream().wait_stream(side)
-        with torch.cuda.graph(g, stream=side, capture_error_mode="relaxed"):
-            self.apply_block(out)
+        plan = self._keep.get("plan") if strands is not None else None
+        if plan is not None:
+            before = plan.two_strands
+            plan.strands(strands)
+        try:
+            g = torch.cuda.CUDAGraph()
+            side = torch.cuda.Stream()
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                self.apply_block(out)
+            torch.cuda.current_stream().wait_stream(side)
+            with torch.cuda.graph(g, stream=side, capture_error_mode="relaxed"):
+                self.apply_block(out)
+        finally:
+            if plan is not None:
+                plan.strands(before)
         return g
 
     def energy_terms(self, V_ext: torch.Tensor | None) -> torch.Tensor:

@@ -32,6 +32,15 @@ class PoissonPlan:
             _lib._lib.gato_poisson_destroy(h)
             self.handle = None
 
+    two_strands = True
+
+    def strands(self, on: bool):
+        """Let a call's transforms run as two strands on two streams (True, the default: the faster single
+        call), or keep them on the caller's stream (False: for two or more calls in flight on streams of
+        their own, which fill each other's gaps already); the same results either way."""
+        _lib.call("gato_poisson_strands", self.handle, int(bool(on)))
+        self.two_strands = bool(on)
+
     def potential(self, rho: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         if out is None:
             out = torch.empty_like(rho)
@@ -59,6 +68,11 @@ class PoissonPlan:
 _TLS = threading.local()
 
 
+def thread_strands(on: bool) -> None:
+    """The ``strands`` setting of the plans that ``get_plan`` makes for the calling thread from here on."""
+    _TLS.strands = bool(on)
+
+
 def _plans() -> "OrderedDict[tuple, PoissonPlan]":
     d = getattr(_TLS, "plans", None)
     if d is None:
@@ -75,6 +89,8 @@ def get_plan(N: int, h: float, eps: float, dtype=torch.float64, max_fields: int 
         if p is not None:
             del _PLANS[key]
         p = PoissonPlan(N, h, eps, dtype, max_fields)
+        if not getattr(_TLS, "strands", True):
+            p.strands(False)
         _PLANS[key] = p
         while len(_PLANS) > 3:
             _PLANS.popitem(last=False)

@@ -160,6 +160,12 @@ int gato_poisson_stage(gato_poisson_t plan, int stage, int nf, void* stream);
  * {128,160,192,256,320}, and a z forward that stages once per CTA
  * instead of persistent CTAs with double-buffered staging).              */
 int gato_poisson_tune(gato_poisson_t plan, int group, int engine);
+/* Tuning (no reference counterpart): 1 (default) lets the transforms of a
+ * call on the plan run as two strands, half of the fields each, one of them
+ * on a stream of the plan's own: the faster single call. 0 keeps them on the
+ * caller's stream: for programs that keep two or more calls in flight on
+ * streams of their own, which fill each other's gaps already. Same bits.   */
+int gato_poisson_strands(gato_poisson_t plan, int on);
 
 /* ---- scf.py ----------------------------------------------------------------
  * rho = 2 sum_i phi_i^2 (scf.py:61-63), orbitals field-major.             */
