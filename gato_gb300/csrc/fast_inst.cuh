@@ -21,7 +21,7 @@ using Row = Launch<T, A, B, kF32 ? L32 : L64>;
 
 template <>
 int rows_L_g<T, kG>(int M) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return kF32 ? L32 : L64;
   switch (M) { GATO_FAST_SHAPES(X) }
 #undef X
@@ -31,7 +31,7 @@ int rows_L_g<T, kG>(int M) {
 template <>
 int cols_g<T, kG>(int M, int mode, const T2* in, T2* out, const ColGeom& g, int outer, int nf, const T2* tw,
                   const T* ghat, int H, cudaStream_t s) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return Row<A, B, L32, L64>::cols(mode, in, out, g, outer, nf, tw, ghat, H, s);
   GATO_FAST_CALL(X);
 #undef X
@@ -39,7 +39,7 @@ int cols_g<T, kG>(int M, int mode, const T2* in, T2* out, const ColGeom& g, int 
 
 template <>
 int rows_fwd_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw, int multi, cudaStream_t s) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return Row<A, B, L32, L64>::rows_fwd(a, f0, nfg, S1, tw, multi, s);
   GATO_FAST_CALL(X);
 #undef X
@@ -48,7 +48,7 @@ int rows_fwd_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, T2* S1, const T
 template <>
 int rows_inv_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,
                       bool energy, double* partials, int64_t slot_stride, cudaStream_t s) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return Row<A, B, L32, L64>::rows_inv(a, f0, nfg, S1, tw, accumulate, energy, partials, slot_stride, s);
   GATO_FAST_CALL(X);
 #undef X
@@ -56,7 +56,7 @@ int rows_inv_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, const T2* S1, c
 
 template <>
 int rows_inv_j_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, cudaStream_t s) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return Row<A, B, L32, L64>::rows_inv_j(a, f0, nfg, S1, tw, s);
   GATO_FAST_CALL(X);
 #undef X
@@ -64,7 +64,7 @@ int rows_inv_j_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, const T2* S1,
 
 template <>
 int rows_fwd_real_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw, cudaStream_t s) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return Row<A, B, L32, L64>::rows_fwd_real(a, f0, nfg, S1, tw, s);
   GATO_FAST_CALL(X);
 #undef X
@@ -73,7 +73,7 @@ int rows_fwd_real_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, T2* S1, co
 template <>
 int rows_inv_real_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, const T2* S1, const T2* tw, int accumulate,
                            bool j, cudaStream_t s) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return Row<A, B, L32, L64>::rows_inv_real(a, f0, nfg, S1, tw, accumulate, j, s);
   GATO_FAST_CALL(X);
 #undef X
@@ -83,7 +83,7 @@ int rows_inv_real_g<T, kG>(int M, const PassArgs& a, int f0, int nfg, const T2* 
 template <>
 int cols_fe_g<T, kG>(int M, const T2* in, const ColGeom& g, int outer, int nf, const T2* tw, const T* ghat, int H,
                      const FeArgs& fa, cudaStream_t s) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return Row<A, B, L32, L64>::cols_fe(in, g, outer, nf, tw, ghat, H, fa, s);
   GATO_FAST_CALL(X);
 #undef X

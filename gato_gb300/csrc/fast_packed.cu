@@ -6,8 +6,16 @@ namespace gato {
 namespace fast {
 
 int shape_r2(int M) {
-#define X(MM, A, B, L32, L64) \
+#define X(MM, A, B, L32, L64, A32, J32) \
   case MM: return B;
+  switch (M) { GATO_FAST_SHAPES_ALL(X) }
+#undef X
+  return 0;
+}
+
+int strand_fields(int M, bool j) {
+#define X(MM, A, B, L32, L64, A32, J32) \
+  case MM: return j ? J32 : A32;
   switch (M) { GATO_FAST_SHAPES_ALL(X) }
 #undef X
   return 0;

@@ -300,12 +300,22 @@ int launch_cols(int mode, const T2* in, T2* out, const ColGeom& g, int outer, in
 // Whether a call's transforms run as two strands, half of the fields each on its own stream: every
 // pass has a last wave that leaves SMs idle and the passes have unlike bounds (memory, the FP64 or FP32
 // pipe, barriers), so one strand fills the other's gaps. Measured, one strand against two, exchange of
-// 3 / 4 / 5 / 8 orbitals, us. FP64: 71 / 41 / 77 / 60 against 52 / 43 / 58 / 54 at N = 16, 113 / 90 / 148 /
-// 151 against 78 / 81 / 115 / 138 at 32, 1076 / 1245 / 1682 / 2480 against 949 / 1168 / 1543 / 2331 at 80,
-// 3344 / 4304 / 5496 / 8456 against 3268 / 4225 / 5410 / 8513 at 128. FP32: 46 / 46 / 56 / 68 against 44 /
-// 42 / 54 / 65 at N = 64, 192 / 201 / 286 / 387 against 182 / 187 / 272 / 353 at 128; below, the fork and the
-// extra launches cost what the overlap gives (30 / 30 / 39 / 43 against 35 / 30 / 38 / 42 at N = 48).
-bool two_strands(size_t ts, int N) { return ts == 8 || N >= 64; }
+// 3 / 4 / 5 / 8 / 10 orbitals (2, 2, 3, 4, 5 fields), us. FP64: 52 / 33 / 60 / 49 / 60 against 39 / 33 / 44 / 46 /
+// 56 at N = 16, 83 / 77 / 117 / 138 / 172 against 69 / 76 / 103 / 130 / 167 at 32, 995 / 1230 / 1599 / 2464 / 2937
+// against 899 / 1163 / 1496 / 2324 / 2915 at 80, 3276 / 4288 / 5428 / 8446 / 10553 against 3214 / 4225 / 5357 / 8509 /
+// 10528 at 128: always. FP32, from N = 64 up (below, the fork and the extra launches cost what the overlap
+// gives): 88 / 91 / 134 / 187 / 233 against 86 / 87 / 127 / 172 / 218 at 96, 180 / 188 / 274 / 376 / 456 against 178 /
+// 184 / 269 / 349 / 444 at 128, a block apply of 2 / 3 / 4 / 5 orbitals (2, 3, 5, 8 fields) 36 / 48 / 72 / 107 against
+// 36 / 46 / 65 / 97 at 64; there, one field a strand is all latency (exchange 31.7 / 32.3 / 44.0 / 56.4 / 73.5 against
+// 34.3 / 34.3 / 43.6 / 55.9 / 68.2), so from three. Shapes without packed column passes gain up to a number of fields
+// of their own (fast_shapes.cuh): N = 98 exchange 117 / 122 / 178 / 238 / 296 against 104 / 106 / 174 / 251 / 325, block
+// 131 / 201 / 311 / 470 against 122 / 213 / 345 / 530; N = 140 exchange 343 / 357 / 512 / 702 / 839 against 337 / 350 / 604 /
+// 816 / 1020, block 316 / 469 / 785 / 1220 against 313 / 475 / 951 / 1485. Energies of FP32 fields take the smaller limit.
+bool two_strands(size_t ts, int N, int fields, int epi) {
+  if (ts == 8) return true;
+  const int acc = fast::strand_fields(2 * N, false), j = fast::strand_fields(2 * N, true);
+  return fields >= (N == 64 ? 3 : 2) && fields <= (epi == EPI_ACC ? acc : epi == EPI_J ? j : std::min(acc, j));
+}
 
 template <typename T>
 int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, double* energy_dev,
@@ -430,7 +440,7 @@ int run_typed(PoissonPlan& pl, const PassArgs& args, int epi, bool accumulate, d
       const int nl = lf0 >= nfull ? std::min(group - nf, args.nf - lf0) : 0;
       // two strands of about equal work, the second on the plan's own stream
       int na = nf, la = nl;
-      if (strands && pl.strands && two_strands(sizeof(T), N)) {
+      if (strands && pl.strands && two_strands(sizeof(T), N, nf + nl, epi)) {
         const int share = (2 * nf + nl + 1) / 2;
         na = std::min(nf, (share + 1) / 2);
         la = na == nf ? std::min(nl, std::max(share - 2 * nf, 0)) : 0;

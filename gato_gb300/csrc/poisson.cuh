@@ -129,6 +129,7 @@ int rows_inv_real_g(int M, const PassArgs& a, int f0, int nfg, const C2<T>* S1, 
   return r
 
 int shape_r2(int M);   // R2 of the register engine's M = R1 R2, 0 if none
+int strand_fields(int M, bool j);   // the most FP32 fields that two strands transform faster than one (j: to J fields)
 template <typename T>
 int rows_L(int M) {    // lines per CTA of the z kernels, 0 if unsupported
   const int r = rows_L_g<T, 0>(M) + rows_L_g<T, 1>(M) + rows_L_g<T, 2>(M) + rows_L_g<T, 3>(M);

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 def captured_edges(call):
-    """(nodes, edges, most edges out of a node) of the graph that call() makes of the current stream."""
+    """(nodes, edges, most edges out of or into a node) of the graph that call() makes of the current stream."""
     cu = C.CDLL("libcuda.so.1")
     stream = torch.cuda.Stream()
     stream.wait_stream(torch.cuda.current_stream())
@@ -28,7 +28,7 @@ def captured_edges(call):
         src, dst = (C.c_void_p * e.value)(), (C.c_void_p * e.value)()
         data = (C.c_uint64 * e.value)()   # eight bytes an edge
         assert cu.cuGraphGetEdges_v2(graph, src, dst, data, C.byref(e)) == 0
-        return n.value, e.value, max(list(src).count(x) for x in src)
+        return n.value, e.value, max(list(q).count(x) for q in (src, dst) for x in q)
     finally:
         cu.cuGraphDestroy(graph)
 
