@@ -65,6 +65,12 @@ static int local_part(gato_operator& op, const void* in, void* out, int nb, cuda
   return GATO_OK;
 }
 
+// A call that fails behind the fork still leaves s behind what it forked: the caller may free the outputs.
+static int joined(int rc, cudaStream_t s, cudaEvent_t join) {
+  if (rc != GATO_OK && join) cudaStreamWaitEvent(s, join, 0);
+  return rc;
+}
+
 // Runs the local part on the side stream from this point of s; returns the join event
 // (null when the local part ran on s itself).
 static int fork_local(gato_operator& op, const void* in, void* out, int nb, cudaStream_t s,
@@ -74,19 +80,19 @@ static int fork_local(gato_operator& op, const void* in, void* out, int nb, cuda
   GATO_TRY(side_get(op.side, s));
   GATO_CUDA_TRY(cudaEventRecord(op.side.fork, s));
   GATO_CUDA_TRY(cudaStreamWaitEvent(op.side.st, op.side.fork, 0));
-  GATO_TRY(local_part(op, in, out, nb, op.side.st));
+  const int rc = local_part(op, in, out, nb, op.side.st);
   GATO_CUDA_TRY(cudaEventRecord(op.side.join, op.side.st));
   *join = op.side.join;
-  return GATO_OK;
+  return joined(rc, s, *join);
 }
 
 int op_apply(gato_operator& op, const void* in, void* out, cudaStream_t s, int chain) {
   if (op.n_orb <= 0) return local_part(op, in, out, 1, s, chain);
-  cudaEvent_t join = nullptr;
-  GATO_TRY(fork_local(op, in, out, 1, s, &join));
   PassArgs a;
   GATO_TRY(exchange_args(a, in, op.orbitals, op.n_orb, op_esize(op), op_n3(op), out, -1.0));
-  return poisson_run(op.pp->p, a, EPI_ACC, true, nullptr, s, join, op.overlap);
+  cudaEvent_t join = nullptr;
+  GATO_TRY(fork_local(op, in, out, 1, s, &join));
+  return joined(poisson_run(op.pp->p, a, EPI_ACC, true, nullptr, s, join, op.overlap), s, join);
 }
 
 static void block_pairs(PassArgs& a, const gato_operator& op, void* out, bool energy) {
@@ -225,24 +231,24 @@ extern "C" int gato_op_apply_block(gato_op_t op, void* out, void* stream) {
   if (!op || !out || op->n_orb < 1) return fail(GATO_EBADARG, "gato_op_apply_block: needs orbitals");
   if (op->n_orb > kMaxOut) return fail(GATO_EUNSUPPORTED, "block apply: at most %d orbitals", kMaxOut);
   cudaStream_t s = as_stream(stream);
-  cudaEvent_t join = nullptr;
-  GATO_TRY(fork_local(*op, op->orbitals, out, op->n_orb, s, &join));
   PassArgs a;
   block_pairs(a, *op, out, false);
   // one orbital has one pair potential with one use: its z-inverse epilogue applies it directly
-  const bool jf = op->block_epi == 1 || (op->block_epi == 0 && op->n_orb > 1);
-  if (jf && poisson_j_supported(op->pp->p)) {
-    // pair potentials to J fields, then one elementwise pass: out_i -= sum_j phi_j J_ij
+  const bool jf = (op->block_epi == 1 || (op->block_epi == 0 && op->n_orb > 1)) && poisson_j_supported(op->pp->p);
+  if (jf) {
     const size_t need = (size_t)2 * a.nf * op_n3(*op) * op_esize(*op);
     GATO_TRY(ws_get(op->jbuf, need, s));
     a.jbase = op->jbuf.p;
     a.jstride = op_n3(*op);
-    GATO_TRY(poisson_run(op->pp->p, a, EPI_J, false, nullptr, s, nullptr, op->overlap));
-    if (join) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
-    GATO_TRY(pair_exchange(op->dtype, op->orbitals, op->n_orb, op->jbuf.p, out, op_n3(*op), s));
-    return ws_used(op->jbuf, s);
   }
-  return poisson_run(op->pp->p, a, EPI_ACC, true, nullptr, s, join, op->overlap);
+  cudaEvent_t join = nullptr;
+  GATO_TRY(fork_local(*op, op->orbitals, out, op->n_orb, s, &join));
+  if (!jf) return joined(poisson_run(op->pp->p, a, EPI_ACC, true, nullptr, s, join, op->overlap), s, join);
+  // pair potentials to J fields, then one elementwise pass: out_i -= sum_j phi_j J_ij
+  GATO_TRY(joined(poisson_run(op->pp->p, a, EPI_J, false, nullptr, s, nullptr, op->overlap), s, join));
+  if (join) GATO_CUDA_TRY(cudaStreamWaitEvent(s, join, 0));
+  GATO_TRY(pair_exchange(op->dtype, op->orbitals, op->n_orb, op->jbuf.p, out, op_n3(*op), s));
+  return ws_used(op->jbuf, s);
 }
 
 extern "C" int gato_op_overlap(gato_op_t op, int on) {
