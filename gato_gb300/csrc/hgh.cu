@@ -10,6 +10,7 @@
 // points, reduce the overlaps <p_q|psi> through distributed shared memory,
 // form the h-matrix contraction and scatter-add each atom's projectors in
 // turn (a cluster barrier between atoms, so overlapping boxes never race).
+#include <atomic>
 #include <cmath>
 #include <vector>
 
@@ -649,10 +650,14 @@ static bool big_boxes(const Nonlocal& nl) {
   return nl.nvals >= (nl.dtype == GATO_F64 ? 1 << 19 : 1 << 17) && 4 * nl.nvals >= (int64_t)nl.N * nl.N * nl.N;
 }
 
-// Whether the GPU takes clusters of kNlClusterBig CTAs of this kernel (more than the portable size).
+// Whether the current GPU takes clusters of kNlClusterBig CTAs of this kernel (more than the portable size, for
+// which the kernel opts in on each device).
 template <typename K>
 static bool big_clusters(K kern) {
-  static const bool ok = [kern] {   // one kernel per instantiation of K's type
+  static std::atomic<int8_t> known[32];   // by device: 0 not asked yet, 1 yes, 2 no; one kernel per type K
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 32) return false;
+  if (known[dev].load() == 0) {
     const void* f = reinterpret_cast<const void*>(kern);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(kNlClusterBig);
@@ -666,9 +671,9 @@ static bool big_clusters(K kern) {
     const bool fits = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
                       cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n > 0;
     cudaGetLastError();
-    return fits;
-  }();
-  return ok;
+    known[dev].store(fits ? 1 : 2);
+  }
+  return known[dev].load() == 1;
 }
 
 int nonlocal_apply(Nonlocal& nl, const void* psi, void* out, int nb, cudaStream_t s, bool after_stencil) {
