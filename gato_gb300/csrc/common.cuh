@@ -93,8 +93,8 @@ void ws_put(WsBuf& b);                                // gives b back
 // Launches a kernel that may begin while the one ahead of it in the stream drains: its launch latency and
 // the work it does before gdc_wait (ptx.cuh: barriers, constant tables) fall under the predecessor's end.
 // Every block calls gdc_wait before it reads or writes anything an earlier kernel touches, so a kernel
-// that has ended vouches for all before it; and it takes no const __restrict__ pointers, whose loads could
-// move ahead of the wait. Exchange of 3 / 8 orbitals, plain launches against these, us: FP32 24 / 30
+// that has ended vouches for all before it; and it takes const __restrict__ pointers, whose loads could
+// move ahead of the wait, only to tables that were complete before the call that made them returned. Exchange of 3 / 8 orbitals, plain launches against these, us: FP32 24 / 30
 // against 14 / 18 at N = 16, 27 / 43 against 19 / 31 at 40, 42 / 66 against 35 / 56 at 64, 182 / 353
 // against 177 / 348 at 128; FP64 52 / 54 against 38 / 46 at N = 16, 80 / 136 against 71 / 130 at 32,
 // 1431 / 3656 against 1426 / 3655 at 96. No FFT kernel lets its successor begin earlier still (gdc_launch

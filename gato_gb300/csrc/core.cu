@@ -346,9 +346,8 @@ int encode_tma(void* out128, int dtype, const void* base, const TmaBox& b) {
 // ---- grid.py reductions --------------------------------------------------------
 
 template <typename T>
-__global__ void k_dot_partials(const T* a, const T* b, int64_t n, double* partials) {
+__global__ void k_dot_partials(const T* __restrict__ a, const T* __restrict__ b, int64_t n, double* partials) {
   __shared__ double sh[32];
-  gdc_wait();
   Acc<T> acc;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {

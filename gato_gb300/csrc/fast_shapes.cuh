@@ -1,8 +1,8 @@
 // Shapes of the register-resident two-pass engine: M = 2N -> (R1, R2, lines per CTA FP32, FP64, FP32
 // strands accumulating, to J).
 // R1 and R2 are even: the zero-padded half of every transform maps to whole register slots, and the
-// x pass folds the kernel spectrum at R2 / 2. Every even N <= 144 whose 2N factors into 2, 3, 5 and 7
-// has one (and N = 160); the rest, odd N among them, takes the Stockham engine. On FP32 fields that
+// x pass folds the kernel spectrum at R2 / 2. Every even N from 16 to 144 whose 2N factors into 2, 3, 5
+// and 7 has one (and N = 160); the rest, smaller and odd N among them, takes the Stockham engine. On FP32 fields that
 // engine is 1.6 (N = 18) to 6 (N = 144) times slower than these shapes (exchange with four orbitals:
 // 462 against 167 us at N = 100, 2088 against 347 at 144); on FP64 fields, where the FP64 pipe binds
 // both, 0 to 25 % (1146 against 917 us at N = 72).

@@ -1206,18 +1206,16 @@ __global__ void __launch_bounds__(256) k_ritz(const T* __restrict__ V, int64_t l
 
 struct LzScratch {
   double *part, *coef, *nrm, *Y, *work, *apart;
-  int nblk;     // k_gemv_n grid
-  int nblk_t;   // k_gemv_t grid
-  int nblk_b;   // bulk-streaming grid (both sweeps)
+  int nblk;     // k_gemv_n grid (FP32)
+  int nblk_t;   // k_gemv_t grid (FP32)
+  int nblk_b;   // bulk-streaming grid (FP32, both sweeps), warp-share grid (FP64)
 };
 
 // One resident wave each: k_gemv_n holds 3 blocks of kLzThreads per SM (80
 // registers); k_gemv_t, which is bound by memory latency, runs as many as its
-// registers allow (48 FP32 / 62 FP64: 5 / 4 blocks) to keep more loads in flight.
+// registers allow (48: 5 blocks) to keep more loads in flight.
 inline int lz_nblk(int64_t n) { return (int)std::min<int64_t>((n + kChunk - 1) / kChunk, 3 * 152); }
-inline int lz_nblk_t(int64_t n, bool fp64) {
-  return (int)std::min<int64_t>((n + kChunk - 1) / kChunk, (fp64 ? 4 : 5) * 152);
-}
+inline int lz_nblk_t(int64_t n) { return (int)std::min<int64_t>((n + kChunk - 1) / kChunk, 5 * 152); }
 // FP32 bulk-streaming kernels: 3 blocks per SM (their ring is 48 KB), at least one item each. FP64
 // warp-share kernels: one block per SM, at least one chunk each.
 inline int lz_nblk_b(int64_t n, bool fp64) {
@@ -1227,8 +1225,8 @@ inline int lz_nblk_b(int64_t n, bool fp64) {
 }
 
 int lz_scratch(cudaStream_t s, int64_t n, int m, int K, LzScratch& z, bool fp64) {
-  z.nblk = lz_nblk(n);
-  z.nblk_t = lz_nblk_t(n, fp64);
+  z.nblk = fp64 ? 0 : lz_nblk(n);
+  z.nblk_t = fp64 ? 0 : lz_nblk_t(n);
   z.nblk_b = lz_nblk_b(n, fp64);
   const int np = std::max(std::max(z.nblk, z.nblk_t), z.nblk_b);
   // partials (m+1)*max(grids), coefficients (m+1), norm, Y (m*K), LU work 7*m*K
@@ -1458,10 +1456,10 @@ int lz_finish(const T* Vb, int64_t n, int m, int K, double tol, const double* al
 // fz_stages). Only the FP32 basis takes this path: FP64 products would make
 // the sweep FP64-bound on GB300. After each sweep, k_fz_form sums the block
 // partials (one warp per row), forms alpha_j, the next correction row and w^_j;
-// k_fz_post2 forms beta_j and the next sweep's coefficients while the operator is
-// applied to w^_j. All are chained launches in one stream; k_fz_post2 lets a
-// local operator's stencil begin once k_fz_form is complete and run beside it
-// (64^3, m = 80, a run: post2 on a stream of its own, forked and joined by
+// k_fz_post2 forms beta_j and the next sweep's coefficients. All are chained
+// launches in one stream; k_fz_post2 lets a local operator's stencil begin once
+// k_fz_form is complete and run beside it, an operator with exchange forks and
+// transforms behind it (64^3, m = 80, a run: post2 on a stream of its own, forked and joined by
 // events, 2937 us; chained in turn 2460; chained and beside 2329; 32^3 2224,
 // 1704, 1629; 128^3, m = 60, 6024, 5816, 5576).
 constexpr int kFzCE = 128;                  // the middle chunk width; n must be a multiple

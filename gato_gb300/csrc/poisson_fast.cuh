@@ -952,8 +952,8 @@ struct Launch {
   // multi: 0 per-field CTAs, 1 multi-field CTAs from three fields up, 2 from two fields up
   // (persistent, double-buffered staging where the rows allow bulk copies), 3 as 2 with one
   // staging round trip per CTA (the non-persistent kernel)
-  // (the default: with bulk staging the multi-field kernel wins at two fields too,
-  // 239 against 244 us for the 128^3 matvec)
+  // (the default: with bulk staging the multi-field kernel wins at two fields too, 239 against 244 us for the
+  // 128^3 matvec in one strand; in two, each strand of a call of two fields has one and takes its own kernel)
   static int rows_fwd(const PassArgs& a, int f0, int nfg, T2* S1, const T2* tw, int multi, cudaStream_t s) {
     // several fields over few distinct inputs: stage the inputs once per CTA
     RowsIn ri;

@@ -325,16 +325,20 @@ __global__ void __launch_bounds__(kZP*(kBY / YPT))
 std::atomic<int> g_rows_per_thread{0};
 constexpr int kDefaultRows = 2;
 
+int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return 152;
+  return sms;
+}
+
 // Resident CTAs of a kernel on the whole GPU (occupancy x SMs).
 template <typename K>
 int resident_ctas(K kernel, int threads, int smem) {
-  int dev = 0, sms = 0, per = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess ||
-      per <= 0)
-    return 152;
-  return per * sms;
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess || per <= 0) per = 1;
+  return per * device_sms();
 }
 
 template <typename T, int R, int YPT, bool HAS_V, bool STORE, bool DOT, bool EDGE>
@@ -369,7 +373,7 @@ int launch_tma_edge(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int
   // on fewer SMs disturbs a one-wave kernel less (helium matvec at 64^3 198 us,
   // spread out 202).
   static const int cap = resident_ctas(kern, kThreads, G::SMEM);   // one value per instantiation
-  constexpr int kSms = 152;
+  static const int sms = device_sms();
   int chunks;
   if (sizeof(T) == 8 && !beside) {
     // FP64 fields: the SM with the most planes on its FP64 pipe sets the time
@@ -378,7 +382,7 @@ int launch_tma_edge(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int
     for (int c = 1; c <= nx; ++c) {
       const int64_t ctas = (int64_t)tiles * nb * ((nx + c - 1) / c);
       if (c < nx && ctas > (int64_t)4096 * nb) continue;   // the dot's partials per field
-      const int64_t load = (ctas + kSms - 1) / kSms * (c + 1);
+      const int64_t load = (ctas + sms - 1) / sms * (c + 1);
       if (load < cost) {
         cost = load;
         best = c;
@@ -387,7 +391,7 @@ int launch_tma_edge(const CUtensorMap& tm, const CUtensorMap& vm, void* out, int
     chunks = (nx + best - 1) / best;
   } else {
     chunks = (int)std::max<int64_t>(1, cap / ((int64_t)tiles * nb));
-    const int fine = sizeof(T) == 8 ? 1 : (int)std::min<int64_t>(nx, kSms / ((int64_t)tiles * nb));
+    const int fine = sizeof(T) == 8 ? 1 : (int)std::min<int64_t>(nx, sms / ((int64_t)tiles * nb));
     chunks = std::min(chunks, std::max(std::max(1, nx / 4), fine));
   }
   const int cx = (nx + chunks - 1) / chunks;

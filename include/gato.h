@@ -152,9 +152,9 @@ int gato_hartree_energy(gato_poisson_t plan, const void* rho, double* E_dev, voi
 int gato_poisson_stage(gato_poisson_t plan, int stage, int nf, void* stream);
 /* Tuning (no reference counterpart): fields per launch group (0 = all of
  * max_fields) and FFT engine (0: register-resident two-pass kernels for
- * even N <= 144 whose M factors into 2, 3, 5, 7 and for N = 160, with the
- * multi-field z forward for two or more fields; 1: generic Stockham; 2: the register
- * kernels with one z-forward CTA per field; 3: the multi-field z forward
+ * even N from 16 to 144 whose M factors into 2, 3, 5, 7 and for N = 160, with
+ * the multi-field z forward for two or more fields of a strand; 1: generic
+ * Stockham; 2: the register kernels with one z-forward CTA per field; 3: the multi-field z forward
  * from three fields; 4: as 0 with the scalar FP32 column passes instead of
  * the packed two-line ones, which FP32 plans use for M in
  * {128,160,192,256,320}, and a z forward that stages once per CTA
